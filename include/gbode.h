@@ -115,12 +115,18 @@ typedef struct {
                             partners with two bodies per thread, 3 = the same with one
                             body per thread; the packed loops need uniform masses
                             (per-body masses run the scalar loop) */
-  int32_t f64_pair;      /* FP64 pair term: 0 = the entry point's default, 1 = r^-3 from a
-                            Newton-refined reciprocal square root with fused multiply-add
-                            sums (a few ulp per term, ~2.5x fewer FP64 operations), 2 = the
-                            reference's operation order (IEEE sqrt and divisions,
-                            NBodyODE.hpp:89-98).  The standalone right-hand sides default to
-                            2; the integrator's FP64 stages default to 1 (exact mode: 2) */
+  int32_t f64_pair;      /* FP64 pair term: 0 = the entry point's default, 1 = fixed-point
+                            terms on the integer pipes (each within 2^-55 of its size, the
+                            sums of a CTA exact), with r^-3 from a Newton-refined reciprocal
+                            square root in FP64 (a few ulp per term) for pairs closer than
+                            about 2^-12 of the system's extent and where fixed point does
+                            not apply (coordinates that are not finite, exponents beyond
+                            2^+-300, negative masses, an extent far below the softening),
+                            2 = the reference's operation order (IEEE sqrt and divisions,
+                            NBodyODE.hpp:89-98).  The integrator's FP64 stages default to 1
+                            (exact mode: 2).  The standalone right-hand sides default to 2
+                            where j_split, lanes or bodies_per_cta is given, else to 1 with
+                            the reference's operation order in the place of the FP64 terms */
 } gb_force_tiling;
 
 int gb_nbody_rhs_f64(const double* x_dev, double* dxdt_dev, int64_t n_particles,
@@ -302,7 +308,8 @@ typedef struct {
   int32_t fsal;               /* reuse the last stage as the next first stage when the
                                  tableau allows it (bit-identical results) */
   int32_t exact;              /* serial-order forces and norm (reference bit pattern) */
-  int32_t attempts_per_sync;  /* attempts per graph replay (0 = 16) */
+  int32_t attempts_per_sync;  /* attempts per graph replay (0 = 16); the host waits for one
+                                 replay at a time, in FP64 without recording for up to 8 */
   int32_t record;             /* deliver every accepted state to the save callback */
   int64_t max_attempts;       /* 0 = unlimited (the reference has no bound) */
   double host_wait_timeout_s; /* bound on one host wait (0 = 600 s) */

@@ -266,8 +266,9 @@ def tiling(j_split=0, lanes=0, bodies_per_cta=0, scalar=False,
     """Force-kernel tiling.  Mixed precision: scalar=True (or mixed_variant=1)
     selects the scalar FP32 pair loop, mixed_variant=2 / 3 the packed f32x2
     loop over pairs of partners with two bodies / one body per thread, 0 the
-    library's choice (3).  FP64: f64_pair=1 the refined-rsqrt pair term,
-    2 the reference's operation order, 0 the entry point's default."""
+    library's choice (3).  FP64: f64_pair=1 fixed-point pair terms (each within
+    2^-55 of its size), 2 the reference's operation order, 0 the entry point's
+    default."""
     return GbForceTiling(j_split, lanes, bodies_per_cta, 1 if scalar else mixed_variant, f64_pair)
 
 
@@ -276,7 +277,9 @@ def tiling(j_split=0, lanes=0, bodies_per_cta=0, scalar=False,
 # ----------------------------------------------------------------------------
 def nbody_rhs_f64(x, n_particles: int, softening: float, mass: float = 1.0, masses=None,
                   tile: GbForceTiling | None = None, out=None, stream=None):
-    """dxdt = f(x) of NBodyODE (FP64, reference operation order)."""
+    """dxdt = f(x) of NBodyODE in FP64: pair terms in the reference's operation
+    order where the tile asks for it (f64_pair=2) or fixes the launch geometry,
+    else fixed-point terms, closer to the exact sum."""
     x = to_device(x)
     out = out if out is not None else _torch().empty_like(x)
     check(lib().gb_nbody_rhs_f64(_ptr(x), _ptr(out), n_particles, softening, mass,

@@ -114,7 +114,7 @@ __device__ __forceinline__ double group_max(double v, double* red, const G& grp)
 // Shared-memory bytes of the partner staging of TG threads.
 template <int PREC, int TG>
 constexpr int batch_smem_bytes() {
-  return PREC == GB_PREC_F64 ? 32 * TG
+  return PREC == GB_PREC_F64 ? f64_smem_bytes<TG>()
                              : (TG <= 128 ? jp_smem_bytes<TG>() : (int)sizeof(PackedBody) * TG);
 }
 
@@ -145,9 +145,7 @@ __device__ __forceinline__ void stage_unit(const DevTableau& tab, const BatchPar
   const bool skip_force = (s == 0 && k0_valid);
   if (!skip_force) {
     if constexpr (PREC == GB_PREC_F64) {
-      double* sh_pos = reinterpret_cast<double*>(sh_raw);
-      force_f64_cta<TG, L>(ysrc, n, i0, 0, n, sy.eps2, nullptr, sh_pos, sh_pos + 3 * TG, part,
-                           true, grp);
+      force_f64_cta<TG, L>(ysrc, n, i0, 0, n, sy.eps2, nullptr, sh_raw, part, kPairFixedFast, grp);
     } else {
       const PackedBody* src = (s == 0) ? P.PX + (long long)px * P.total_bodies + sy.body_off
                                        : P.PY + (long long)(s & 1) * P.total_bodies + sy.body_off;
@@ -307,9 +305,7 @@ __device__ __forceinline__ void rhs_unit(const BatchParams& P, long long u,
   const long long i0 = (long long)un.tile * BI;
   const double* xs = x + sy.var_off;
   if constexpr (PREC == GB_PREC_F64) {
-    double* sh_pos = reinterpret_cast<double*>(sh_raw);
-    force_f64_cta<TG, L>(xs, n, i0, 0, n, sy.eps2, nullptr, sh_pos, sh_pos + 3 * TG, part, false,
-                         grp);
+    force_f64_cta<TG, L>(xs, n, i0, 0, n, sy.eps2, nullptr, sh_raw, part, kPairFixedIeee, grp);
   } else {
     if constexpr (PK) {
       force_mixed_cta_jp<TG, L, BPT>(packed + sy.body_off, n, i0, 0, n, sy.eps2f, sh_raw, part,

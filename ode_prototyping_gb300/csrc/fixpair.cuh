@@ -1,0 +1,375 @@
+// fixpair.cuh -- softened pair terms of FP64 accuracy on the integer pipes.
+//
+// GB300 retires two FP64 operations per SM and clock, 16 times fewer than
+// 32 x 32 -> 64 bit integer multiply-adds (IMAD.WIDE: measured 4 cycles per
+// warp and sub-partition against 64 for a DFMA), and a pair term in FP64 takes
+// 18 of them even with a refined reciprocal square root.  Here the whole term
+// is fixed point: positions are 96-bit integers on a grid common to the bodies
+// a CTA reads, so the difference of two is exact; r^2, its reciprocal square
+// root, r^-3 and the products keep 57 bits or more; and the sums are integers,
+// exact and independent of the order.  36 IMAD.WIDE and about 75 simple
+// instructions per term.
+//
+// Scales.  The grid is U = 2^(Ex - 94) with |x_j - x_i| < 2^Ex in every
+// component and eps < 2^(Ex - 1); coordinates are taken modulo 2^96 U, so only
+// the differences have to fit and a system far from the origin loses nothing.
+// A pair is normalised by 2^k, k >= 0 such that R = (|d|^2 + eps^2) 4^k in
+// units of (2^64 U)^2 lies in [2^60, 2^62); its contribution carries the
+// weight 4^k.  Pairs closer than about 2^-12 2^Ex (k > kFxMaxK) do not fit the
+// sums' window: they get weight 0 here and are added by the caller in FP64.
+//
+// Error: d is exact where a coordinate's last bit is a multiple of U (every
+// coordinate above 2^-41 2^Ex) and enters with 62 bits; R and the Newton
+// residual hold 2^-58.  A term is within 2^-55 of its size (0.04 2^-53 rms; a
+// term in FP64: 1.3 2^-53 rms, up to 5 2^-53).
+//
+// Measured at N = 16384 (right-hand side): 1.6 ms against 22.3 ms for the FP64
+// loop in the reference's operation order and 12 ms with the refined
+// reciprocal square root; about 111 instructions and 220 cycles of a
+// sub-partition per 32 terms, the multiply-add pipe (4 cycles for an IMAD.WIDE)
+// 80 % busy.
+#pragma once
+
+#include <cstdint>
+#include <cstring>
+
+namespace gb {
+
+#ifdef __CUDACC__
+#define GB_HD __host__ __device__ __forceinline__
+#else
+#define GB_HD inline
+#endif
+
+constexpr int kFxMaxK = 13;       // largest normalisation inside the window
+constexpr int kFxRows = kFxMaxK + 2;  // table rows (the last: weight 0)
+
+struct Fx96 {  // two's complement, w0 least significant
+  uint32_t w0, w1, w2;
+};
+
+// row k of the softening table: eps^2 at normalisation k, the weight 4^k
+struct alignas(16) FxRow {
+  uint32_t e_lo, e_hi;
+  uint32_t p;
+  uint32_t pad;
+};
+
+struct FxAcc {  // sum of the terms, weight 2^32, 1 and 2
+  long long h;
+  unsigned long long l;
+  long long m;
+};
+
+// 32 x 32 -> 64 bit products and words, each one instruction.  In PTX: from C
+// the compiler turns products of a 64-bit value's high word into full 64-bit
+// multiplications (a term took 168 instructions so, against 109).
+GB_HD uint32_t fx_lo(uint64_t v) { return (uint32_t)v; }
+GB_HD uint32_t fx_hi(uint64_t v) {
+#ifdef __CUDA_ARCH__
+  uint32_t hi;
+  asm("{.reg .b32 lo; mov.b64 {lo, %0}, %1;}" : "=r"(hi) : "l"(v));
+  return hi;
+#else
+  return (uint32_t)(v >> 32);
+#endif
+}
+GB_HD uint64_t fx_pair(uint32_t lo, uint32_t hi) {
+#ifdef __CUDA_ARCH__
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+  return v;
+#else
+  return ((uint64_t)hi << 32) | lo;
+#endif
+}
+GB_HD uint64_t fx_mul(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+  uint64_t v;
+  asm("mul.wide.u32 %0, %1, %2;" : "=l"(v) : "r"(a), "r"(b));
+  return v;
+#else
+  return (uint64_t)a * b;
+#endif
+}
+GB_HD uint64_t fx_mad(uint32_t a, uint32_t b, uint64_t c) {
+#ifdef __CUDA_ARCH__
+  uint64_t v;
+  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(v) : "r"(a), "r"(b), "l"(c));
+  return v;
+#else
+  return (uint64_t)a * b + c;
+#endif
+}
+GB_HD int64_t fx_muls(int32_t a, int32_t b) {
+#ifdef __CUDA_ARCH__
+  int64_t v;
+  asm("mul.wide.s32 %0, %1, %2;" : "=l"(v) : "r"(a), "r"(b));
+  return v;
+#else
+  return (int64_t)a * b;
+#endif
+}
+GB_HD int64_t fx_mads(int32_t a, int32_t b, int64_t c) {
+#ifdef __CUDA_ARCH__
+  int64_t v;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(v) : "r"(a), "r"(b), "l"(c));
+  return v;
+#else
+  return (int64_t)a * b + c;
+#endif
+}
+
+GB_HD uint32_t fx_shl(uint32_t lo, uint32_t hi, int k) {  // high word of (hi:lo) << k, k < 32
+#ifdef __CUDA_ARCH__
+  return __funnelshift_l(lo, hi, k);
+#else
+  return k ? (hi << k) | (lo >> (32 - k)) : hi;
+#endif
+}
+
+GB_HD uint32_t fx_float_bits(float f) {
+#ifdef __CUDA_ARCH__
+  return __float_as_uint(f);
+#else
+  uint32_t u;
+  memcpy(&u, &f, 4);
+  return u;
+#endif
+}
+
+// v in units of U = 2^(ex - 94) modulo 2^96, truncated (exact when v is a
+// multiple of U).
+GB_HD Fx96 fx_from_double(double v, int ex) {
+#ifdef __CUDA_ARCH__
+  const uint64_t bits = (uint64_t)__double_as_longlong(v);
+#else
+  uint64_t bits;
+  memcpy(&bits, &v, 8);
+#endif
+  const int e = (int)((bits >> 52) & 0x7ff);
+  uint64_t m = bits & 0xfffffffffffffull;
+  if (e) m |= 1ull << 52;
+  const int sh = (e ? e : 1) - 1075 - ex + 94;
+  uint64_t lo = 0, hi = 0;
+  if (sh >= 64) {
+    hi = sh < 96 ? m << (sh - 64) : 0;
+  } else if (sh > 0) {
+    lo = m << sh;
+    hi = m >> (64 - sh);
+  } else if (sh > -64) {
+    lo = m >> -sh;
+  }
+  if (bits >> 63) {
+    lo = ~lo + 1;
+    hi = ~hi + (lo == 0);
+  }
+  return Fx96{(uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi};
+}
+
+GB_HD Fx96 fx_sub(const Fx96& a, const Fx96& b) {
+  Fx96 r;
+#ifdef __CUDA_ARCH__
+  asm("sub.cc.u32 %0, %3, %6;\n\tsubc.cc.u32 %1, %4, %7;\n\tsubc.u32 %2, %5, %8;"
+      : "=r"(r.w0), "=r"(r.w1), "=r"(r.w2)
+      : "r"(a.w0), "r"(a.w1), "r"(a.w2), "r"(b.w0), "r"(b.w1), "r"(b.w2));
+#else
+  const uint64_t al = fx_pair(a.w0, a.w1), bl = fx_pair(b.w0, b.w1), d = al - bl;
+  r.w0 = fx_lo(d);
+  r.w1 = fx_hi(d);
+  r.w2 = a.w2 - b.w2 - (al < bl);
+#endif
+  return r;
+}
+
+// Normalisation of a difference from the high words, clamped to kFxMaxK + 1:
+// R 4^k in [2^60 (1 - 2^-8), 2^62 (1 - 2^-9)], so that every component's high
+// word stays below 2^31 (the high words, truncated, know r to 2^-13 at k = 13).
+GB_HD int fx_norm(const Fx96& dx, const Fx96& dy, const Fx96& dz, float eps2f) {
+  const float fx = (float)(int32_t)dx.w2, fy = (float)(int32_t)dy.w2, fz = (float)(int32_t)dz.w2;
+#ifdef __CUDA_ARCH__
+  const float f = __fmaf_rn(fx, fx, __fmaf_rn(fy, fy, __fmaf_rn(fz, fz, eps2f)));
+#else
+  const float f = fx * fx + fy * fy + fz * fz + eps2f;
+#endif
+  const int k = (int)((0x5e7fffffu - 0x8000u - fx_float_bits(f)) >> 24);
+  return k < kFxMaxK + 1 ? k : kFxMaxK + 1;
+}
+
+struct FxDiff {  // a normalised component: (h 2^31 + l), 0 <= l < 2^31
+  int32_t h, l;
+};
+
+GB_HD FxDiff fx_scale(const Fx96& d, int k) {
+  return FxDiff{(int32_t)fx_shl(d.w1, d.w2, k), (int32_t)(fx_shl(d.w0, d.w1, k) >> 1)};
+}
+
+// R = (|d|^2 + eps^2) 4^k; the table's eps^2 carries the mean of what is dropped.
+GB_HD uint64_t fx_r2(const FxDiff& x, const FxDiff& y, const FxDiff& z, uint64_t eps2) {
+  int64_t a = fx_mads(z.h, z.h, fx_mads(y.h, y.h, fx_mads(x.h, x.h, (int64_t)eps2)));
+  const int64_t b = fx_mads(z.h, z.l, fx_mads(y.h, y.l, fx_muls(x.h, x.l)));
+  return (uint64_t)fx_mads((int32_t)fx_hi((uint64_t)b), 4, a);
+}
+
+// Y <= 2^61 / sqrt(R), within 2^-19.9 of it from below: 24 bits from the SFU's
+// reciprocal square root (relative error <= 2^-22.9), scaled down by 5 2^-24
+// so that the residual 1 - R Y^2 / 2^122 is positive.
+GB_HD uint32_t fx_rsqrt_seed(uint64_t r) {
+  const float rh = (float)fx_hi(r);
+  constexpr float kScale = 35184372088832.0f * (1.0f - 5.0f / 16777216.0f);
+#ifdef __CUDA_ARCH__
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(rh));
+  return __float2uint_rz(__fmul_rn(y, kScale));
+#else
+  return (uint32_t)((float)(1.0 / __builtin_sqrt((double)rh)) * kScale);
+#endif
+}
+
+// Residual e = 1 - R Q / 2^122 of Q = Y^2, in units of 2^-58.
+GB_HD uint64_t fx_residual(uint64_t r, uint64_t q) {
+  const uint64_t m = fx_mad(fx_lo(r), fx_hi(q), fx_mul(fx_hi(r), fx_lo(q)));
+  const uint64_t rq = fx_mad(fx_hi(r), fx_hi(q), fx_pair(fx_hi(m), 0));
+  return (1ull << 58) - 1 - rq;
+}
+
+// S = 2^151 R^(-3/2) = Y^3 (1 - e)^(-3/2) (in [2^58, 2^61]):
+// (1 - e)^(-3/2) = 1 + 3/2 e + 15/8 e^2 + O(2^-58.5).
+GB_HD uint64_t fx_rinv3(uint64_t r) {
+  const uint32_t y = fx_rsqrt_seed(r);
+  const uint64_t q = fx_mul(y, y);
+  const uint64_t e = fx_residual(r, q);
+  const uint32_t eh = (uint32_t)(e >> 12);
+  // g = (3/2 e + 15/8 e^2) in units of 2^-64
+  const uint64_t g0 = fx_mad(fx_lo(e), 96u, fx_pair(fx_hi(fx_mul(eh * 30u, eh)), 0));
+  const uint32_t gl = fx_lo(g0), gh = fx_hi(g0) + fx_hi(e) * 96u;
+  // Y (1 + g) in units of 2^-32
+  const uint64_t y1 = fx_mad(y, gh, fx_pair(fx_hi(fx_mul(y, gl)), y));
+  const uint64_t m = fx_mad(fx_lo(y1), fx_hi(q), fx_mul(fx_hi(y1), fx_lo(q)));
+  return fx_mad(fx_hi(y1), fx_hi(q), fx_pair(fx_hi(m), 0));
+}
+
+// Adds weight p times the component S (h 2^31 + l) / 2^62.
+GB_HD void fx_add(FxAcc& a, int32_t sh, int32_t sl, const FxDiff& d, uint32_t p) {
+  const uint64_t hh = (uint64_t)fx_muls(sh, d.h);
+  const uint64_t m = (uint64_t)fx_mads(sl, d.h, fx_mads(sh, d.l, 1ll << 31));
+  a.h = fx_mads((int32_t)fx_hi(hh), (int32_t)p, a.h);
+  a.l = fx_mad(fx_lo(hh), p, a.l);
+  a.m = fx_mads((int32_t)fx_hi(m), (int32_t)p, a.m);
+}
+
+// Terms added between two folds: a.l stays below 2^63 (2^32 2^26 a term).
+constexpr int kFxChunk = 32;
+
+GB_HD void fx_fold(__int128& tot, FxAcc& a) {
+  tot += ((__int128)a.h << 32) + (__int128)a.l + ((__int128)a.m << 1);
+  a.h = 0;
+  a.l = 0;
+  a.m = 0;
+}
+
+// v 2^sc to the nearest double (|v| < 2^126, the result's exponent in range).
+GB_HD double fx_to_double(__int128 v, int sc) {
+  const bool neg = v < 0;
+  unsigned __int128 u = neg ? (unsigned __int128)(-v) : (unsigned __int128)v;
+  uint64_t hi = (uint64_t)(u >> 64), lo = (uint64_t)u;
+  if ((hi | lo) == 0) return 0.0;
+#ifdef __CUDA_ARCH__
+  const int z = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo);
+#else
+  const int z = hi ? __builtin_clzll(hi) : 64 + __builtin_clzll(lo);
+#endif
+  u <<= z;
+  hi = (uint64_t)(u >> 64);
+  lo = (uint64_t)u;
+  // 53 bits, nearest even
+  uint64_t m = hi >> 11;
+  const uint64_t rest = hi & 0x7ff;
+  if (rest > 0x400 || (rest == 0x400 && (lo != 0 || (m & 1)))) ++m;
+  // value = m 2^(127 - z - 52 + sc); m may have become 2^53
+  const uint64_t bits = ((uint64_t)(127 - z + sc + 1022) << 52) + m + (neg ? 1ull << 63 : 0);
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double((long long)bits);
+#else
+  double d;
+  memcpy(&d, &bits, 8);
+  return d;
+#endif
+}
+
+// Row k of the softening table on the grid of ex: eps^2 in units of (2^64 U)^2
+// times 4^k (the 2 is the mean of what fx_r2 drops), 4^k as the weight.
+GB_HD FxRow fx_row(int k, double eps2, int ex) {
+#ifdef __CUDA_ARCH__
+  const double v = scalbn(eps2, 2 * (30 - ex + k));
+  const uint64_t e = (v < 4.6e18 ? (uint64_t)__double2ull_rn(v) : 1ull << 62) + 2;
+#else
+  const double v = __builtin_scalbn(eps2, 2 * (30 - ex + k));
+  const uint64_t e = (v < 4.6e18 ? (uint64_t)(v + 0.5) : 1ull << 62) + 2;
+#endif
+  return FxRow{(uint32_t)e, (uint32_t)(e >> 32), k <= kFxMaxK ? 1u << (2 * k) : 0u, 0u};
+}
+
+// A partner's record.  Per-body masses: mass = mu 2^(em + q - 61) with mu in
+// [2^61, 2^62), q <= 0, em the largest mass's exponent; mu = 0 for a mass of 0.
+struct alignas(16) FxBody {
+  Fx96 x, y, z;
+  uint32_t mu_lo, mu_hi;
+  int32_t q;
+};
+
+GB_HD void fx_mass(FxBody& b, double mass, int em) {
+#ifdef __CUDA_ARCH__
+  const uint64_t bits = (uint64_t)__double_as_longlong(mass);
+#else
+  uint64_t bits;
+  memcpy(&bits, &mass, 8);
+#endif
+  const int e = (int)((bits >> 52) & 0x7ff);
+  const uint64_t mu = e ? ((bits & 0xfffffffffffffull) | (1ull << 52)) << 9 : 0;
+  b.mu_lo = fx_lo(mu);
+  b.mu_hi = fx_hi(mu);
+  b.q = e ? e - 1023 - em : 0;
+}
+
+// One term into the three sums; returns its normalisation (kFxMaxK + 1: not
+// added).  With masses the weight is 4^k 2^q: what is below 1 shifts S right,
+// which drops only bits below the heaviest body's at the largest distance.
+template <bool MASS>
+GB_HD int fx_term(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& zi, float eps2f,
+                  const FxRow* tab, FxAcc (&a)[3]) {
+  const Fx96 ux = fx_sub(j.x, xi), uy = fx_sub(j.y, yi), uz = fx_sub(j.z, zi);
+  const int k = fx_norm(ux, uy, uz, eps2f);
+  const FxRow row = tab[k];
+  const FxDiff dx = fx_scale(ux, k), dy = fx_scale(uy, k), dz = fx_scale(uz, k);
+  uint64_t s = fx_rinv3(fx_r2(dx, dy, dz, fx_pair(row.e_lo, row.e_hi)));
+  uint32_t p = row.p;
+  if (MASS) {
+    s <<= 2;
+    const uint64_t m = fx_mad(fx_lo(s), j.mu_hi, fx_mul(fx_hi(s), j.mu_lo));
+    s = fx_mad(fx_hi(s), j.mu_hi, fx_pair(fx_hi(m), 0));  // S mass 2^(-em - q - 1)
+    const int t = 2 * k + j.q;
+    if (t < 0) s = t > -63 ? (s + (1ull << (-t - 1))) >> -t : 0;
+    p = k <= kFxMaxK ? 1u << (t > 0 ? t : 0) : 0u;
+  }
+  const int32_t sh = (int32_t)(s >> 31), sl = (int32_t)((uint32_t)s & 0x7fffffffu);
+  fx_add(a[0], sh, sl, dx, p);
+  fx_add(a[1], sh, sl, dy, p);
+  fx_add(a[2], sh, sl, dz, p);
+  return k;
+}
+
+// exponent of a term's unit: sum 2^(fx_out_exp(ex)) is the sum of d / r^3, and
+// sum 2^(fx_out_exp(ex) + em + 1) that of mass d / r^3
+GB_HD int fx_out_exp(int ex) { return -60 - 2 * ex; }
+
+// eps^2 in units of (2^64 U)^2
+GB_HD float fx_eps2f(double eps2, int ex) {
+#ifdef __CUDA_ARCH__
+  return (float)scalbn(eps2, 2 * (30 - ex));
+#else
+  return (float)__builtin_scalbn(eps2, 2 * (30 - ex));
+#endif
+}
+
+}  // namespace gb

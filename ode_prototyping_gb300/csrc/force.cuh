@@ -17,6 +17,7 @@
 
 #include <type_traits>
 
+#include "fixpair.cuh"
 #include "gb_internal.cuh"
 
 namespace gb {
@@ -125,6 +126,7 @@ __device__ __forceinline__ void cluster_combine_rows(double (*part)[3], int rank
 // ---------------------------------------------------------------------------
 struct WholeCta {
   __device__ __forceinline__ unsigned tid() const { return threadIdx.x; }
+  __device__ __forceinline__ int id() const { return 0; }
   __device__ __forceinline__ void sync() const { __syncthreads(); }
 };
 
@@ -134,6 +136,7 @@ struct WarpGroup {
   unsigned t;  // thread index within the group
   int bar;     // named barrier id, 1..4 (0 is __syncthreads)
   __device__ __forceinline__ unsigned tid() const { return t; }
+  __device__ __forceinline__ int id() const { return bar; }
   __device__ __forceinline__ void sync() const {
     // immediate ids, so the kernel reserves barriers 0..4 only
     switch (bar) {
@@ -146,22 +149,280 @@ struct WarpGroup {
 };
 
 // ---------------------------------------------------------------------------
+// FP64 accuracy on the integer pipes (fixpair.cuh): partial sums of one CTA (or
+// thread group) over its partner chunk.  The grid is that of the bodies the CTA
+// reads (a scan of their extents first: all its partners once more from L2, 1 %
+// of the time of the pairs), so the differences are exact and the sums
+// independent of the order, of T and of L.  Pairs too close for the window are
+// added in FP64; where most pairs are (one body very far from the others), a
+// warp gives the fixed-point terms up and runs in FP64.
+// ---------------------------------------------------------------------------
+template <int T>
+constexpr int f64_smem_bytes() {
+  // partner records (at least the 32 T bytes of the FP64 loop), table, reduction
+  return ((int)sizeof(FxBody) * T + (int)sizeof(FxRow) * kFxRows + 28 * (T / 32) + 15) / 16 * 16;
+}
+
+// Pair terms of the FP64 loops.
+enum { kPairIeee = 0, kPairFast = 1, kPairFixedFast = 2, kPairFixedIeee = 3 };
+
+// One partner's term in FP64, added to s.
+__device__ __forceinline__ void add_pair_f64(const double* pos, long long i, long long j,
+                                             double eps2, const double* masses, bool ieee,
+                                             double* s) {
+  const double mj = masses ? masses[j] : 1.0;
+  if (ieee) {
+    double ax, ay, az;
+    pair_term_f64(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], pos[3 * j], pos[3 * j + 1],
+                  pos[3 * j + 2], eps2, ax, ay, az);
+    if (masses) {
+      ax = dmul(ax, mj);
+      ay = dmul(ay, mj);
+      az = dmul(az, mj);
+    }
+    s[0] = dadd(s[0], ax);
+    s[1] = dadd(s[1], ay);
+    s[2] = dadd(s[2], az);
+  } else {
+    const double dx = pos[3 * j] - pos[3 * i];
+    const double dy = pos[3 * j + 1] - pos[3 * i + 1];
+    const double dz = pos[3 * j + 2] - pos[3 * i + 2];
+    double r3 = rinv3_f64(fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))));
+    if (masses) r3 *= mj;
+    s[0] = fma(dx, r3, s[0]);
+    s[1] = fma(dy, r3, s[1]);
+    s[2] = fma(dz, r3, s[2]);
+  }
+}
+
+// The partners of one lane's chunk (j0 + u L, u < steps) whose bits are set in
+// `mask` (bit steps - 1 - u) in FP64, lanes side by side: as many rounds as the
+// warp's lane with most of them, which is returned.  The whole warp calls it.
+static __device__ __noinline__ int fx_chunk_f64(unsigned mask, int steps, long long j0, int L,
+                                                const double* pos, long long i, double eps2,
+                                                const double* masses, bool ieee, double* s) {
+  int rounds = 0;
+#pragma unroll 1
+  while (__any_sync(0xffffffffu, mask != 0)) {
+    ++rounds;
+    if (mask) {
+      const int u = steps - 32 + __clz(mask);
+      mask &= ~(0x80000000u >> __clz(mask));
+      add_pair_f64(pos, i, j0 + (long long)u * L, eps2, masses, ieee, s);
+    }
+  }
+  return rounds;
+}
+
+// Barrier of a group of `threads` threads: the whole CTA (bar 0) or a warp
+// group with its own named barrier.
+__device__ __forceinline__ void group_bar(int bar, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(threads) : "memory");
+}
+
+// The tiles of one CTA or group.  Not inlined, and the geometry (T threads, L
+// lanes) a run-time value: the loop is long enough for the call, and a copy of
+// it in each of the FP64 kernels would make them slow to build.
+template <bool MASS>
+__device__ __noinline__ void force_fx_tiles(const double* __restrict__ pos, long long n,
+                                            long long i0, long long jb, long long je, double eps2,
+                                            const double* __restrict__ masses, int ex, int em,
+                                            bool ieee, int T, int L, int tid, int bar,
+                                            FxBody* rec, const FxRow* tab, double (*part)[3]) {
+  const int b = tid / L;
+  const int l = tid % L;
+  const long long i = i0 + b;
+  const bool valid = i < n;
+  Fx96 xi = {}, yi = {}, zi = {};
+  if (valid) {
+    xi = fx_from_double(pos[3 * i], ex);
+    yi = fx_from_double(pos[3 * i + 1], ex);
+    zi = fx_from_double(pos[3 * i + 2], ex);
+  }
+  const float eps2f = fx_eps2f(eps2, ex);
+  __int128 tot[3] = {0, 0, 0};
+  double near[3] = {0.0, 0.0, 0.0};
+  bool in_f64 = false;  // uniform in the warp
+  for (long long j0 = jb; j0 < je; j0 += T) {
+    const int cnt = (int)min((long long)T, je - j0);
+    group_bar(bar, T);
+    if (tid < cnt) {
+      const long long j = j0 + tid;
+      FxBody r;
+      r.x = fx_from_double(pos[3 * j], ex);
+      r.y = fx_from_double(pos[3 * j + 1], ex);
+      r.z = fx_from_double(pos[3 * j + 2], ex);
+      r.mu_lo = r.mu_hi = 0;
+      r.q = 0;
+      if (MASS) fx_mass(r, masses[j], em);
+      rec[tid] = r;
+    }
+    group_bar(bar, T);
+    for (int c0 = l; c0 - l < cnt; c0 += kFxChunk * L) {
+      const int end = min(cnt, c0 + kFxChunk * L);
+      const int steps = c0 < end ? (end - c0 + L - 1) / L : 0;
+      unsigned mask = in_f64 && steps ? 0xffffffffu >> (32 - steps) : 0u;
+      if (!in_f64) {
+        FxAcc a[3] = {};
+        // unrolled twice: 1.59 ms at N = 16384 against 1.72 ms (1) and 1.73 ms (4)
+#pragma unroll 2
+        for (int jj = c0; jj < end; jj += L) {
+          const int k = fx_term<MASS>(rec[jj], xi, yi, zi, eps2f, tab, a);
+          mask = __funnelshift_l((unsigned)(kFxMaxK - k), mask, 1);  // 1 when k > kFxMaxK
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) fx_fold(tot[d], a[d]);
+      }
+      if (__any_sync(0xffffffffu, mask != 0)) {
+        if (!valid) mask = 0;
+        const long long self = i - j0 - c0;  // not the body itself
+        if (self >= 0 && self < (long long)steps * L && self % L == 0)
+          mask &= ~(1u << (steps - 1 - (int)(self / L)));
+        const int rounds = fx_chunk_f64(mask, steps, j0 + c0, L, pos, i, eps2, masses, ieee, near);
+        // an FP64 term costs 5 fixed-point ones: where a lane needs more than 4
+        // in 5 of its terms in FP64, the others' are not worth their time
+        in_f64 = in_f64 || rounds > kFxChunk * 4 / 5;
+      }
+    }
+  }
+  const int sc = fx_out_exp(ex) + (MASS ? em + 1 : 0);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    __int128 v = tot[d];
+    double s = near[d];
+    for (int off = L / 2; off >= 1; off /= 2) {
+      const unsigned long long lo = __shfl_down_sync(0xffffffffu, (unsigned long long)v, off);
+      const unsigned long long hi =
+          __shfl_down_sync(0xffffffffu, (unsigned long long)(v >> 64), off);
+      v += (__int128)(((unsigned __int128)hi << 64) | lo);
+      s = dadd(s, __shfl_down_sync(0xffffffffu, s, off));
+    }
+    if (l == 0) part[b][d] = dadd(fx_to_double(v, sc), s);
+  }
+}
+
+// Signed integers in the order of the doubles with these high words.
+__device__ __forceinline__ int order_key(double v) {
+  const int h = __double2hiint(v);
+  return h ^ ((h >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ double key_bound(int key, bool upper) {
+  const int h = key ^ ((key >> 31) & 0x7fffffff);
+  return __hiloint2double(h, (h < 0) != upper ? -1 : 0);  // outwards over the low word
+}
+
+// Returns false, uniformly in the group, when there is no grid: a coordinate
+// that is not finite, bodies all within a sixteenth of the softening,
+// exponents beyond 2^+-300, or a mass that is negative, not finite or all of
+// them zero.  smem: f64_smem_bytes<T>() bytes.
+static __device__ __noinline__ bool force_fx_group(const double* __restrict__ pos, long long n,
+                                                   long long i0, long long jb, long long je,
+                                                   double eps2, const double* __restrict__ masses,
+                                                   bool ieee, unsigned char* smem,
+                                                   double (*part)[3], int T, int L, int tid,
+                                                   int bar) {
+  FxBody* rec = reinterpret_cast<FxBody*>(smem);
+  FxRow* tab = reinterpret_cast<FxRow*>(rec + T);
+  int* red = reinterpret_cast<int*>(tab + kFxRows);
+  const int nw = T / 32;
+  int lo[3], hi[3];
+  unsigned mm = 0;
+  {
+    const long long i = min(i0 + tid / L, n - 1);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) lo[c] = hi[c] = order_key(pos[3 * i + c]);
+  }
+#pragma unroll 4
+  for (long long j = jb + tid; j < je; j += T) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int k = order_key(pos[3 * j + c]);
+      lo[c] = min(lo[c], k);
+      hi[c] = max(hi[c], k);
+    }
+  }
+  if (masses) {
+    // a negative mass reads as a large unsigned word
+#pragma unroll 4
+    for (long long j = jb + tid; j < je; j += T) mm = max(mm, (unsigned)__double2hiint(masses[j]));
+  }
+  mm = __reduce_max_sync(0xffffffffu, mm);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    lo[c] = __reduce_min_sync(0xffffffffu, lo[c]);
+    hi[c] = __reduce_max_sync(0xffffffffu, hi[c]);
+  }
+  if ((tid & 31) == 0) {
+    int* r = red + 7 * (tid / 32);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      r[c] = lo[c];
+      r[3 + c] = hi[c];
+    }
+    r[6] = (int)mm;
+  }
+  group_bar(bar, T);
+  for (int w = 0; w < nw; ++w) {
+    const int* r = red + 7 * w;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      lo[c] = min(lo[c], r[c]);
+      hi[c] = max(hi[c], r[3 + c]);
+    }
+    mm = max(mm, (unsigned)r[6]);
+  }
+  constexpr int kInf = 0x7ff00000;
+  int xe = 0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    if (hi[c] >= kInf || lo[c] <= ~kInf) return false;
+    const double ext = key_bound(hi[c], true) - key_bound(lo[c], false);
+    xe = max(xe, __double2hiint(ext) >> 20);
+  }
+  int ex = xe - 1022;  // the extents are below 2^ex
+  const int e2 = (__double2hiint(eps2) >> 20) & 0x7ff;
+  if (e2) {
+    const int ee = ((e2 - 1023) >> 1) + 1;  // eps < 2^ee
+    if (ex < ee - 4) return false;
+    ex = max(ex, ee + 1);
+  }
+  const int em = (int)(mm >> 20) - 1023;  // 2^em <= the largest mass < 2^(em + 1)
+  if (ex < -300 || ex > 300 || (masses && (em < -300 || em > 300))) return false;
+  if (tid < kFxRows) tab[tid] = fx_row(tid, eps2, ex);
+  if (masses)
+    force_fx_tiles<true>(pos, n, i0, jb, je, eps2, masses, ex, em, ieee, T, L, tid, bar, rec, tab,
+                         part);
+  else
+    force_fx_tiles<false>(pos, n, i0, jb, je, eps2, nullptr, ex, 0, ieee, T, L, tid, bar, rec,
+                          tab, part);
+  return true;
+}
+
+// ---------------------------------------------------------------------------
 // FP64: partial sums of one CTA (or thread group) over its partner chunk.
-// sh_pos holds 3*T doubles, sh_m T doubles (per-body masses only).  Results
-// land in part[b].  fast = false: every pair term in the reference's
-// operation order (IEEE sqrt and divisions, NBodyODE.hpp:89-98), summed with
-// IEEE adds; fast = true: r^-3 from the refined reciprocal square root
-// (rinv3_f64) and fused multiply-add accumulation, a few ulp per term from
-// the reference's.  With L lanes, lane l takes the partners j = l (mod L) in
-// ascending order whatever T is, so the sums do not depend on the group size.
+// smem: f64_smem_bytes<T>() bytes, 16-byte aligned.  Results land in part[b].
+// pair = kPairIeee: every pair term in the reference's operation order (IEEE
+// sqrt and divisions, NBodyODE.hpp:89-98), summed with IEEE adds.  kPairFast:
+// r^-3 from the refined reciprocal square root (rinv3_f64) and fused
+// multiply-add accumulation.  kPairFixed...: the fixed-point terms, and one of
+// the two where they do not apply.  With L lanes, lane l takes the partners
+// j = l (mod L) in ascending order whatever T is, so the sums do not depend on
+// the group size.
 // ---------------------------------------------------------------------------
 template <int T, int L, class G = WholeCta>
 __device__ __forceinline__ void force_f64_cta(const double* __restrict__ pos, long long n,
                                               long long i0, long long jb, long long je,
                                               double eps2, const double* __restrict__ masses,
-                                              double* sh_pos, double* sh_m, double (*part)[3],
-                                              bool fast = false, const G& grp = G{}) {
+                                              unsigned char* smem, double (*part)[3], int pair,
+                                              const G& grp = G{}) {
   constexpr int BI = T / L;
+  const bool ieee = pair == kPairIeee || pair == kPairFixedIeee;
+  if (pair >= kPairFixedFast &&
+      force_fx_group(pos, n, i0, jb, je, eps2, masses, ieee, smem, part, T, L, (int)grp.tid(),
+                     grp.id()))
+    return;
+  double* sh_pos = reinterpret_cast<double*>(smem);
+  double* sh_m = sh_pos + 3 * T;
   const unsigned tid = grp.tid();
   const int b = tid / L;
   const int l = tid % L;
@@ -181,7 +442,7 @@ __device__ __forceinline__ void force_f64_cta(const double* __restrict__ pos, lo
       for (int k = tid; k < cnt; k += T) sh_m[k] = masses[j0 + k];
     grp.sync();
     if (i >= n) continue;
-    if (fast) {
+    if (!ieee) {
       for (int jj = l; jj < cnt; jj += L) {
         if (j0 + jj == i) continue;
         const double dx = sh_pos[3 * jj] - xi;

@@ -94,7 +94,7 @@ struct FusedParams {
   const void* mlp;     // device MLP weights (learned controller) or null
   long long n, n_var, n_itiles, n_parts;
   int exact;
-  int f64_fast;        // FP64 stages: refined-rsqrt pair term (not exact mode)
+  int f64_pair;        // FP64 stages' pair term (kPair...)
   int S;
   // partner-chunk split without clusters (packed mixed path)
   int n_chunks;          // partner chunks per i-tile

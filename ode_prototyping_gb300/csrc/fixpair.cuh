@@ -233,20 +233,33 @@ GB_HD uint64_t fx_residual(uint64_t r, uint64_t q) {
   return (1ull << 58) - 1 - rq;
 }
 
-// S = 2^151 R^(-3/2) = Y^3 (1 - e)^(-3/2) (in [2^58, 2^61]):
-// (1 - e)^(-3/2) = 1 + 3/2 e + 15/8 e^2 + O(2^-58.5).
+// y (1 - e)^(-c) in units of 2^-32 for Y = y, to the second order in e (the
+// third is below 2^-58): e1 = 2^6 c, e2 = 2^4 c (c + 1) / 2.
+GB_HD uint64_t fx_refine(uint32_t y, uint64_t e, uint32_t e1, uint32_t e2) {
+  const uint32_t eh = (uint32_t)(e >> 12);
+  // the correction in units of 2^-64
+  const uint64_t g0 = fx_mad(fx_lo(e), e1, fx_pair(fx_hi(fx_mul(eh * e2, eh)), 0));
+  const uint32_t gl = fx_lo(g0), gh = fx_hi(g0) + fx_hi(e) * e1;
+  return fx_mad(y, gh, fx_pair(fx_hi(fx_mul(y, gl)), y));
+}
+
+// The high 64 bits of a product (without the low words' part: 1 unit).
+GB_HD uint64_t fx_mul_hi(uint64_t a, uint64_t b) {
+  const uint64_t m = fx_mad(fx_lo(a), fx_hi(b), fx_mul(fx_hi(a), fx_lo(b)));
+  return fx_mad(fx_hi(a), fx_hi(b), fx_pair(fx_hi(m), 0));
+}
+
+// S = 2^151 R^(-3/2) = Y^3 (1 - e)^(-3/2) (in [2^58, 2^61]).
 GB_HD uint64_t fx_rinv3(uint64_t r) {
   const uint32_t y = fx_rsqrt_seed(r);
   const uint64_t q = fx_mul(y, y);
-  const uint64_t e = fx_residual(r, q);
-  const uint32_t eh = (uint32_t)(e >> 12);
-  // g = (3/2 e + 15/8 e^2) in units of 2^-64
-  const uint64_t g0 = fx_mad(fx_lo(e), 96u, fx_pair(fx_hi(fx_mul(eh * 30u, eh)), 0));
-  const uint32_t gl = fx_lo(g0), gh = fx_hi(g0) + fx_hi(e) * 96u;
-  // Y (1 + g) in units of 2^-32
-  const uint64_t y1 = fx_mad(y, gh, fx_pair(fx_hi(fx_mul(y, gl)), y));
-  const uint64_t m = fx_mad(fx_lo(y1), fx_hi(q), fx_mul(fx_hi(y1), fx_lo(q)));
-  return fx_mad(fx_hi(y1), fx_hi(q), fx_pair(fx_hi(m), 0));
+  return fx_mul_hi(fx_refine(y, fx_residual(r, q), 96u, 30u), q);
+}
+
+// 2^93 R^(-1/2) = Y (1 - e)^(-1/2) 2^32 (in [2^62, 2^63]).
+GB_HD uint64_t fx_rinv1(uint64_t r) {
+  const uint32_t y = fx_rsqrt_seed(r);
+  return fx_refine(y, fx_residual(r, fx_mul(y, y)), 32u, 6u);
 }
 
 // Adds weight p times the component S (h 2^31 + l) / 2^62.
@@ -332,9 +345,10 @@ GB_HD void fx_mass(FxBody& b, double mass, int em) {
   b.q = e ? e - 1023 - em : 0;
 }
 
-// One term into the three sums; returns its normalisation (kFxMaxK + 1: not
-// added).  With masses the weight is 4^k 2^q: what is below 1 shifts S right,
-// which drops only bits below the heaviest body's at the largest distance.
+// One term of the accelerations into the three sums; returns its
+// normalisation (kFxMaxK + 1: not added).  With masses the weight is 4^k 2^q:
+// what is below 1 shifts S right, which drops only bits below the heaviest
+// body's at the largest distance.
 template <bool MASS>
 GB_HD int fx_term(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& zi, float eps2f,
                   const FxRow* tab, FxAcc (&a)[3]) {
@@ -345,9 +359,7 @@ GB_HD int fx_term(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& z
   uint64_t s = fx_rinv3(fx_r2(dx, dy, dz, fx_pair(row.e_lo, row.e_hi)));
   uint32_t p = row.p;
   if (MASS) {
-    s <<= 2;
-    const uint64_t m = fx_mad(fx_lo(s), j.mu_hi, fx_mul(fx_hi(s), j.mu_lo));
-    s = fx_mad(fx_hi(s), j.mu_hi, fx_pair(fx_hi(m), 0));  // S mass 2^(-em - q - 1)
+    s = fx_mul_hi(s << 2, fx_pair(j.mu_lo, j.mu_hi));  // S mass 2^(-em - q - 1)
     const int t = 2 * k + j.q;
     if (t < 0) s = t > -63 ? (s + (1ull << (-t - 1))) >> -t : 0;
     p = k <= kFxMaxK ? 1u << (t > 0 ? t : 0) : 0u;
@@ -359,9 +371,35 @@ GB_HD int fx_term(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& z
   return k;
 }
 
+// One term of the potential, [mass] / sqrt(|d|^2 + eps^2), into a.h and a.l.
+template <bool MASS>
+GB_HD int fx_term_pot(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& zi, float eps2f,
+                      const FxRow* tab, FxAcc& a) {
+  const Fx96 ux = fx_sub(j.x, xi), uy = fx_sub(j.y, yi), uz = fx_sub(j.z, zi);
+  const int k = fx_norm(ux, uy, uz, eps2f);
+  const FxRow row = tab[k];
+  const FxDiff dx = fx_scale(ux, k), dy = fx_scale(uy, k), dz = fx_scale(uz, k);
+  uint64_t y = fx_rinv1(fx_r2(dx, dy, dz, fx_pair(row.e_lo, row.e_hi)));
+  int t = k;
+  if (MASS) {
+    y = fx_mul_hi(y, fx_pair(j.mu_lo, j.mu_hi));  // y mass 2^(-em - q - 3)
+    t += j.q;
+    if (t < 0) {
+      y = t > -63 ? (y + (1ull << (-t - 1))) >> -t : 0;
+      t = 0;
+    }
+  }
+  const uint32_t p = k <= kFxMaxK ? 1u << t : 0u;
+  a.h = (long long)fx_mad(fx_hi(y), p, (uint64_t)a.h);
+  a.l = fx_mad(fx_lo(y), p, a.l);
+  return k;
+}
+
 // exponent of a term's unit: sum 2^(fx_out_exp(ex)) is the sum of d / r^3, and
-// sum 2^(fx_out_exp(ex) + em + 1) that of mass d / r^3
+// sum 2^(fx_out_exp(ex) + em + 1) that of mass d / r^3; of the potential:
+// 1 / r, and with em + 3 mass / r
 GB_HD int fx_out_exp(int ex) { return -60 - 2 * ex; }
+GB_HD int fx_out_exp_pot(int ex) { return -63 - ex; }
 
 // eps^2 in units of (2^64 U)^2
 GB_HD float fx_eps2f(double eps2, int ex) {

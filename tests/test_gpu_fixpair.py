@@ -72,3 +72,21 @@ def test_rhs_f64_not_finite(gb, torch_cuda, bad, pair):
         np.testing.assert_array_equal(np.isnan(got), np.isnan(ref))
     assert np.isnan(got[3 * n + 3 * 77 + 1])
     np.testing.assert_array_equal(got[: 3 * n], x[3 * n:])
+
+
+@pytest.mark.parametrize("kind", ["plain", "far from the origin", "masses", "close pairs",
+                                  "one far body", "tiny", "grid"])
+@pytest.mark.parametrize("n", [2, 31, 33, 129, 517])
+def test_potential_energy_against_extended_precision(gb, torch_cuda, kind, n):
+    """The potential energy within 24 2^-53 of itself (its terms have one sign): a term is within
+    2^-55 (fixed point) or 4 2^-53 (FP64), a CTA's sum per body exact in fixed point; the sums
+    over 8 ranks, 128 bodies (tree) and the tiles, the masses and a half are rounded."""
+    x, soft, m = _system(kind, n)
+    p = x[: 3 * n].reshape(n, 3).astype(np.longdouble)
+    ml = np.full(n, np.longdouble(1.0 / n)) if m is None else m.astype(np.longdouble)
+    d = p[None, :, :] - p[:, None, :]
+    r = np.sqrt((d * d).sum(2) + np.longdouble(soft * soft))
+    np.fill_diagonal(r, np.inf)
+    ref = -0.5 * (ml[:, None] * ml[None, :] / r).sum()
+    e = gb.energy(x, n, soft, 1.0 / n, None if m is None else gb.to_device(m))
+    assert abs(e["pe"] - ref) <= 24 * 2.0 ** -53 * abs(ref), float((e["pe"] - ref) / ref * 2 ** 53)

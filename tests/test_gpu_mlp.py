@@ -101,3 +101,40 @@ def test_training_lowers_loss(gb, torch_cuda):
     m0, loss0 = learned.train(x, y, epochs=1, lr=1e-3)
     m1, loss1 = learned.train(x, y, epochs=600, lr=3e-3)
     assert loss1 < 0.2 * loss0, (loss0, loss1)
+
+
+@pytest.mark.parametrize("B", [1, 4, 9, 609, 2001])
+def test_training_epochs_equal_the_single_passes(gb, torch_cuda, B):
+    """gb_mlp_train's three kernels per epoch against forward, backward and Adam called one by
+    one: batches of one sample, of part of a CTA, and of slices with and without a remainder.
+    The gradients' FP64 sums differ in their order only, so a rounded gradient differs by at
+    most 2^-23 of itself and a step of 3 by lr 2^-20."""
+    torch, L = torch_cuda, gb.lib()
+    rng = np.random.default_rng(B)
+    x = torch.as_tensor(rng.normal(size=(B, 16)).astype(np.float32), device="cuda")
+    target = rng.normal(size=B).astype(np.float32)
+    td = torch.as_tensor(target, device="cuda")
+    lr, over, epochs = 1e-3, 3.0, 3
+    w = _dev(torch, _mlp(gb, 5))
+    ref = w.clone()
+    loss = C.c_float(0)
+    assert L.gb_mlp_train(w.data_ptr(), x.data_ptr(), td.data_ptr(), B, epochs, lr, over,
+                          C.byref(loss), None) == 0
+    y = torch.empty(B, dtype=torch.float32, device="cuda")
+    act = torch.empty(L.gb_mlp_act_floats(B), dtype=torch.float32, device="cuda")
+    work = torch.empty(L.gb_mlp_backward_workspace_bytes(B), dtype=torch.uint8, device="cuda")
+    G, M, V = (torch.zeros(C.sizeof(gb.GbMlp), dtype=torch.uint8, device="cuda")
+               for _ in range(3))
+    for step in range(1, epochs + 1):
+        assert L.gb_mlp_forward_f32(ref.data_ptr(), x.data_ptr(), y.data_ptr(), B, act.data_ptr(),
+                                    None) == 0
+        r = y.cpu().numpy() - target
+        wt = np.where(r > 0, np.float32(over), np.float32(1))
+        dy = torch.as_tensor(np.float32(2) * wt * r / np.float32(B), device="cuda")
+        assert L.gb_mlp_backward_f32(ref.data_ptr(), x.data_ptr(), act.data_ptr(), dy.data_ptr(),
+                                     G.data_ptr(), B, work.data_ptr(), None) == 0
+        assert L.gb_mlp_adam_step(ref.data_ptr(), G.data_ptr(), M.data_ptr(), V.data_ptr(), lr,
+                                  0.9, 0.999, 1e-8, step, None) == 0
+    a, b = (np.frombuffer(t.cpu().numpy().tobytes(), dtype=np.float32) for t in (w, ref))
+    np.testing.assert_allclose(a, b, rtol=2.0 ** -22, atol=epochs * lr * 2.0 ** -20)
+    assert np.isfinite(loss.value)

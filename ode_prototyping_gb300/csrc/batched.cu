@@ -400,7 +400,8 @@ __global__ void batch_elem_kernel(const BatchParams P, int mode, const double* _
     const double d0 = d[3 * k], d1 = d[3 * k + 1];
     dt0 = (d0 < 1.0e-5 || d1 < 1.0e-5) ? 1.0e-6 : 0.01 * (d0 / d1);
   }
-  for (long long e = threadIdx.x; e < nv; e += blockDim.x) {
+  for (long long e = blockIdx.y * (long long)blockDim.x + threadIdx.x; e < nv;
+       e += (long long)gridDim.y * blockDim.x) {
     const long long g = sy.var_off + e;
     if (mode == 0) {
       out[g] = dadd(dmul(fabs(a[g]), sy.rtol), sy.atol);
@@ -412,23 +413,43 @@ __global__ void batch_elem_kernel(const BatchParams P, int mode, const double* _
   }
 }
 
-// Per-system RMS norm of v / s: one warp per system, fixed order.
-__global__ void batch_norm_kernel(const BatchParams P, const double* __restrict__ v,
-                                  const double* __restrict__ s, double* __restrict__ out,
-                                  int slot) {
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int k = blockIdx.x * 4 + warp;
-  if (k >= P.n_sys) return;
+// Per-system RMS norm of v / s in a fixed order: a cluster of 4 CTAs per
+// system, thread sums, a tree per CTA, then the CTAs in rank order.  Bound by
+// the FP64 pipe (an IEEE division, a multiply and an add an element): one warp
+// per system left a 4096-body system 280 us on one sub-partition.
+constexpr int kNormCtas = 4, kNormThreads = 256;
+__global__ void __cluster_dims__(kNormCtas, 1, 1) __launch_bounds__(kNormThreads)
+    batch_norm_kernel(const BatchParams P, const double* __restrict__ v,
+                      const double* __restrict__ s, double* __restrict__ out, int slot) {
+  __shared__ double red[kNormThreads];
+  __shared__ double part;
+  const int k = blockIdx.x / kNormCtas, rank = blockIdx.x % kNormCtas;
   const BSys sy = P.sys[k];
   const long long nv = 6 * sy.n;
   double acc = 0.0;
-  for (long long e = lane; e < nv; e += 32) {
+  for (long long e = rank * kNormThreads + threadIdx.x; e < nv; e += kNormCtas * kNormThreads) {
     const double q = __ddiv_rn(v[sy.var_off + e], s[sy.var_off + e]);
     acc = dadd(acc, dmul(q, q));
   }
-#pragma unroll
-  for (int off = 16; off >= 1; off /= 2) acc = dadd(acc, __shfl_xor_sync(0xffffffffu, acc, off));
-  if (lane == 0) out[3 * k + slot] = sqrt(acc / (double)nv);
+  const double sum = group_sum<kNormThreads>(acc, red, WholeCta{});
+  if (threadIdx.x == 0) part = sum;
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  if (rank == 0 && threadIdx.x == 0) {
+    double t = part;
+    for (int r = 1; r < kNormCtas; ++r) t = dadd(t, *cl.map_shared_rank(&part, r));
+    out[3 * k + slot] = sqrt(t / (double)nv);
+  }
+  cl.sync();
+}
+
+// The systems' current states, one after the other.
+__global__ void batch_state_kernel(const BatchParams P, double* __restrict__ x) {
+  const BSys sy = P.sys[blockIdx.x];
+  const double* r = P.ring + (long long)P.ctrl[blockIdx.x].cur * P.total_var;
+  for (long long e = blockIdx.y * (long long)blockDim.x + threadIdx.x; e < 6 * sy.n;
+       e += (long long)gridDim.y * blockDim.x)
+    x[sy.var_off + e] = r[sy.var_off + e];
 }
 
 __global__ void batch_init_ctrl_kernel(const BatchParams P, const double* __restrict__ d,
@@ -513,7 +534,8 @@ bool pick_batch(int prec, int T, int L, int BPT, int G, BatchKernels* k) {
   GB_BK(GB_PREC_MIXED, 128, 1, 2, 4) GB_BK(GB_PREC_MIXED, 128, 2, 2, 2)
   GB_BK(GB_PREC_MIXED, 64, 1, 1, 2)
   GB_BK(GB_PREC_F64, 128, 1, 1, 1) GB_BK(GB_PREC_F64, 128, 2, 1, 1)
-  GB_BK(GB_PREC_F64, 128, 4, 1, 1) GB_BK(GB_PREC_F64, 64, 1, 1, 1)
+  GB_BK(GB_PREC_F64, 128, 4, 1, 1) GB_BK(GB_PREC_F64, 128, 8, 1, 1)
+  GB_BK(GB_PREC_F64, 64, 1, 1, 1)
   GB_BK(GB_PREC_F64, 64, 2, 1, 1)
   GB_BK(GB_PREC_F64, 128, 1, 1, 2) GB_BK(GB_PREC_F64, 128, 1, 1, 4)
   GB_BK(GB_PREC_F64, 128, 2, 1, 2) GB_BK(GB_PREC_F64, 64, 1, 1, 2)
@@ -792,9 +814,9 @@ extern "C" int gb_batch_create(const gb_tableau* tab, int32_t n_sys, const int64
     for (long long i = 0; i < b->n[k]; ++i) body_sys.push_back(k);
   }
   b->total_var = 6 * b->total_bodies;
-  // the smallest tile any candidate geometry uses is 32 bodies
+  // the smallest tile any candidate geometry uses is 16 bodies
   b->max_units = 0;
-  for (int k = 0; k < n_sys; ++k) b->max_units += (b->n[k] + 31) / 32;
+  for (int k = 0; k < n_sys; ++k) b->max_units += (b->n[k] + 15) / 16;
   const long long tv = b->total_var, tb = b->total_bodies;
   cudaError_t e = cudaSuccess;
   auto alloc = [&](void** p, size_t bytes) {
@@ -864,7 +886,17 @@ extern "C" int gb_batch_create(const gb_tableau* tab, int32_t n_sys, const int64
     P.mlp = b->mlp_dev;
   }
   const int T = opts.tiling.threads_per_cta > 0 ? opts.tiling.threads_per_cta : 128;
-  const int L = opts.tiling.lanes > 0 ? opts.tiling.lanes : 2;
+  // Lanes per body.  FP64: as many as leave up to 10 CTAs (8 lanes) or 27 CTAs
+  // (4) per SM, so that few or small systems fill the GPU: 24 systems of 64 to
+  // 1024 bodies 55 us a stage with 8 lanes against 108 with 2, 128 systems of
+  // 64 to 4096 1.66 ms with 4 against 1.77; above that 2 (512 systems 6.30 ms
+  // against 6.42 with 4).
+  int L = opts.tiling.lanes;
+  if (L <= 0) {
+    L = 2;
+    if (opts.precision == GB_PREC_F64 && T == 128 && opts.tiling.systems_per_cta <= 1)
+      L = tb * 8 <= 128LL * 10 * num_sms() ? 8 : (tb * 4 <= 128LL * 27 * num_sms() ? 4 : 2);
+  }
   const int BPT = opts.precision == GB_PREC_F64
                       ? 1
                       : (opts.tiling.bodies_per_thread > 0 ? opts.tiling.bodies_per_thread : 1);
@@ -905,16 +937,16 @@ extern "C" int gb_batch_start(gb_batch b, const double* x0, const double* t0, co
   double* x1 = b->Y + tv;
   double* f0 = b->ks;
   double* df = b->ks + tv;
-  batch_elem_kernel<<<ns, 256, 0, s>>>(P, 0, b->ring, nullptr, tg, nullptr);
+  batch_elem_kernel<<<dim3(ns, 4), 256, 0, s>>>(P, 0, b->ring, nullptr, tg, nullptr);
   GB_TRY(launch_rhs(b, b->ring, b->PX, f0));
-  batch_norm_kernel<<<(ns + 3) / 4, 128, 0, s>>>(P, b->ring, tg, b->dscal, 0);
-  batch_norm_kernel<<<(ns + 3) / 4, 128, 0, s>>>(P, f0, tg, b->dscal, 1);
-  batch_elem_kernel<<<ns, 256, 0, s>>>(P, 1, b->ring, f0, x1, b->dscal);
+  batch_norm_kernel<<<ns * kNormCtas, kNormThreads, 0, s>>>(P, b->ring, tg, b->dscal, 0);
+  batch_norm_kernel<<<ns * kNormCtas, kNormThreads, 0, s>>>(P, f0, tg, b->dscal, 1);
+  batch_elem_kernel<<<dim3(ns, 4), 256, 0, s>>>(P, 1, b->ring, f0, x1, b->dscal);
   if (b->opts.precision == GB_PREC_MIXED)
     batch_pack_kernel<<<(unsigned)((tb + 255) / 256), 256, 0, s>>>(P, x1, b->PY);
   GB_TRY(launch_rhs(b, x1, b->PY, df));
-  batch_elem_kernel<<<ns, 256, 0, s>>>(P, 2, nullptr, f0, df, nullptr);
-  batch_norm_kernel<<<(ns + 3) / 4, 128, 0, s>>>(P, df, tg, b->dscal, 2);
+  batch_elem_kernel<<<dim3(ns, 4), 256, 0, s>>>(P, 2, nullptr, f0, df, nullptr);
+  batch_norm_kernel<<<ns * kNormCtas, kNormThreads, 0, s>>>(P, df, tg, b->dscal, 2);
   const int q = std::min(b->htab.p, b->htab.pt);
   const double safety = std::pow(0.38, 1.0 / (1.0 + q));
   batch_init_ctrl_kernel<<<(ns + 127) / 128, 128, 0, s>>>(P, b->dscal, b->tv, b->tv + ns,
@@ -996,17 +1028,12 @@ extern "C" int gb_batch_stats(gb_batch b, gb_integrate_stats* totals, gb_integra
 extern "C" int gb_batch_state(gb_batch b, double* x_dev, double* t_host) {
   if (!b || !b->started) return GB_ERR_INVALID_ARGUMENT;
   GB_TRY(read_ctrl(b));
-  std::vector<BSys> hs(b->n_sys);
-  GB_CUDA_TRY(cudaMemcpy(hs.data(), b->sys, b->n_sys * sizeof(BSys), cudaMemcpyDeviceToHost));
-  for (int k = 0; k < b->n_sys; ++k) {
-    const Ctrl& c = b->hctrl[k];
-    if (x_dev)
-      GB_CUDA_TRY(cudaMemcpyAsync(x_dev + hs[k].var_off,
-                                  b->ring + (long long)c.cur * b->total_var + hs[k].var_off,
-                                  6 * hs[k].n * sizeof(double), cudaMemcpyDeviceToDevice,
-                                  b->stream));
-    if (t_host) t_host[k] = c.t;
+  if (x_dev) {
+    batch_state_kernel<<<dim3(b->n_sys, 4), 256, 0, b->stream>>>(b->P, x_dev);
+    GB_CUDA_TRY(cudaGetLastError());
   }
+  if (t_host)
+    for (int k = 0; k < b->n_sys; ++k) t_host[k] = b->hctrl[k].t;
   GB_CUDA_TRY(cudaStreamSynchronize(b->stream));
   return GB_OK;
 }
@@ -1043,8 +1070,8 @@ extern "C" int gb_batch_autotune(gb_batch b, int32_t reps, gb_batch_tiling* chos
                          {128, 1, 2, 4}, {128, 2, 2, 2}, {64, 1, 1, 2}};
     for (auto& t : tl) add(t[0], t[1], t[2], t[3]);
   } else {
-    const int tl[][4] = {{128, 1, 1, 1}, {128, 2, 1, 1}, {128, 4, 1, 1}, {64, 1, 1, 1},
-                         {64, 2, 1, 1},  {128, 1, 1, 2}, {128, 1, 1, 4}, {128, 2, 1, 2},
+    const int tl[][4] = {{128, 1, 1, 1}, {128, 2, 1, 1}, {128, 4, 1, 1}, {128, 8, 1, 1},
+                         {64, 1, 1, 1},  {64, 2, 1, 1},  {128, 1, 1, 2}, {128, 1, 1, 4}, {128, 2, 1, 2},
                          {64, 1, 1, 2}};
     for (auto& t : tl) add(t[0], t[1], t[2], t[3]);
   }

@@ -56,30 +56,77 @@ __global__ void __launch_bounds__(T) rhs_f64_kernel(const double* __restrict__ p
   }
 }
 
-__global__ void centroid_kernel(const double* __restrict__ pos, long long n, double* c_out) {
-  __shared__ double sh[3][1024];
-  double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-    s0 += pos[3 * i];
-    s1 += pos[3 * i + 1];
-    s2 += pos[3 * i + 2];
+__device__ __forceinline__ PackedBody pack_row(const double* __restrict__ pos,
+                                               const double* __restrict__ masses, double cx,
+                                               double cy, double cz, long long i) {
+  const float w = masses ? (float)masses[i] : 1.0f;
+  return pack_body(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], cx, cy, cz, w);
+}
+
+// Centroid of n bodies: 1024 chains (body t, t + 1024, ... added in order), then
+// a tree over the chains.  Bound by the FP64 pipe, 3 n adds: one CTA of 1024
+// threads took 9.4 us at N = 4096 and 93 us at 100003, so a cluster of 8 CTAs
+// holds 128 chains each and its first CTA, thread t with chains t, t + 128, ...,
+// runs the tree, the same additions.  PACK: the cluster then packs the
+// bodies itself (it saves the launch of the packing kernel; up to
+// kFusedPackBodies, where eight SMs are as fast as a launch).
+constexpr int kCentroidCtas = 8;
+constexpr long long kFusedPackBodies = 4096;
+template <bool PACK>
+__global__ void __cluster_dims__(kCentroidCtas, 1, 1) __launch_bounds__(128)
+    centroid_kernel(const double* __restrict__ pos, const double* __restrict__ masses, long long n,
+                    double* c_out, PackedBody* out) {
+  __shared__ double chain[3][128];
+  __shared__ double cen[3];
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank(), t = threadIdx.x;
+  double v[3] = {0.0, 0.0, 0.0};
+#pragma unroll 4
+  for (long long i = rank * 128 + t; i < n; i += 1024) {
+    v[0] += pos[3 * i];
+    v[1] += pos[3 * i + 1];
+    v[2] += pos[3 * i + 2];
   }
-  sh[0][threadIdx.x] = s0;
-  sh[1][threadIdx.x] = s1;
-  sh[2][threadIdx.x] = s2;
-  __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st /= 2) {
-    if ((int)threadIdx.x < st) {
-      sh[0][threadIdx.x] += sh[0][threadIdx.x + st];
-      sh[1][threadIdx.x] += sh[1][threadIdx.x + st];
-      sh[2][threadIdx.x] += sh[2][threadIdx.x + st];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) chain[c][t] = v[c];
+  cl.sync();
+  if (rank == 0) {
+    double w[3][8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const double(*rc)[128] = cl.map_shared_rank(chain, r);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) w[c][r] = rc[c][t];
     }
+#pragma unroll
+    for (int st = 4; st >= 1; st /= 2)  // chains 512, 256 and 128 apart
+#pragma unroll
+      for (int r = 0; r < st; ++r)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) w[c][r] += w[c][r + st];
     __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 3; ++c) chain[c][t] = w[c][0];
+    __syncthreads();
+    for (int st = 64; st > 0; st /= 2) {
+      if (t < st) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) chain[c][t] += chain[c][t + st];
+      }
+      __syncthreads();
+    }
+    if (t < 3) {
+      cen[t] = chain[t][0] / (double)n;
+      c_out[t] = cen[t];
+    }
   }
-  if (threadIdx.x == 0) {
-    c_out[0] = sh[0][0] / (double)n;
-    c_out[1] = sh[1][0] / (double)n;
-    c_out[2] = sh[2][0] / (double)n;
+  cl.sync();
+  if (PACK) {
+    const double* c = cl.map_shared_rank(cen, 0);
+    const double cx = c[0], cy = c[1], cz = c[2];
+    for (long long i = rank * 128 + t; i < n; i += 1024)
+      out[i] = pack_row(pos, masses, cx, cy, cz, i);
+    cl.sync();  // rank 0's centroid stays until every CTA has read it
   }
 }
 
@@ -87,17 +134,18 @@ __global__ void pack_kernel(const double* __restrict__ pos, const double* __rest
                             const double* __restrict__ c, long long n, PackedBody* out) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const float w = masses ? (float)masses[i] : 1.0f;
-  out[i] = pack_body(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], c[0], c[1], c[2], w);
+  out[i] = pack_row(pos, masses, c[0], c[1], c[2], i);
 }
 
+// Registers: the one-lane packed loop (large systems) runs fastest with 56, 9
+// CTAs of 128 threads on an SM (N = 100003 4.62 ms; 4.68 at 8, 4.80 at 10, 4.87
+// at 5, 5.2 at 6 and 7; the same order at 16384 and 65536), the other forms,
+// whose launches are shorter, with what 5 CTAs leave.
 template <int T, int L, int BPT, bool PACKED>
-__global__ void __launch_bounds__(T) rhs_mixed_kernel(const PackedBody* __restrict__ packed,
-                                                      const double* __restrict__ vel,
-                                                      double* __restrict__ out_vel,
-                                                      double* __restrict__ out_acc,
-                                                      long long n, float eps2, double mass,
-                                                      int uniform_mass) {
+__global__ void __launch_bounds__(T, (PACKED && L == 1 && BPT == 1 ? 9 : 5) * 128 / T)
+    rhs_mixed_kernel(const PackedBody* __restrict__ packed, const double* __restrict__ vel,
+                     double* __restrict__ out_vel, double* __restrict__ out_acc, long long n,
+                     float eps2, double mass, int uniform_mass) {
   constexpr int BI = (T / L) * BPT;
   constexpr int SH = PACKED ? jp_smem_bytes<T>() : (int)sizeof(PackedBody) * T;
   __shared__ __align__(16) unsigned char sh_raw[SH];
@@ -279,6 +327,12 @@ ForceGeom choose_geom(long long n, int precision, const gb_force_tiling* tiling,
       while (L < 8 && (long long)L * 2 * n <= 32768) L *= 2;
       g.P = 8;
       g.L = L;
+    } else if (n < 768) {
+      // a few pairs a lane: lanes rather than ranks (fixed-point terms, N = 257
+      // 12.6 us against 14.9 with 8 ranks x 4 lanes, 512 12.5 against 16.8, 1024
+      // 17.1 against 16.8)
+      g.P = 4;
+      g.L = 8;
     } else {
       // Aim for ~8 resident warps per SM over the whole grid.
       long long want = (long long)sms * 8 * 32;
@@ -355,9 +409,13 @@ namespace gb {
 int mixed_rhs_into(const double* x, double* dxdt, long long n, double softening, double mass,
                    const double* masses, PackedBody* packed, double* c,
                    const gb_force_tiling* tiling, cudaStream_t s) {
-  centroid_kernel<<<1, 1024, 0, s>>>(x, n, c);
-  GB_CUDA_TRY(cudaGetLastError());
-  pack_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(x, masses, c, n, packed);
+  if (n <= kFusedPackBodies) {
+    centroid_kernel<true><<<kCentroidCtas, 128, 0, s>>>(x, masses, n, c, packed);
+  } else {
+    centroid_kernel<false><<<kCentroidCtas, 128, 0, s>>>(x, nullptr, n, c, nullptr);
+    GB_CUDA_TRY(cudaGetLastError());
+    pack_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(x, masses, c, n, packed);
+  }
   GB_CUDA_TRY(cudaGetLastError());
   ForceGeom g = choose_geom(n, GB_PREC_MIXED, tiling, 0, masses == nullptr);
   const void* k = nullptr;
@@ -467,7 +525,7 @@ extern "C" int gb_nbody_rhs_mixed_sorted(const double* x, double* dxdt, int64_t 
   SortedWork w = sorted_layout(n, work);
   if (work_bytes < w.total) return GB_ERR_CAPACITY;
   cudaStream_t s = as_cuda(stream);
-  centroid_kernel<<<1, 1024, 0, s>>>(x, n, w.cref);
+  centroid_kernel<false><<<kCentroidCtas, 128, 0, s>>>(x, nullptr, n, w.cref, nullptr);
   GB_CUDA_TRY(cudaGetLastError());
   const long long nt = (n + 127) / 128;
   GB_TRY(sort_and_pack(x, nullptr, 0, n, w.sb, masses, w.cref, w.near, w.far, w.meta, nullptr,

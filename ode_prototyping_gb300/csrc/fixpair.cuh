@@ -311,15 +311,19 @@ GB_HD double fx_to_double(__int128 v, int sc) {
 }
 
 // Row k of the softening table on the grid of ex: eps^2 in units of (2^64 U)^2
-// times 4^k (the 2 is the mean of what fx_r2 drops), 4^k as the weight.
+// times 4^k, truncated (the 2 is the mean of what fx_r2 drops), 4^k as the
+// weight.  A row whose eps^2 does not fit is never read: R would exceed 2^62.
 GB_HD FxRow fx_row(int k, double eps2, int ex) {
 #ifdef __CUDA_ARCH__
-  const double v = scalbn(eps2, 2 * (30 - ex + k));
-  const uint64_t e = (v < 4.6e18 ? (uint64_t)__double2ull_rn(v) : 1ull << 62) + 2;
+  const uint64_t bits = (uint64_t)__double_as_longlong(eps2);
 #else
-  const double v = __builtin_scalbn(eps2, 2 * (30 - ex + k));
-  const uint64_t e = (v < 4.6e18 ? (uint64_t)(v + 0.5) : 1ull << 62) + 2;
+  uint64_t bits;
+  memcpy(&bits, &eps2, 8);
 #endif
+  const int ee = (int)(bits >> 52);  // eps^2 >= 0; subnormals count as zero
+  const uint64_t m = ee ? (bits & 0xfffffffffffffull) | (1ull << 52) : 0;
+  const int sh = ee - 1075 + 2 * (30 - ex + k);
+  const uint64_t e = (sh > 9 ? 1ull << 62 : sh >= 0 ? m << sh : sh > -64 ? m >> -sh : 0) + 2;
   return FxRow{(uint32_t)e, (uint32_t)(e >> 32), k <= kFxMaxK ? 1u << (2 * k) : 0u, 0u};
 }
 
@@ -403,11 +407,8 @@ GB_HD int fx_out_exp_pot(int ex) { return -63 - ex; }
 
 // eps^2 in units of (2^64 U)^2
 GB_HD float fx_eps2f(double eps2, int ex) {
-#ifdef __CUDA_ARCH__
-  return (float)scalbn(eps2, 2 * (30 - ex));
-#else
-  return (float)__builtin_scalbn(eps2, 2 * (30 - ex));
-#endif
+  const FxRow r = fx_row(0, eps2, ex);  // at most 2^58 and its first row
+  return (float)fx_pair(r.e_lo, r.e_hi);
 }
 
 }  // namespace gb

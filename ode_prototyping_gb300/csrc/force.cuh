@@ -64,6 +64,28 @@ __device__ __forceinline__ double lane_reduce(double v) {
   return v;
 }
 
+// Sum over the cluster's ranks of element e of their part arrays, in rank order
+// 0, 1, ..., size - 1.  Up to 8 ranks' values are loaded together before the
+// first addition (one after the other, each load waited for the addition
+// before it: 2 us of a small system's launch).
+__device__ __forceinline__ double cluster_sum(cg::cluster_group cl, const double* part, int e,
+                                              int size) {
+  if (size > 8) {
+    double s = cl.map_shared_rank(part, 0)[e];
+    for (int r = 1; r < size; ++r) s = dadd(s, cl.map_shared_rank(part, r)[e]);
+    return s;
+  }
+  double v[8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r)
+    if (r < size) v[r] = cl.map_shared_rank(part, r)[e];
+  double s = v[0];
+#pragma unroll
+  for (int r = 1; r < 8; ++r)
+    if (r < size) s = dadd(s, v[r]);
+  return s;
+}
+
 // Cluster-wide combine of per-body partials part[BI][3] held in each CTA's
 // shared memory; on return rank 0's part holds the totals (ranks added in
 // order 0, 1, ..., P-1).  All threads of all CTAs of the cluster must call it.
@@ -72,18 +94,8 @@ __device__ __forceinline__ void cluster_combine(double (*part)[3], int rank, int
   cg::cluster_group cl = cg::this_cluster();
   cl.sync();
   if (rank == 0 && size > 1) {
-    for (int b = threadIdx.x; b < BI; b += blockDim.x) {
-      double s0 = part[b][0], s1 = part[b][1], s2 = part[b][2];
-      for (int r = 1; r < size; ++r) {
-        double(*rp)[3] = cl.map_shared_rank(part, r);
-        s0 = dadd(s0, rp[b][0]);
-        s1 = dadd(s1, rp[b][1]);
-        s2 = dadd(s2, rp[b][2]);
-      }
-      part[b][0] = s0;
-      part[b][1] = s1;
-      part[b][2] = s2;
-    }
+    double* p = &part[0][0];
+    for (int e = threadIdx.x; e < 3 * BI; e += blockDim.x) p[e] = cluster_sum(cl, p, e, size);
   }
   cl.sync();
 }
@@ -101,19 +113,9 @@ __device__ __forceinline__ void cluster_combine_rows(double (*part)[3], int rank
   if (size > 1) {
     const int R = (BI + size - 1) / size;
     const int lo = rank * R, hi = min(BI, lo + R);
-    double(*p0)[3] = cl.map_shared_rank(part, 0);
-    for (int b = lo + (int)threadIdx.x; b < hi; b += blockDim.x) {
-      double s0 = p0[b][0], s1 = p0[b][1], s2 = p0[b][2];
-      for (int r = 1; r < size; ++r) {
-        double(*rp)[3] = cl.map_shared_rank(part, r);
-        s0 = dadd(s0, rp[b][0]);
-        s1 = dadd(s1, rp[b][1]);
-        s2 = dadd(s2, rp[b][2]);
-      }
-      part[b][0] = s0;
-      part[b][1] = s1;
-      part[b][2] = s2;
-    }
+    double* p = &part[0][0];
+    for (int e = 3 * lo + (int)threadIdx.x; e < 3 * hi; e += blockDim.x)
+      p[e] = cluster_sum(cl, p, e, size);
   }
   cl.sync();
 }
@@ -251,7 +253,7 @@ __device__ __noinline__ void force_fx_tiles(const double* __restrict__ pos, long
   const float eps2f = fx_eps2f(eps2, ex);
   __int128 tot[NC] = {};
   double near[NC] = {};
-  bool in_f64 = false;  // uniform in the warp
+  bool in_f64 = false, any_near = false;  // uniform in the warp
   for (long long j0 = jb; j0 < je; j0 += T) {
     const int cnt = (int)min((long long)T, je - j0);
     group_bar(bar, T);
@@ -306,23 +308,30 @@ __device__ __noinline__ void force_fx_tiles(const double* __restrict__ pos, long
         // an FP64 term costs 5 fixed-point ones: where a lane needs more than 4
         // in 5 of its terms in FP64, the others' are not worth their time
         in_f64 = in_f64 || rounds > kFxChunk * 4 / 5;
+        any_near = any_near || rounds > 0;
       }
     }
   }
   const int sc = POT ? fx_out_exp_pot(ex) + (MASS ? em + 3 : 0)
                      : fx_out_exp(ex) + (MASS ? em + 1 : 0);
+  for (int off = L / 2; off >= 1; off /= 2) {
 #pragma unroll
-  for (int d = 0; d < NC; ++d) {
-    __int128 v = tot[d];
-    double s = near[d];
-    for (int off = L / 2; off >= 1; off /= 2) {
-      const unsigned long long lo = __shfl_down_sync(0xffffffffu, (unsigned long long)v, off);
+    for (int d = 0; d < NC; ++d) {
+      const unsigned long long lo =
+          __shfl_down_sync(0xffffffffu, (unsigned long long)tot[d], off);
       const unsigned long long hi =
-          __shfl_down_sync(0xffffffffu, (unsigned long long)(v >> 64), off);
-      v += (__int128)(((unsigned __int128)hi << 64) | lo);
-      s = dadd(s, __shfl_down_sync(0xffffffffu, s, off));
+          __shfl_down_sync(0xffffffffu, (unsigned long long)(tot[d] >> 64), off);
+      tot[d] += (__int128)(((unsigned __int128)hi << 64) | lo);
+      if (any_near) near[d] = dadd(near[d], __shfl_down_sync(0xffffffffu, near[d], off));
     }
-    if (l == 0) part[b][d] = dadd(fx_to_double(v, sc), s);
+  }
+  if (l == 0) {
+#pragma unroll
+    for (int d = 0; d < NC; ++d) {
+      double v = fx_to_double(tot[d], sc);
+      if (any_near) v = dadd(v, near[d]);
+      part[b][d] = v;
+    }
   }
 }
 

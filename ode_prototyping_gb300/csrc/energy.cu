@@ -2,33 +2,127 @@
 // Restates the softened potential energy and kinetic energy of
 // scripts/nbody_physics/energy.py:146-192 (PE = -sum_{i<j} m_i m_j /
 // sqrt(r^2 + eps^2), KE = sum m v^2 / 2; the reference has unit masses) with
-// masses, plus linear and angular momentum.  Owner-computes: body i sums
-// -m_j / sqrt(r_ij^2 + eps^2) over all j != i; PE = 1/2 sum_i m_i phi_i.
-// Deterministic: per-CTA tree sums, then CTA partials added in order.
+// masses, plus linear and angular momentum.  Deterministic: per-CTA tree sums,
+// then CTA partials added in order.
 //
-// The pair sum is bound by the FP64 pipe (IEEE square root and division: about
-// 23 operations a pair, 14.8 ms at N = 16384 with one CTA per 128 bodies), so
-// it runs in fixed point on the integer pipes (fixpair.cuh), the partners
-// split over the CTAs of a cluster; the FP64 loop is left for systems without a
-// fixed-point grid.
+// Each pair is taken once: body i has the partners i + 1, ..., i + h (modulo n),
+// h = (n - 1) / 2, and for even n the first half of the bodies i + n / 2 too, so
+// every body has the same share.  A CTA's 128 bodies i0 + b and the partners
+// i0 + v: the pair counts where 1 <= v - b <= h, which cuts off the corners of
+// the first and last 128 partners.
+//
+// The FP64 pair sum is bound by the FP64 pipe (IEEE square root and division,
+// about 23 operations a pair), so it runs in fixed point on the integer pipes
+// (fixpair.cuh), the partners split over the CTAs of a cluster; the FP64 loop is
+// left for systems without a fixed-point grid.  N = 16384: 14.8 ms with every
+// pair twice in FP64 on one CTA per 128 bodies, 1.13 ms in fixed point, 0.65
+// ms with each pair once.
 #include "force.cuh"
 
 namespace gb {
 namespace {
 
 constexpr int kT = 128;
-// CTAs of the pair kernel on an SM: N = 16384 1.21 ms at 5, 1.16 at 6, 1.13 at
-// 7, 1.16 at 8 (135 cycles of a sub-partition per 32 terms, ~95 instructions)
+// CTAs of the pair kernel on an SM: with every pair twice N = 16384 took 1.21 ms
+// at 5, 1.16 at 6, 1.13 at 7, 1.16 at 8 (135 cycles of a sub-partition per 32
+// terms, ~95 instructions)
 constexpr int kCtasPerSm = 7;
+
+// Body i's sum of [m_j] / r over its partners v in [vb, ve), in FP64.
+__device__ __noinline__ double pot_f64(const double* __restrict__ pos, long long n, long long i0,
+                                       long long vb, long long ve, long long span, double eps2,
+                                       const double* __restrict__ masses, double* sh) {
+  const int b = threadIdx.x;
+  const long long i = i0 + b;
+  double xi = 0, yi = 0, zi = 0, phi = 0.0;
+  if (i < n) {
+    xi = pos[3 * i];
+    yi = pos[3 * i + 1];
+    zi = pos[3 * i + 2];
+  }
+  for (long long v0 = vb; v0 < ve; v0 += kT) {
+    const int cnt = (int)min((long long)kT, ve - v0);
+    __syncthreads();
+    if (b < cnt) {
+      const long long j = (i0 + v0 + b) % n;
+      sh[4 * b] = pos[3 * j];
+      sh[4 * b + 1] = pos[3 * j + 1];
+      sh[4 * b + 2] = pos[3 * j + 2];
+      sh[4 * b + 3] = masses ? masses[j] : 1.0;
+    }
+    __syncthreads();
+    for (int k = 0; k < cnt; ++k) {
+      const long long d = v0 + k - b;
+      if (d < 1 || d > span) continue;
+      const double dx = sh[4 * k] - xi, dy = sh[4 * k + 1] - yi, dz = sh[4 * k + 2] - zi;
+      phi += sh[4 * k + 3] / sqrt(dx * dx + dy * dy + dz * dz + eps2);
+    }
+  }
+  return phi;
+}
+
+// The same in fixed point on the grid of ex; close pairs in FP64.
+template <bool MASS>
+__device__ __noinline__ double pot_fx(const double* __restrict__ pos, long long n, long long i0,
+                                      long long vb, long long ve, long long span, double eps2,
+                                      const double* __restrict__ masses, int ex, int em,
+                                      FxBody* rec, const FxRow* tab) {
+  const int b = threadIdx.x;
+  const long long i = min(i0 + b, n - 1);
+  const Fx96 xi = fx_from_double(pos[3 * i], ex), yi = fx_from_double(pos[3 * i + 1], ex),
+             zi = fx_from_double(pos[3 * i + 2], ex);
+  const float eps2f = fx_eps2f(eps2, ex);
+  __int128 tot = 0;
+  double near = 0.0;
+  for (long long v0 = vb; v0 < ve; v0 += kT) {
+    const int cnt = (int)min((long long)kT, ve - v0);
+    __syncthreads();
+    if (b < cnt) {
+      const long long j = (i0 + v0 + b) % n;
+      FxBody r;
+      r.x = fx_from_double(pos[3 * j], ex);
+      r.y = fx_from_double(pos[3 * j + 1], ex);
+      r.z = fx_from_double(pos[3 * j + 2], ex);
+      r.mu_lo = r.mu_hi = 0;
+      r.q = 0;
+      if (MASS) fx_mass(r, masses[j], em);
+      rec[b] = r;
+    }
+    __syncthreads();
+    // partner k counts where 0 <= k - first < span
+    const long long first = b + 1 - v0;
+    for (int c = 0; c < cnt; c += kFxChunk) {
+      const int end = min(cnt, c + kFxChunk);
+      unsigned mask = 0;
+      FxAcc a = {};
+#pragma unroll 2
+      for (int k = c; k < end; ++k) {
+        const bool on = (unsigned long long)(k - first) < (unsigned long long)span;
+        const int norm = fx_term_pot<MASS>(rec[k], xi, yi, zi, eps2f, tab, on, a);
+        mask = (mask << 1) | (on && norm > kFxMaxK ? 1u : 0u);
+      }
+      fx_fold(tot, a);
+      while (mask) {  // close pairs
+        const int k = end - 32 + __clz(mask);
+        mask &= ~(0x80000000u >> __clz(mask));
+        const long long j = (i0 + v0 + k) % n;
+        const double dx = pos[3 * j] - pos[3 * i], dy = pos[3 * j + 1] - pos[3 * i + 1],
+                     dz = pos[3 * j + 2] - pos[3 * i + 2];
+        near += (MASS ? masses[j] : 1.0) / sqrt(dx * dx + dy * dy + dz * dz + eps2);
+      }
+    }
+  }
+  return fx_to_double(tot, fx_out_exp_pot(ex) + (MASS ? em + 3 : 0)) + near;
+}
 
 __global__ void __launch_bounds__(kT, kCtasPerSm)
     energy_partial_kernel(const double* __restrict__ x, long long n, double eps2, double mass,
                           const double* __restrict__ masses, double* __restrict__ partial) {
   __shared__ __align__(16) unsigned char sh_raw[f64_smem_bytes<kT>()];
-  __shared__ double part[kT][3];
+  __shared__ double part[kT];
   __shared__ double red[8][kT];
   const ClusterInfo ci = cluster_info();
-  const long long i = ci.itile * kT + threadIdx.x;
+  const long long i0 = ci.itile * kT, i = i0 + threadIdx.x;
   const double* pos = x;
   const double* vel = x + 3 * n;
   double xi = 0, yi = 0, zi = 0;
@@ -37,39 +131,29 @@ __global__ void __launch_bounds__(kT, kCtasPerSm)
     yi = pos[3 * i + 1];
     zi = pos[3 * i + 2];
   }
-  long long jb, je;
-  j_chunk(n, ci.rank, ci.size, 32, jb, je);  // whole chunks of the fixed-point loop
-  if (!force_fx_group<true>(pos, n, ci.itile * kT, jb, je, eps2, masses, kF64Pot, sh_raw, part, kT,
-                            1, (int)threadIdx.x, 0)) {
-    double* sh = reinterpret_cast<double*>(sh_raw);
-    double phi = 0.0;
-    for (long long j0 = jb; j0 < je; j0 += kT) {
-      const int cnt = (int)min((long long)kT, je - j0);
-      __syncthreads();
-      for (int k = threadIdx.x; k < cnt; k += kT) {
-        sh[4 * k] = pos[3 * (j0 + k)];
-        sh[4 * k + 1] = pos[3 * (j0 + k) + 1];
-        sh[4 * k + 2] = pos[3 * (j0 + k) + 2];
-        sh[4 * k + 3] = masses ? masses[j0 + k] : 1.0;
-      }
-      __syncthreads();
-      if (i < n) {
-        for (int k = 0; k < cnt; ++k) {
-          if (j0 + k == i) continue;
-          const double dx = sh[4 * k] - xi, dy = sh[4 * k + 1] - yi, dz = sh[4 * k + 2] - zi;
-          phi += sh[4 * k + 3] / sqrt(dx * dx + dy * dy + dz * dz + eps2);
-        }
-      }
-    }
-    part[threadIdx.x][0] = phi;
+  const long long h = (n - 1) / 2, even = 1 - n % 2;
+  const long long span = i < n ? h + (even && i < n / 2 ? 1 : 0) : 0;  // partners of the body
+  long long vb, ve;
+  j_chunk(h + even + kT, ci.rank, ci.size, kFxChunk, vb, ve);
+  FxBody* rec = reinterpret_cast<FxBody*>(sh_raw);
+  FxRow* tab = reinterpret_cast<FxRow*>(rec + kT);
+  int ex, em;
+  if (fx_grid(pos, n, min(i, n - 1), (i0 + vb) % n, min(n, ve - vb), eps2, masses,
+              reinterpret_cast<int*>(tab + kFxRows), kT, threadIdx.x, 0, &ex, &em)) {
+    if (threadIdx.x < kFxRows) tab[threadIdx.x] = fx_row(threadIdx.x, eps2, ex);
+    part[threadIdx.x] =
+        masses ? pot_fx<true>(pos, n, i0, vb, ve, span, eps2, masses, ex, em, rec, tab)
+               : pot_fx<false>(pos, n, i0, vb, ve, span, eps2, nullptr, ex, 0, rec, tab);
+  } else {
+    part[threadIdx.x] = pot_f64(pos, n, i0, vb, ve, span, eps2, masses,
+                                reinterpret_cast<double*>(sh_raw));
   }
   // rank 0 adds the ranks' sums in rank order
   cg::cluster_group cl = cg::this_cluster();
   cl.sync();
   double phi = 0.0;
   if (ci.rank == 0) {
-    phi = part[threadIdx.x][0];
-    for (int r = 1; r < ci.size; ++r) phi += cl.map_shared_rank(part, r)[threadIdx.x][0];
+    phi = cluster_sum(cl, part, threadIdx.x, ci.size);
     if (!masses) phi *= mass;
     phi = -phi;
   }
@@ -80,7 +164,7 @@ __global__ void __launch_bounds__(kT, kCtasPerSm)
     const double mi = masses ? masses[i] : mass;
     const double vx = vel[3 * i], vy = vel[3 * i + 1], vz = vel[3 * i + 2];
     v[0] = 0.5 * mi * (vx * vx + vy * vy + vz * vz);
-    v[1] = 0.5 * mi * phi;
+    v[1] = mi * phi;
     v[2] = mi * vx;
     v[3] = mi * vy;
     v[4] = mi * vz;
@@ -98,13 +182,17 @@ __global__ void __launch_bounds__(kT, kCtasPerSm)
   if (threadIdx.x < 8) partial[ci.itile * 8 + threadIdx.x] = red[threadIdx.x][0];
 }
 
-__global__ void energy_final_kernel(const double* __restrict__ partial, int nb,
-                                    double* __restrict__ out) {
-  const int c = threadIdx.x;
-  if (c >= 8) return;
+// One warp per quantity: lanes over the CTAs' partials, then a tree (one thread
+// adding them one after the other waited for a load and an FP64 addition each).
+__global__ void __launch_bounds__(256)
+    energy_final_kernel(const double* __restrict__ partial, int nb, double* __restrict__ out) {
+  const int c = threadIdx.x / 32, lane = threadIdx.x % 32;
   double s = 0.0;
-  for (int b = 0; b < nb; ++b) s += partial[b * 8 + c];
-  out[c] = s;
+#pragma unroll 4
+  for (int b = lane; b < nb; b += 32) s += partial[b * 8 + c];
+#pragma unroll
+  for (int off = 16; off >= 1; off /= 2) s += __shfl_xor_sync(0xffffffffu, s, off);
+  if (lane == 0) out[c] = s;
 }
 
 }  // namespace
@@ -144,7 +232,7 @@ extern "C" int gb_nbody_energy_f64(const double* x, int64_t n, double softening,
   void* args[] = {(void*)&x, (void*)&nn, (void*)&eps2, (void*)&mass, (void*)&masses,
                   (void*)&partial};
   GB_TRY(launch_cluster((const void*)energy_partial_kernel, g, 0, s, args));
-  energy_final_kernel<<<1, 32, 0, s>>>(partial, nb, out_dev);
+  energy_final_kernel<<<1, 256, 0, s>>>(partial, nb, out_dev);
   GB_CUDA_TRY(cudaGetLastError());
   return GB_OK;
 }

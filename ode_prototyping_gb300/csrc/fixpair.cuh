@@ -375,10 +375,11 @@ GB_HD int fx_term(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& z
   return k;
 }
 
-// One term of the potential, [mass] / sqrt(|d|^2 + eps^2), into a.h and a.l.
+// One term of the potential, [mass] / sqrt(|d|^2 + eps^2), into a.h and a.l;
+// with weight 0 where `on` is false.
 template <bool MASS>
 GB_HD int fx_term_pot(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& zi, float eps2f,
-                      const FxRow* tab, FxAcc& a) {
+                      const FxRow* tab, bool on, FxAcc& a) {
   const Fx96 ux = fx_sub(j.x, xi), uy = fx_sub(j.y, yi), uz = fx_sub(j.z, zi);
   const int k = fx_norm(ux, uy, uz, eps2f);
   const FxRow row = tab[k];
@@ -393,7 +394,7 @@ GB_HD int fx_term_pot(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx9
       t = 0;
     }
   }
-  const uint32_t p = k <= kFxMaxK ? 1u << t : 0u;
+  const uint32_t p = on && k <= kFxMaxK ? 1u << t : 0u;
   a.h = (long long)fx_mad(fx_hi(y), p, (uint64_t)a.h);
   a.l = fx_mad(fx_lo(y), p, a.l);
   return k;

@@ -167,20 +167,13 @@ constexpr int f64_smem_bytes() {
 
 // Pair terms of the FP64 loops.
 enum { kPairIeee = 0, kPairFast = 1, kPairFixedFast = 2, kPairFixedIeee = 3 };
-// What the fixed-point loop's FP64 terms add up: accelerations by the refined
-// reciprocal square root or in the reference's operation order, or potentials.
-enum { kF64Fast = 0, kF64Ieee = 1, kF64Pot = 2 };
 
 // One partner's term in FP64, added to s.
 __device__ __forceinline__ void add_pair_f64(const double* pos, long long i, long long j,
-                                             double eps2, const double* masses, int kind,
+                                             double eps2, const double* masses, bool ieee,
                                              double* s) {
   const double mj = masses ? masses[j] : 1.0;
-  if (kind == kF64Pot) {
-    const double dx = pos[3 * j] - pos[3 * i], dy = pos[3 * j + 1] - pos[3 * i + 1],
-                 dz = pos[3 * j + 2] - pos[3 * i + 2];
-    s[0] += mj / sqrt(dx * dx + dy * dy + dz * dz + eps2);
-  } else if (kind == kF64Ieee) {
+  if (ieee) {
     double ax, ay, az;
     pair_term_f64(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], pos[3 * j], pos[3 * j + 1],
                   pos[3 * j + 2], eps2, ax, ay, az);
@@ -209,7 +202,7 @@ __device__ __forceinline__ void add_pair_f64(const double* pos, long long i, lon
 // warp's lane with most of them, which is returned.  The whole warp calls it.
 static __device__ __noinline__ int fx_chunk_f64(unsigned mask, int steps, long long j0, int L,
                                                 const double* pos, long long i, double eps2,
-                                                const double* masses, int kind, double* s) {
+                                                const double* masses, bool ieee, double* s) {
   int rounds = 0;
 #pragma unroll 1
   while (__any_sync(0xffffffffu, mask != 0)) {
@@ -217,7 +210,7 @@ static __device__ __noinline__ int fx_chunk_f64(unsigned mask, int steps, long l
     if (mask) {
       const int u = steps - 32 + __clz(mask);
       mask &= ~(0x80000000u >> __clz(mask));
-      add_pair_f64(pos, i, j0 + (long long)u * L, eps2, masses, kind, s);
+      add_pair_f64(pos, i, j0 + (long long)u * L, eps2, masses, ieee, s);
     }
   }
   return rounds;
@@ -232,14 +225,12 @@ __device__ __forceinline__ void group_bar(int bar, int threads) {
 // The tiles of one CTA or group.  Not inlined, and the geometry (T threads, L
 // lanes) a run-time value: the loop is long enough for the call, and a copy of
 // it in each of the FP64 kernels would make them slow to build.
-// POT: potentials (into part[.][0]) instead of accelerations.
-template <bool MASS, bool POT>
+template <bool MASS>
 __device__ __noinline__ void force_fx_tiles(const double* __restrict__ pos, long long n,
                                             long long i0, long long jb, long long je, double eps2,
                                             const double* __restrict__ masses, int ex, int em,
-                                            int kind, int T, int L, int tid, int bar,
+                                            bool ieee, int T, int L, int tid, int bar,
                                             FxBody* rec, const FxRow* tab, double (*part)[3]) {
-  constexpr int NC = POT ? 1 : 3;
   const int b = tid / L;
   const int l = tid % L;
   const long long i = i0 + b;
@@ -251,8 +242,8 @@ __device__ __noinline__ void force_fx_tiles(const double* __restrict__ pos, long
     zi = fx_from_double(pos[3 * i + 2], ex);
   }
   const float eps2f = fx_eps2f(eps2, ex);
-  __int128 tot[NC] = {};
-  double near[NC] = {};
+  __int128 tot[3] = {};
+  double near[3] = {};
   bool in_f64 = false, any_near = false;  // uniform in the warp
   for (long long j0 = jb; j0 < je; j0 += T) {
     const int cnt = (int)min((long long)T, je - j0);
@@ -278,33 +269,18 @@ __device__ __noinline__ void force_fx_tiles(const double* __restrict__ pos, long
         // unrolled twice: 1.59 ms at N = 16384 against 1.72 ms (1) and 1.73 ms (4)
 #pragma unroll 2
         for (int jj = c0; jj < end; jj += L) {
-          int k;
-          if constexpr (POT)
-            k = fx_term_pot<MASS>(rec[jj], xi, yi, zi, eps2f, tab, a[0]);
-          else
-            k = fx_term<MASS>(rec[jj], xi, yi, zi, eps2f, tab, a);
+          const int k = fx_term<MASS>(rec[jj], xi, yi, zi, eps2f, tab, a);
           mask = __funnelshift_l((unsigned)(kFxMaxK - k), mask, 1);  // 1 when k > kFxMaxK
         }
 #pragma unroll
-        for (int d = 0; d < NC; ++d) fx_fold(tot[d], a[d]);
-      }
-      const auto self_step = [&]() {  // the step of the body itself, or -1
-        const long long self = i - j0 - c0;
-        return self >= 0 && self < (long long)steps * L && self % L == 0 ? (int)self / L : -1;
-      };
-      if (POT && !in_f64 && self_step() >= 0) {
-        // its term is in the sum (that of an acceleration is zero): out again
-        FxAcc a = {};
-        __int128 t = 0;
-        fx_term_pot<MASS>(rec[i - j0], xi, yi, zi, eps2f, tab, a);
-        fx_fold(t, a);
-        tot[0] -= t;
+        for (int d = 0; d < 3; ++d) fx_fold(tot[d], a[d]);
       }
       if (__any_sync(0xffffffffu, mask != 0)) {
         if (!valid) mask = 0;
-        const int self = self_step();
-        if (self >= 0) mask &= ~(1u << (steps - 1 - self));
-        const int rounds = fx_chunk_f64(mask, steps, j0 + c0, L, pos, i, eps2, masses, kind, near);
+        const long long self = i - j0 - c0;  // not the body itself
+        if (self >= 0 && self < (long long)steps * L && self % L == 0)
+          mask &= ~(1u << (steps - 1 - (int)self / L));
+        const int rounds = fx_chunk_f64(mask, steps, j0 + c0, L, pos, i, eps2, masses, ieee, near);
         // an FP64 term costs 5 fixed-point ones: where a lane needs more than 4
         // in 5 of its terms in FP64, the others' are not worth their time
         in_f64 = in_f64 || rounds > kFxChunk * 4 / 5;
@@ -312,11 +288,10 @@ __device__ __noinline__ void force_fx_tiles(const double* __restrict__ pos, long
       }
     }
   }
-  const int sc = POT ? fx_out_exp_pot(ex) + (MASS ? em + 3 : 0)
-                     : fx_out_exp(ex) + (MASS ? em + 1 : 0);
+  const int sc = fx_out_exp(ex) + (MASS ? em + 1 : 0);
   for (int off = L / 2; off >= 1; off /= 2) {
 #pragma unroll
-    for (int d = 0; d < NC; ++d) {
+    for (int d = 0; d < 3; ++d) {
       const unsigned long long lo =
           __shfl_down_sync(0xffffffffu, (unsigned long long)tot[d], off);
       const unsigned long long hi =
@@ -327,7 +302,7 @@ __device__ __noinline__ void force_fx_tiles(const double* __restrict__ pos, long
   }
   if (l == 0) {
 #pragma unroll
-    for (int d = 0; d < NC; ++d) {
+    for (int d = 0; d < 3; ++d) {
       double v = fx_to_double(tot[d], sc);
       if (any_near) v = dadd(v, near[d]);
       part[b][d] = v;
@@ -345,29 +320,25 @@ __device__ __forceinline__ double key_bound(int key, bool upper) {
   return __hiloint2double(h, (h < 0) != upper ? -1 : 0);  // outwards over the low word
 }
 
+// The grid of a group's own body i and of the `count` partners from jb on
+// (modulo n): exponents ex and, with masses, em; red holds 7 words a warp.
 // Returns false, uniformly in the group, when there is no grid: a coordinate
 // that is not finite, bodies all within a sixteenth of the softening,
 // exponents beyond 2^+-300, or a mass that is negative, not finite or all of
-// them zero.  smem: f64_smem_bytes<T>() bytes.
-template <bool POT>
-__device__ __noinline__ bool force_fx_group(const double* __restrict__ pos, long long n,
-                                            long long i0, long long jb, long long je, double eps2,
-                                            const double* __restrict__ masses, int kind,
-                                            unsigned char* smem, double (*part)[3], int T, int L,
-                                            int tid, int bar) {
-  FxBody* rec = reinterpret_cast<FxBody*>(smem);
-  FxRow* tab = reinterpret_cast<FxRow*>(rec + T);
-  int* red = reinterpret_cast<int*>(tab + kFxRows);
+// them zero.
+static __device__ __noinline__ bool fx_grid(const double* __restrict__ pos, long long n,
+                                            long long i, long long jb, long long count,
+                                            double eps2, const double* __restrict__ masses,
+                                            int* red, int T, int tid, int bar, int* ex_out,
+                                            int* em_out) {
   const int nw = T / 32;
   int lo[3], hi[3];
   unsigned mm = 0;
-  {
-    const long long i = min(i0 + tid / L, n - 1);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) lo[c] = hi[c] = order_key(pos[3 * i + c]);
-  }
+  for (int c = 0; c < 3; ++c) lo[c] = hi[c] = order_key(pos[3 * i + c]);
 #pragma unroll 4
-  for (long long j = jb + tid; j < je; j += T) {
+  for (long long v = tid; v < count; v += T) {
+    const long long j = jb + v < n ? jb + v : jb + v - n;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const int k = order_key(pos[3 * j + c]);
@@ -378,7 +349,10 @@ __device__ __noinline__ bool force_fx_group(const double* __restrict__ pos, long
   if (masses) {
     // a negative mass reads as a large unsigned word
 #pragma unroll 4
-    for (long long j = jb + tid; j < je; j += T) mm = max(mm, (unsigned)__double2hiint(masses[j]));
+    for (long long v = tid; v < count; v += T) {
+      const long long j = jb + v < n ? jb + v : jb + v - n;
+      mm = max(mm, (unsigned)__double2hiint(masses[j]));
+    }
   }
   mm = __reduce_max_sync(0xffffffffu, mm);
 #pragma unroll
@@ -422,13 +396,33 @@ __device__ __noinline__ bool force_fx_group(const double* __restrict__ pos, long
   }
   const int em = (int)(mm >> 20) - 1023;  // 2^em <= the largest mass < 2^(em + 1)
   if (ex < -300 || ex > 300 || (masses && (em < -300 || em > 300))) return false;
+  *ex_out = ex;
+  *em_out = em;
+  return true;
+}
+
+// The fixed-point partial sums of a group, or false where there is no grid.
+// smem: f64_smem_bytes<T>() bytes.
+static __device__ __noinline__ bool force_fx_group(const double* __restrict__ pos, long long n,
+                                                   long long i0, long long jb, long long je,
+                                                   double eps2, const double* __restrict__ masses,
+                                                   bool ieee, unsigned char* smem,
+                                                   double (*part)[3], int T, int L, int tid,
+                                                   int bar) {
+  FxBody* rec = reinterpret_cast<FxBody*>(smem);
+  FxRow* tab = reinterpret_cast<FxRow*>(rec + T);
+  int* red = reinterpret_cast<int*>(tab + kFxRows);
+  int ex, em;
+  if (!fx_grid(pos, n, min(i0 + tid / L, n - 1), jb, je - jb, eps2, masses, red, T, tid, bar, &ex,
+               &em))
+    return false;
   if (tid < kFxRows) tab[tid] = fx_row(tid, eps2, ex);
   if (masses)
-    force_fx_tiles<true, POT>(pos, n, i0, jb, je, eps2, masses, ex, em, kind, T, L, tid, bar, rec,
-                              tab, part);
+    force_fx_tiles<true>(pos, n, i0, jb, je, eps2, masses, ex, em, ieee, T, L, tid, bar, rec, tab,
+                         part);
   else
-    force_fx_tiles<false, POT>(pos, n, i0, jb, je, eps2, nullptr, ex, 0, kind, T, L, tid, bar,
-                               rec, tab, part);
+    force_fx_tiles<false>(pos, n, i0, jb, je, eps2, nullptr, ex, 0, ieee, T, L, tid, bar, rec,
+                          tab, part);
   return true;
 }
 
@@ -452,8 +446,8 @@ __device__ __forceinline__ void force_f64_cta(const double* __restrict__ pos, lo
   constexpr int BI = T / L;
   const bool ieee = pair == kPairIeee || pair == kPairFixedIeee;
   if (pair >= kPairFixedFast &&
-      force_fx_group<false>(pos, n, i0, jb, je, eps2, masses, ieee ? kF64Ieee : kF64Fast, smem,
-                            part, T, L, (int)grp.tid(), grp.id()))
+      force_fx_group(pos, n, i0, jb, je, eps2, masses, ieee, smem, part, T, L, (int)grp.tid(),
+                     grp.id()))
     return;
   double* sh_pos = reinterpret_cast<double*>(smem);
   double* sh_m = sh_pos + 3 * T;

@@ -10,9 +10,8 @@
 //              sample order (deterministic, no atomics);
 //   adam     : one thread per parameter.
 // A training epoch (gb_mlp_train) is three kernels, deterministic as well:
-// samples (forward, loss and deltas, a thread per output), gradients (FP64
-// partial sums of a slice of the samples) and update (the slices' sums in
-// order, then Adam).
+// samples (forward, loss and deltas, a thread per output), gradients (sums over
+// a slice of the samples) and update (the slices' sums in order, then Adam).
 // Inference in the controller uses BF16-rounded weights with FP32
 // accumulation (mlp.cuh); gb_mlp_infer_bf16 exposes the same arithmetic.
 #include <algorithm>
@@ -189,29 +188,39 @@ __global__ void adam_kernel(gb_mlp* W, const gb_mlp* G, gb_mlp* M, gb_mlp* V, fl
 // ---------------------------------------------------------------------------
 // The three kernels of a training epoch.
 // ---------------------------------------------------------------------------
-// Forward pass, loss and deltas of 8 samples per CTA, a thread per (output, two
+// acc + w0 v0 + w1 v1 + ..., one multiply-add after the other
+__device__ __forceinline__ float chain4(float4 w, float4 v, float acc) {
+  return fmaf(w.w, v.w, fmaf(w.z, v.z, fmaf(w.y, v.y, fmaf(w.x, v.x, acc))));
+}
+
+// Forward pass, loss (the asymmetric squared error w (y - t)^2 with w = over_w
+// where y > t) and deltas of 8 samples per CTA, a thread per (output, two
 // samples).  Every output is the same chain of multiply-adds as in
 // forward_kernel and delta_kernel, so the values are theirs bit for bit; with
 // one thread per sample 16 CTAs walked 64 such chains one after the other
-// (2000 samples: 21 us for the two passes, against 5 us here).  The weights'
-// rows are padded to 65 floats, free of bank conflicts along both indices.
+// (2000 samples: 28 us for each pass, against 8 us here for both).  The
+// weights' rows are padded by 4 floats: 16-byte reads along them and single
+// reads across them without bank conflicts.
 constexpr int kSamples = 8;
 __global__ void __launch_bounds__(256)
     samples_kernel(const gb_mlp* __restrict__ W, const float* __restrict__ x,
                    const float* __restrict__ target, long long B, float over_w,
                    float* __restrict__ delta, float* __restrict__ dy,
                    float* __restrict__ lsample) {
-  __shared__ float w1[kHid][kIn + 1], w2[kHid][kHid + 1];
-  __shared__ float xs[kSamples][kIn], h1[kSamples][kHid], h2[kSamples][kHid];
+  __shared__ __align__(16) float w1[kHid][kIn + 4], w2[kHid][kHid + 4];
+  __shared__ __align__(16) float xs[kSamples][kIn], h1[kSamples][kHid], h2[kSamples][kHid];
   __shared__ float sg[kSamples], w3[kHid];
   const int t = threadIdx.x, o = t % kHid, g = t / kHid;
   const long long s0 = blockIdx.x * (long long)kSamples;
+#pragma unroll
   for (int k = t; k < kHid * kIn; k += 256) w1[k / kIn][k % kIn] = (&W->w1[0][0])[k];
+#pragma unroll
   for (int k = t; k < kHid * kHid; k += 256) w2[k / kHid][k % kHid] = (&W->w2[0][0])[k];
-  if (t < kSamples * kIn) {
-    const long long s = s0 + t / kIn;
-    const int k = t % kIn;
-    xs[t / kIn][k] = s < B ? (x[s * kIn + k] - W->in_mean[k]) * W->in_scale[k] : 0.f;
+#pragma unroll
+  for (int e = t; e < kSamples * kIn; e += 256) {
+    const long long s = s0 + e / kIn;
+    const int k = e % kIn;
+    xs[e / kIn][k] = s < B ? (x[s * kIn + k] - W->in_mean[k]) * W->in_scale[k] : 0.f;
   }
   if (t < kHid) w3[t] = W->w3[t];
   __syncthreads();
@@ -220,18 +229,23 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
   for (int r = 0; r < R; ++r) z1[r] = W->b1[o];
 #pragma unroll
-  for (int k = 0; k < kIn; ++k)
+  for (int k = 0; k < kIn; k += 4) {
+    const float4 w = *reinterpret_cast<const float4*>(&w1[o][k]);
 #pragma unroll
-    for (int r = 0; r < R; ++r) z1[r] = fmaf(w1[o][k], xs[g + 4 * r][k], z1[r]);
+    for (int r = 0; r < R; ++r) z1[r] = chain4(w, *reinterpret_cast<const float4*>(&xs[g + 4 * r][k]), z1[r]);
+  }
 #pragma unroll
   for (int r = 0; r < R; ++r) h1[g + 4 * r][o] = silu(z1[r]);
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < R; ++r) z2[r] = W->b2[o];
-#pragma unroll 16
-  for (int k = 0; k < kHid; ++k)
+#pragma unroll 4
+  for (int k = 0; k < kHid; k += 4) {
+    const float4 w = *reinterpret_cast<const float4*>(&w2[o][k]);
 #pragma unroll
-    for (int r = 0; r < R; ++r) z2[r] = fmaf(w2[o][k], h1[g + 4 * r][k], z2[r]);
+    for (int r = 0; r < R; ++r)
+      z2[r] = chain4(w, *reinterpret_cast<const float4*>(&h1[g + 4 * r][k]), z2[r]);
+  }
 #pragma unroll
   for (int r = 0; r < R; ++r) h2[g + 4 * r][o] = silu(z2[r]);
   __syncthreads();
@@ -263,10 +277,13 @@ __global__ void __launch_bounds__(256)
   float acc[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) acc[r] = 0.f;
-#pragma unroll 16
-  for (int k = 0; k < kHid; ++k)
+#pragma unroll 4
+  for (int k = 0; k < kHid; k += 4) {
+    const float4 w = make_float4(w2[k][o], w2[k + 1][o], w2[k + 2][o], w2[k + 3][o]);
 #pragma unroll
-    for (int r = 0; r < R; ++r) acc[r] = fmaf(w2[k][o], h1[g + 4 * r][k], acc[r]);
+    for (int r = 0; r < R; ++r)
+      acc[r] = chain4(w, *reinterpret_cast<const float4*>(&h1[g + 4 * r][k]), acc[r]);
+  }
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const long long s = s0 + g + 4 * r;
@@ -279,92 +296,153 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Gradient sums of a slice of the samples, all parameters, in FP64 as in
-// grad_kernel: the samples' vectors are converted once into shared memory and
-// every thread keeps a 4 x 4 block of w2's sums, a 1 x 4 block of w1's and one
-// of the vectors'.  Bound by the FP64 pipe, 5313 multiply-adds a sample over
-// all SMs: 2000 samples 19 us, where one thread per parameter took 330 us on
-// 42 CTAs with two conversions and a sum a sample in its chain.
-constexpr int kSliceBatch = 8;  // samples staged at a time
-__global__ void __launch_bounds__(256)
+// An unevaluated sum of three floats, about 72 bits: exact products and sums of
+// FP32 values to more than FP64's precision on the FP32 pipe, where a product
+// and its sum take 22 cycles of a sub-partition and an FP64 multiply-add 76
+// (with two conversions of 64 before it).  A product's error term is exact down
+// to 2^-149 (products above 2^-102); what is lost below that is nothing beside
+// Adam's 1e-8.
+struct Sum3 {
+  float h = 0.f, m = 0.f, l = 0.f;
+};
+
+// Knuth's error-free sum: s + e == a + b.
+__device__ __forceinline__ void exact_sum(float a, float b, float& s, float& e) {
+  s = __fadd_rn(a, b);
+  const float bb = __fsub_rn(s, a);
+  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+}
+// t += h + m + l
+__device__ __forceinline__ void add3(Sum3& t, float h, float m, float l) {
+  float e1, e2, e3, s;
+  exact_sum(t.h, h, s, e1);
+  t.h = s;
+  exact_sum(t.m, m, s, e2);
+  exact_sum(s, e1, t.m, e3);
+  t.l = __fadd_rn(t.l, __fadd_rn(l, __fadd_rn(e2, e3)));
+}
+// t += a b
+__device__ __forceinline__ void add_product(Sum3& t, float a, float b) {
+  const float p = __fmul_rn(a, b);
+  add3(t, p, __fmaf_rn(a, b, -p), 0.f);
+}
+__device__ __forceinline__ void add_value(Sum3& t, float a) {
+  float e, s;
+  exact_sum(t.h, a, s, e);
+  t.h = s;
+  exact_sum(t.m, e, s, e);
+  t.m = s;
+  t.l = __fadd_rn(t.l, e);
+}
+
+// Gradient sums of a slice of the samples, all parameters: every thread keeps a
+// 4 x 4 block of w2's sums, a 1 x 4 block of w1's and one of the vectors', as
+// sums of three floats of exact products.  2000 samples: 29 us with FP64
+// multiply-adds (5313 a sample, the FP64 pipe's rate), 14 us so; one thread per
+// parameter took 330 us on 42 CTAs.  partial: [slice][3][parameter].
+constexpr int kSliceBatch = 8;   // samples staged at a time
+constexpr int kGradThreads = 512;
+constexpr int kPartial = (kTrainable + 3) / 4 * 4;  // parameters, for 16-byte stores
+__global__ void __launch_bounds__(kGradThreads)
     gradient_kernel(const gb_mlp* __restrict__ W, const float* __restrict__ x,
                     const float* __restrict__ delta, const float* __restrict__ dy, long long B,
-                    long long per, double* __restrict__ partial) {
-  __shared__ double d[kSliceBatch][kDeltaPerSample];
-  __shared__ double xs[kSliceBatch][kIn];
-  __shared__ double sg[kSliceBatch];
+                    long long per, float* __restrict__ partial) {
+  __shared__ float4 d4[kSliceBatch][kDeltaPerSample / 4];
+  __shared__ float4 x4[kSliceBatch][kIn / 4];
+  __shared__ float sg[kSliceBatch];
   const int t = threadIdx.x;
   const long long s0 = blockIdx.x * per, s1 = min(B, s0 + per);
-  const int o4 = (t / 16) * 4, k4 = (t % 16) * 4;  // w2's block
-  const int o1 = t / 4, k1 = (t % 4) * 4;          // w1's
-  double a2[4][4] = {}, a1[4] = {}, av = 0.0;
+  const int o2 = t / 16, k4 = t % 16;  // w2's block: rows 2 o2, 2 o2 + 1, columns 4 k4 ...
+  const int o1 = t / 8, k2 = t % 8;    // w1's: columns 2 k2, 2 k2 + 1
+  Sum3 a2[2][4], a1[2], av;
   const float os = W->out_scale;
   for (long long b = s0; b < s1; b += kSliceBatch) {
     const int m = (int)min((long long)kSliceBatch, s1 - b);
     __syncthreads();
-    for (int r = 0; r < m; ++r) d[r][t] = (double)delta[(b + r) * kDeltaPerSample + t];
+#pragma unroll
+    for (int r = 0; r < kSliceBatch; r += kGradThreads / (kDeltaPerSample / 4)) {
+      const int q = r + t / (kDeltaPerSample / 4), c = t % (kDeltaPerSample / 4);
+      if (q < m)
+        d4[q][c] = reinterpret_cast<const float4*>(delta + (b + q) * kDeltaPerSample)[c];
+    }
     if (t < m * kIn) {
       const int k = t % kIn;
-      xs[t / kIn][k] = (double)((x[(b + t / kIn) * kIn + k] - W->in_mean[k]) * W->in_scale[k]);
+      reinterpret_cast<float*>(x4[t / kIn])[k] =
+          (x[(b + t / kIn) * kIn + k] - W->in_mean[k]) * W->in_scale[k];
     }
-    if (t < m) sg[t] = (double)(dy[b + t] * os);
+    if (t < m) sg[t] = dy[b + t] * os;
     __syncthreads();
+#pragma unroll 1
     for (int r = 0; r < m; ++r) {
-      const double *h1 = d[r], *dz1 = d[r] + kHid, *h2 = d[r] + 2 * kHid, *dz2 = d[r] + 3 * kHid;
+      const float4* h1 = d4[r];
+      const float *dz1 = reinterpret_cast<const float*>(h1 + kHid / 4), *h2 = dz1 + kHid,
+                  *dz2 = h2 + kHid;
+      const float2 go = reinterpret_cast<const float2*>(dz2)[o2];
+      const float4 gk = h1[k4];
+      const float2 gx = reinterpret_cast<const float2*>(x4[r])[k2];
+      const float ao[2] = {go.x, go.y}, ak[4] = {gk.x, gk.y, gk.z, gk.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) a2[i][j] = fma(dz2[o4 + i], h1[k4 + j], a2[i][j]);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) a1[j] = fma(dz1[o1], xs[r][k1 + j], a1[j]);
+        for (int j = 0; j < 4; ++j) add_product(a2[i][j], ao[i], ak[j]);
+      add_product(a1[0], dz1[o1], gx.x);
+      add_product(a1[1], dz1[o1], gx.y);
       if (t < kHid)
-        av += dz1[t];
+        add_value(av, dz1[t]);
       else if (t < 2 * kHid)
-        av += dz2[t - kHid];
+        add_value(av, dz2[t - kHid]);
       else if (t < 3 * kHid)
-        av = fma(sg[r], h2[t - 2 * kHid], av);
+        add_product(av, sg[r], h2[t - 2 * kHid]);
       else if (t == 3 * kHid)
-        av += sg[r];
+        add_value(av, sg[r]);
     }
   }
-  double* out = partial + (long long)blockIdx.x * kTrainable;
+  float* out = partial + (long long)blockIdx.x * 3 * kPartial;
+  constexpr int w2 = kParamsW1 + kHid;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) out[o1 * kIn + k1 + j] = a1[j];
-  double* w2 = out + kParamsW1 + kHid;
+  for (int i = 0; i < 2; ++i) {
+    const int q = (w2 + (2 * o2 + i) * kHid) / 4 + k4;
+    const Sum3* v = a2[i];
+    reinterpret_cast<float4*>(out)[q] = make_float4(v[0].h, v[1].h, v[2].h, v[3].h);
+    reinterpret_cast<float4*>(out + kPartial)[q] = make_float4(v[0].m, v[1].m, v[2].m, v[3].m);
+    reinterpret_cast<float4*>(out + 2 * kPartial)[q] = make_float4(v[0].l, v[1].l, v[2].l, v[3].l);
+  }
+  const auto put = [&](int p, const Sum3& v) {
+    out[p] = v.h;
+    out[kPartial + p] = v.m;
+    out[2 * kPartial + p] = v.l;
+  };
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) w2[(o4 + i) * kHid + k4 + j] = a2[i][j];
+  for (int j = 0; j < 2; ++j) put(o1 * kIn + 2 * k2 + j, a1[j]);
   if (t < kHid)
-    out[kParamsW1 + t] = av;
+    put(kParamsW1 + t, av);
   else if (t <= 3 * kHid)  // b2, w3, b3 follow w2
-    w2[kParamsW2 + t - kHid] = av;
+    put(w2 + kParamsW2 + t - kHid, av);
 }
 
-// The slices' sums of a parameter (8 lanes, each its slices in order, then a
-// tree), rounded to FP32, and the Adam step.
+// The slices' sums of 32 parameters (warp g adds slices g, g + 8, ... in order,
+// then the warps' sums are added in order), rounded to FP32, and the Adam step.
 __global__ void __launch_bounds__(256)
-    update_kernel(gb_mlp* W, const double* __restrict__ partial, int slices, gb_mlp* M, gb_mlp* V,
+    update_kernel(gb_mlp* W, const float* __restrict__ partial, int slices, gb_mlp* M, gb_mlp* V,
                   float lr, float b1, float b2, float eps, float c1, float c2) {
-  const int lane = threadIdx.x % 8;
-  const int p = (blockIdx.x * 256 + threadIdx.x) / 8;
-  double v = 0.0;
-  if (p < kTrainable)
-    for (int c = lane; c < slices; c += 8) v += partial[(long long)c * kTrainable + p];
+  __shared__ Sum3 sums[8][32];
+  const int lane = threadIdx.x % 32, g = threadIdx.x / 32;
+  const int p = blockIdx.x * 32 + lane;
+  Sum3 v;
+  if (p < kTrainable) {
+#pragma unroll 5
+    for (int c = g; c < slices; c += 8) {
+      const float* q = partial + (long long)c * 3 * kPartial + p;
+      add3(v, q[0], q[kPartial], q[2 * kPartial]);
+    }
+  }
+  sums[g][lane] = v;
+  __syncthreads();
+  if (g == 0 && p < kTrainable) {
 #pragma unroll
-  for (int off = 4; off >= 1; off /= 2) v += __shfl_down_sync(0xffffffffu, v, off, 8);
-  if (p < kTrainable && lane == 0) adam_param(W, (float)v, M, V, p, lr, b1, b2, eps, c1, c2);
-}
-
-// Asymmetric squared error: w (y - t)^2 with w = over_weight when y > t.
-__global__ void loss_kernel(const float* __restrict__ y, const float* __restrict__ t, long long B,
-                            float over_w, float* __restrict__ dy, float* __restrict__ lsample) {
-  const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (s >= B) return;
-  const float r = y[s] - t[s];
-  const float w = r > 0.f ? over_w : 1.f;
-  dy[s] = 2.f * w * r / (float)B;
-  lsample[s] = w * r * r;
+    for (int r = 1; r < 8; ++r) add3(v, sums[r][lane].h, sums[r][lane].m, sums[r][lane].l);
+    adam_param(W, __fadd_rn(v.h, __fadd_rn(v.m, v.l)), M, V, p, lr, b1, b2, eps, c1, c2);
+  }
 }
 
 __global__ void mean_kernel(const float* __restrict__ v, long long B, float* out) {
@@ -506,22 +584,22 @@ extern "C" int gb_mlp_train(gb_mlp* W, const float* x, const float* target, int6
   // slices of the gradient sums: one per SM, at least 4 samples each
   const long long per = std::max(4LL, ((long long)B + num_sms() - 1) / num_sms());
   const int slices = (int)((B + per - 1) / per);
-  // one allocation: partial sums (doubles first), deltas, y, dy, losses, moments
-  const size_t n_partial = (size_t)slices * kTrainable * sizeof(double);
+  // one allocation: partial sums, deltas, dy, losses, moments
+  const size_t n_partial = (size_t)slices * 3 * kPartial * sizeof(float);
   const size_t n_delta = (size_t)B * kDeltaPerSample * sizeof(float);
   const size_t n_sample = (size_t)B * sizeof(float);
   unsigned char* base = nullptr;
   int rc = GB_OK;
-  cudaError_t e = cudaMalloc((void**)&base, n_partial + n_delta + 3 * n_sample +
+  cudaError_t e = cudaMalloc((void**)&base, n_partial + n_delta + 2 * n_sample +
                                                 2 * sizeof(gb_mlp) + sizeof(float));
   if (e != cudaSuccess) {
     note_cuda_error(e);
     return GB_ERR_CUDA;
   }
-  double* partial = reinterpret_cast<double*>(base);
+  float* partial = reinterpret_cast<float*>(base);
   float* delta = reinterpret_cast<float*>(base + n_partial);
-  float* y = reinterpret_cast<float*>(base + n_partial + n_delta);
-  float *dy = y + B, *ls = dy + B;
+  float* dy = reinterpret_cast<float*>(base + n_partial + n_delta);
+  float* ls = dy + B;
   gb_mlp* M = reinterpret_cast<gb_mlp*>(ls + B);
   gb_mlp* V = M + 1;
   float* loss = reinterpret_cast<float*>(V + 1);
@@ -530,8 +608,8 @@ extern "C" int gb_mlp_train(gb_mlp* W, const float* x, const float* target, int6
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)ep), c2 = 1.f - std::pow(b2, (float)ep);
     samples_kernel<<<nblk(B, kSamples), 256, 0, s>>>(W, x, target, B, over_w, delta, dy, ls);
-    gradient_kernel<<<(unsigned)slices, 256, 0, s>>>(W, x, delta, dy, B, per, partial);
-    update_kernel<<<nblk(8LL * kTrainable, 256), 256, 0, s>>>(W, partial, slices, M, V, lr, b1,
+    gradient_kernel<<<(unsigned)slices, kGradThreads, 0, s>>>(W, x, delta, dy, B, per, partial);
+    update_kernel<<<nblk(kTrainable, 32), 256, 0, s>>>(W, partial, slices, M, V, lr, b1,
                                                               b2, 1e-8f, c1, c2);
     e = cudaGetLastError();
   }
@@ -540,19 +618,17 @@ extern "C" int gb_mlp_train(gb_mlp* W, const float* x, const float* target, int6
     rc = GB_ERR_CUDA;
   }
   if (rc == GB_OK) {
-    rc = gb_mlp_forward_f32(W, x, y, B, nullptr, stream);
-    if (rc == GB_OK) {
-      loss_kernel<<<nblk(B, 256), 256, 0, s>>>(y, target, B, over_w, dy, ls);
-      mean_kernel<<<1, 256, 0, s>>>(ls, B, loss);
-      float hl = 0.f;
-      e = cudaMemcpyAsync(&hl, loss, sizeof(float), cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-      if (e != cudaSuccess) {
-        note_cuda_error(e);
-        rc = GB_ERR_CUDA;
-      } else if (loss_host) {
-        *loss_host = hl;
-      }
+    // the loss of the trained network
+    samples_kernel<<<nblk(B, kSamples), 256, 0, s>>>(W, x, target, B, over_w, delta, dy, ls);
+    mean_kernel<<<1, 256, 0, s>>>(ls, B, loss);
+    float hl = 0.f;
+    e = cudaMemcpyAsync(&hl, loss, sizeof(float), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) {
+      note_cuda_error(e);
+      rc = GB_ERR_CUDA;
+    } else if (loss_host) {
+      *loss_host = hl;
     }
   }
   cudaStreamSynchronize(s);

@@ -253,16 +253,18 @@ __global__ void __launch_bounds__(128)
   const BSys sy = P.sys[k];
   const int S = tab.n_stages;
   double v = 0.0, m = 0.0;
-  for (int t = lane; t < sy.n_units; t += 32) {
-    const int u = P.sys_units[sy.unit_off + t];
-    v = dadd(v, P.partials[u]);
-    m = fmax(m, P.aux[u]);
+  {
+    long long mb = 0;  // squares: non-negative, so their bit patterns order like integers
+    for (int t = lane; t < sy.n_units; t += 32) {
+      const int u = P.sys_units[sy.unit_off + t];
+      v = dadd(v, P.partials[u]);
+      const long long b = __double_as_longlong(P.aux[u]);
+      mb = b > mb ? b : mb;
+    }
+    m = sqrt(warp_max_nonneg(__longlong_as_double(mb)));
   }
 #pragma unroll
-  for (int off = 16; off >= 1; off /= 2) {
-    v = dadd(v, __shfl_xor_sync(0xffffffffu, v, off));
-    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
-  }
+  for (int off = 16; off >= 1; off /= 2) v = dadd(v, __shfl_xor_sync(0xffffffffu, v, off));
   const double err = sqrt(v / (double)(6 * sy.n));
   int want = 0;
   if (lane == 0) {

@@ -18,6 +18,13 @@ constexpr double kMinStepScale = 0.33;  // RKEmbeddedParallel.hpp:22
 // are too long.
 constexpr double kLearnedMaxLogCorrection = 1.0986122886681098;  // log(3)
 
+// The floor dt / span < 1e-12 of a step; twice the floor away the division (a
+// tenth of the controller thread's FP64 operations) cannot decide otherwise.
+__device__ __forceinline__ double floor_step(double dt, double span) {
+  if (span > 0.0 && dt > 2.0e-12 * span) return dt;
+  return dt / span < 1.0e-12 ? span * 1.0e-12 : dt;
+}
+
 // The reference's elementary controller (RKEmbeddedParallel.hpp:65-74):
 // dtnew = dt * safety / err^(1/(1+q)), clamped to x6 / x0.33, with a floor
 // at (tf - t0) * 1e-12 reached only inside the clamp window.
@@ -27,8 +34,7 @@ __device__ __forceinline__ double reference_step(double dt, double err, double s
   const double dtnew = dt * safety / (exact_pow ? dd_pow(err, e) : pow(err, e));
   if (fabs(dtnew) > kMaxStepScale * fabs(dt)) return dt * kMaxStepScale;
   if (fabs(dtnew) < kMinStepScale * fabs(dt)) return dt * kMinStepScale;
-  if (dtnew / (tf - t0) < 1.0e-12) return (tf - t0) * 1.0e-12;
-  return dtnew;
+  return floor_step(dtnew, tf - t0);
 }
 
 // PI controller in the form of Hairer, Norsett & Wanner (and Numerical
@@ -52,9 +58,7 @@ __device__ __forceinline__ double pi_step(Ctrl& c, double dt, double err, bool a
     scale = fmax(c.safety * pow(err, -c.pi_alpha), kMinStepScale);
     c.reject_prev = 1;
   }
-  double dtn = dt * scale;
-  if (dtn / (c.tf - c.t0) < 1.0e-12) dtn = (c.tf - c.t0) * 1.0e-12;
-  return dtn;
+  return floor_step(dt * scale, c.tf - c.t0);
 }
 
 // Per-system environment of the end-of-attempt decision.

@@ -19,28 +19,54 @@ __device__ __forceinline__ int kslot(int l, int S, int k0slot) {
   return l;
 }
 
+// Sum over the threads of the CTA as a tree of halving distance: red[t] +=
+// red[t + st], the distances below a warp's width by shuffles (the same
+// additions; five barriers fewer).
 __device__ __forceinline__ double block_sum(double v, double* red) {
   red[threadIdx.x] = v;
   __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st /= 2) {
+  for (int st = blockDim.x / 2; st >= 32; st /= 2) {
     if ((int)threadIdx.x < st) red[threadIdx.x] = dadd(red[threadIdx.x], red[threadIdx.x + st]);
     __syncthreads();
   }
-  double r = red[0];
+  if (threadIdx.x < 32) {
+    double r = red[threadIdx.x];
+#pragma unroll
+    for (int off = 16; off >= 1; off /= 2) r = dadd(r, __shfl_down_sync(0xffffffffu, r, off));
+    if (threadIdx.x == 0) red[0] = r;
+  }
+  __syncthreads();
+  const double r = red[0];
   __syncthreads();
   return r;
 }
 
-__device__ __forceinline__ double block_max(double v, double* red) {
-  red[threadIdx.x] = v;
-  __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st /= 2) {
-    if ((int)threadIdx.x < st) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + st]);
-    __syncthreads();
+// Maximum over a warp of values >= 0 (NaN counts as 0, as in fmax with 0): their
+// bit patterns order like integers, and an FP64 compare would take the FP64
+// pipe like an addition.
+__device__ __forceinline__ double warp_max_nonneg(double v) {
+  long long b = __double_as_longlong(v);
+  b = b > 0x7ff0000000000000ll || b < 0 ? 0 : b;
+#pragma unroll
+  for (int off = 16; off >= 1; off /= 2) {
+    const long long o = __shfl_xor_sync(0xffffffffu, b, off);
+    b = o > b ? o : b;
   }
-  double r = red[0];
+  return __longlong_as_double(b);
+}
+
+// Maximum over the CTA of values >= 0.
+__device__ __forceinline__ double block_max(double v, double* red) {
+  v = warp_max_nonneg(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x / 32] = v;
   __syncthreads();
-  return r;
+  long long m = 0;
+  for (int w = 0; w < (int)blockDim.x / 32; ++w) {
+    const long long o = __double_as_longlong(red[w]);
+    m = o > m ? o : m;
+  }
+  __syncthreads();
+  return __longlong_as_double(m);
 }
 
 struct EpiCtx {
@@ -67,7 +93,8 @@ struct EpiCtx {
 
 // One body's six state elements.  `acc` is the unscaled pair sum (ignored
 // when the stage derivative is reused).  Adds the body's scaled squares to
-// sq_acc and its |a| to amax (both at the last stage).
+// sq_acc and its |a|^2 to amax (both at the last stage; the square root of the
+// largest is the largest root, taken once by the controller).
 template <int PREC>
 __device__ __forceinline__ void body_epilogue(const EpiCtx& E, long long i, const double* acc,
                                               double& sq_acc, double& amax,
@@ -94,7 +121,7 @@ __device__ __forceinline__ void body_epilogue(const EpiCtx& E, long long i, cons
     }
 #pragma unroll
     for (int e = 0; e < 6; ++e) ks_s[idx[e]] = k[e];
-    if (E.last) amax = fmax(amax, sqrt(k[3] * k[3] + k[4] * k[4] + k[5] * k[5]));
+    if (E.last) amax = fmax(amax, k[3] * k[3] + k[4] * k[4] + k[5] * k[5]);
   }
   // Stage sums: the stage index runs outermost so that a stage's six loads
   // are in flight together; every element still sums its terms from 0.0 in
@@ -233,7 +260,7 @@ __device__ __forceinline__ void rows_epilogue(const EpiCtx& E, long long i0, int
         double k[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) k[c] = E.masses ? a[c] : dmul(a[c], E.mass);
-        amax = fmax(amax, sqrt(k[0] * k[0] + k[1] * k[1] + k[2] * k[2]));
+        amax = fmax(amax, k[0] * k[0] + k[1] * k[1] + k[2] * k[2]);
       }
     }
   }

@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(T, 6 * 128 / T)
   for (int b = threadIdx.x; b < b_hi; b += T) {
     const double k0 = dmul(pw[3 * b], P.mass), k1 = dmul(pw[3 * b + 1], P.mass),
                  k2 = dmul(pw[3 * b + 2], P.mass);
-    amax = fmax(amax, sqrt(k0 * k0 + k1 * k1 + k2 * k2));
+    amax = fmax(amax, k0 * k0 + k1 * k1 + k2 * k2);
   }
   const double m = block_max(amax, red);
   const double tile_sum = block_sum(sq_acc, red);
@@ -685,13 +685,19 @@ __global__ void __launch_bounds__(256)
     total = block_sum(v, red);
   }
   const int k0_valid = C->k0_valid;
-  double amax_all = 0.0;
+  double amax_all = 0.0, err = 0.0;
   {
-    double v = 0.0;
-    for (long long k = threadIdx.x; k < P.n_parts; k += T) v = fmax(v, P.aux[k]);
-    amax_all = block_max(v, red);
+    long long m = 0;  // squares: non-negative, so their bit patterns order like integers
+    for (long long k = threadIdx.x; k < P.n_parts; k += T) {
+      const long long b = __double_as_longlong(P.aux[k]);
+      m = b > m ? b : m;
+    }
+    const double v = block_max(__longlong_as_double(m), red);
+    if (threadIdx.x == 0) {
+      amax_all = sqrt(v);
+      err = sqrt(total / (double)n_var);
+    }
   }
-  const double err = sqrt(total / (double)n_var);
   // Learned proposal: features of the post-attempt state (thread 0), then
   // the 16 -> 64 -> 64 -> 1 network across the CTA.
   if (threadIdx.x == 0) {

@@ -167,133 +167,28 @@ __global__ void zero_nontrainable_kernel(gb_mlp* G) {
   }
 }
 
-__device__ __forceinline__ void adam_param(gb_mlp* W, float g, gb_mlp* M, gb_mlp* V, int p,
-                                           float lr, float b1, float b2, float eps, float c1,
-                                           float c2) {
-  float& m = *param_ptr(M, p);
-  float& v = *param_ptr(V, p);
+__device__ __forceinline__ void adam_param(float g, float& w, float& m, float& v, float lr,
+                                           float b1, float b2, float eps, float c1, float c2) {
   m = b1 * m + (1.f - b1) * g;
   v = b2 * v + (1.f - b2) * g * g;
   const float mh = m / c1, vh = v / c2;
-  *param_ptr(W, p) -= lr * mh / (sqrtf(vh) + eps);
+  w -= lr * mh / (sqrtf(vh) + eps);
 }
 
 __global__ void adam_kernel(gb_mlp* W, const gb_mlp* G, gb_mlp* M, gb_mlp* V, float lr,
                             float b1, float b2, float eps, float c1, float c2) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= kTrainable) return;
-  adam_param(W, *param_ptr(const_cast<gb_mlp*>(G), p), M, V, p, lr, b1, b2, eps, c1, c2);
+  adam_param(*param_ptr(const_cast<gb_mlp*>(G), p), *param_ptr(W, p), *param_ptr(M, p),
+             *param_ptr(V, p), lr, b1, b2, eps, c1, c2);
 }
 
 // ---------------------------------------------------------------------------
-// The three kernels of a training epoch.
+// The two kernels of a training epoch.
 // ---------------------------------------------------------------------------
 // acc + w0 v0 + w1 v1 + ..., one multiply-add after the other
 __device__ __forceinline__ float chain4(float4 w, float4 v, float acc) {
   return fmaf(w.w, v.w, fmaf(w.z, v.z, fmaf(w.y, v.y, fmaf(w.x, v.x, acc))));
-}
-
-// Forward pass, loss (the asymmetric squared error w (y - t)^2 with w = over_w
-// where y > t) and deltas of 8 samples per CTA, a thread per (output, two
-// samples).  Every output is the same chain of multiply-adds as in
-// forward_kernel and delta_kernel, so the values are theirs bit for bit; with
-// one thread per sample 16 CTAs walked 64 such chains one after the other
-// (2000 samples: 28 us for each pass, against 8 us here for both).  The
-// weights' rows are padded by 4 floats: 16-byte reads along them and single
-// reads across them without bank conflicts.
-constexpr int kSamples = 8;
-__global__ void __launch_bounds__(256)
-    samples_kernel(const gb_mlp* __restrict__ W, const float* __restrict__ x,
-                   const float* __restrict__ target, long long B, float over_w,
-                   float* __restrict__ delta, float* __restrict__ dy,
-                   float* __restrict__ lsample) {
-  __shared__ __align__(16) float w1[kHid][kIn + 4], w2[kHid][kHid + 4];
-  __shared__ __align__(16) float xs[kSamples][kIn], h1[kSamples][kHid], h2[kSamples][kHid];
-  __shared__ float sg[kSamples], w3[kHid];
-  const int t = threadIdx.x, o = t % kHid, g = t / kHid;
-  const long long s0 = blockIdx.x * (long long)kSamples;
-#pragma unroll
-  for (int k = t; k < kHid * kIn; k += 256) w1[k / kIn][k % kIn] = (&W->w1[0][0])[k];
-#pragma unroll
-  for (int k = t; k < kHid * kHid; k += 256) w2[k / kHid][k % kHid] = (&W->w2[0][0])[k];
-#pragma unroll
-  for (int e = t; e < kSamples * kIn; e += 256) {
-    const long long s = s0 + e / kIn;
-    const int k = e % kIn;
-    xs[e / kIn][k] = s < B ? (x[s * kIn + k] - W->in_mean[k]) * W->in_scale[k] : 0.f;
-  }
-  if (t < kHid) w3[t] = W->w3[t];
-  __syncthreads();
-  constexpr int R = kSamples * kHid / 256;  // samples of a thread: g, g + 4
-  float z1[R], z2[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) z1[r] = W->b1[o];
-#pragma unroll
-  for (int k = 0; k < kIn; k += 4) {
-    const float4 w = *reinterpret_cast<const float4*>(&w1[o][k]);
-#pragma unroll
-    for (int r = 0; r < R; ++r) z1[r] = chain4(w, *reinterpret_cast<const float4*>(&xs[g + 4 * r][k]), z1[r]);
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r) h1[g + 4 * r][o] = silu(z1[r]);
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < R; ++r) z2[r] = W->b2[o];
-#pragma unroll 4
-  for (int k = 0; k < kHid; k += 4) {
-    const float4 w = *reinterpret_cast<const float4*>(&w2[o][k]);
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      z2[r] = chain4(w, *reinterpret_cast<const float4*>(&h1[g + 4 * r][k]), z2[r]);
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r) h2[g + 4 * r][o] = silu(z2[r]);
-  __syncthreads();
-  if (t < kSamples) {
-    const long long s = s0 + t;
-    float out = W->b3;
-#pragma unroll 16
-    for (int k = 0; k < kHid; ++k) out = fmaf(w3[k], h2[t][k], out);
-    const float y = W->out_scale * out + W->out_bias;
-    float d = 0.f;
-    if (s < B) {
-      const float res = y - target[s];
-      const float w = res > 0.f ? over_w : 1.f;
-      d = 2.f * w * res / (float)B;
-      dy[s] = d;
-      lsample[s] = w * res * res;
-    }
-    sg[t] = d * W->out_scale;
-  }
-  __syncthreads();
-  // deltas: h1, dz1, h2, dz2; dz2 takes h1's place in shared memory
-  float hv[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) hv[r] = h1[g + 4 * r][o];
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < R; ++r) h1[g + 4 * r][o] = sg[g + 4 * r] * w3[o] * dsilu(z2[r]);
-  __syncthreads();
-  float acc[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) acc[r] = 0.f;
-#pragma unroll 4
-  for (int k = 0; k < kHid; k += 4) {
-    const float4 w = make_float4(w2[k][o], w2[k + 1][o], w2[k + 2][o], w2[k + 3][o]);
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      acc[r] = chain4(w, *reinterpret_cast<const float4*>(&h1[g + 4 * r][k]), acc[r]);
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const long long s = s0 + g + 4 * r;
-    if (s >= B) continue;
-    float* d = delta + s * kDeltaPerSample;
-    d[o] = hv[r];
-    d[kHid + o] = acc[r] * dsilu(z1[r]);
-    d[2 * kHid + o] = h2[g + 4 * r][o];
-    d[3 * kHid + o] = h1[g + 4 * r][o];
-  }
 }
 
 // An unevaluated sum of three floats, about 72 bits: exact products and sums of
@@ -335,113 +230,215 @@ __device__ __forceinline__ void add_value(Sum3& t, float a) {
   t.l = __fadd_rn(t.l, e);
 }
 
-// Gradient sums of a slice of the samples, all parameters: every thread keeps a
-// 4 x 4 block of w2's sums, a 1 x 4 block of w1's and one of the vectors', as
-// sums of three floats of exact products.  2000 samples: 29 us with FP64
-// multiply-adds (5313 a sample, the FP64 pipe's rate), 14 us so; one thread per
-// parameter took 330 us on 42 CTAs.  partial: [slice][3][parameter].
-constexpr int kSliceBatch = 8;   // samples staged at a time
-constexpr int kGradThreads = 512;
+// t rounded to FP32: the parts made disjoint first, as the sums above may leave
+// the middle one as large as the first after a cancellation.
+__device__ __forceinline__ float round3(const Sum3& t) {
+  float h, m, l;
+  exact_sum(t.h, t.m, h, m);
+  exact_sum(m, t.l, m, l);
+  exact_sum(h, m, h, m);
+  return __fadd_rn(h, __fadd_rn(m, l));
+}
+
+// Forward pass, loss (the asymmetric squared error w (y - t)^2 with w = over_w
+// where y > t), deltas and gradient sums of a slice of the samples, 16 samples
+// at a time.  GRAD false: the forward pass and each sample's loss alone.
+//
+// Forward and deltas: a thread per (output, two samples); every output is the
+// same chain of multiply-adds as in forward_kernel and delta_kernel, so the
+// values are theirs bit for bit.  The weights' rows are padded by 4 floats:
+// 16-byte reads along them and single reads across them without bank conflicts.
+// Gradient: every thread keeps a 2 x 4 block of w2's sums, a 1 x 2 block of w1's
+// and one of the vectors', as sums of three floats of exact products (29 us at
+// 2000 samples with FP64 multiply-adds: 5313 a sample, the FP64 pipe's rate).
+// partial: [slice][3][parameter].
+//
+// The chip's SMs have one slice each, so what bounds an epoch is the chain
+// within a CTA: the deltas stay in shared memory (as a kernel of their own the
+// forward pass took 8 us and the gradient sums 14.5: an epoch 30.2 -> 26.8 us).
+constexpr int kBatch = 16;  // samples staged at a time
+constexpr int kEpochThreads = 512;
 constexpr int kPartial = (kTrainable + 3) / 4 * 4;  // parameters, for 16-byte stores
-__global__ void __launch_bounds__(kGradThreads)
-    gradient_kernel(const gb_mlp* __restrict__ W, const float* __restrict__ x,
-                    const float* __restrict__ delta, const float* __restrict__ dy, long long B,
-                    long long per, float* __restrict__ partial) {
-  __shared__ float4 d4[kSliceBatch][kDeltaPerSample / 4];
-  __shared__ float4 x4[kSliceBatch][kIn / 4];
-  __shared__ float sg[kSliceBatch];
-  const int t = threadIdx.x;
+template <bool GRAD>
+__global__ void __launch_bounds__(kEpochThreads)
+    epoch_kernel(const gb_mlp* __restrict__ W, const float* __restrict__ x,
+                 const float* __restrict__ target, long long B, long long per, float over_w,
+                 float* __restrict__ partial, float* __restrict__ lsample) {
+  constexpr int T = kEpochThreads, G = T / kHid, R = kBatch / G, kPad = kHid + 4;
+  __shared__ __align__(16) float w1[kHid][kIn + 4], w2[kHid][kPad];
+  __shared__ __align__(16) float xs[kBatch][kIn], h1[kBatch][kPad], h2[kBatch][kPad],
+      dz1[GRAD ? kBatch : 1][kPad], dz2[GRAD ? kBatch : 1][kPad], w3[kHid];
+  __shared__ float sg[kBatch];
+  const int t = threadIdx.x, o = t % kHid, g = t / kHid;
   const long long s0 = blockIdx.x * per, s1 = min(B, s0 + per);
+#pragma unroll
+  for (int k = t; k < kHid * kIn; k += T) w1[k / kIn][k % kIn] = (&W->w1[0][0])[k];
+#pragma unroll
+  for (int k = t; k < kHid * kHid; k += T) w2[k / kHid][k % kHid] = (&W->w2[0][0])[k];
+  if (t < kHid) w3[t] = W->w3[t];
+  const float mean = W->in_mean[t % kIn], scale = W->in_scale[t % kIn];
+  const float b1 = W->b1[o], b2 = W->b2[o], b3 = W->b3, os = W->out_scale, ob = W->out_bias;
   const int o2 = t / 16, k4 = t % 16;  // w2's block: rows 2 o2, 2 o2 + 1, columns 4 k4 ...
   const int o1 = t / 8, k2 = t % 8;    // w1's: columns 2 k2, 2 k2 + 1
   Sum3 a2[2][4], a1[2], av;
-  const float os = W->out_scale;
-  for (long long b = s0; b < s1; b += kSliceBatch) {
-    const int m = (int)min((long long)kSliceBatch, s1 - b);
+  for (long long b = s0; b < s1; b += kBatch) {
+    const int m = (int)min((long long)kBatch, s1 - b);
+    if (t < m * kIn) xs[t / kIn][t % kIn] = (x[b * kIn + t] - mean) * scale;
+    __syncthreads();
+    float z1[R], z2[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) z1[r] = b1;
+#pragma unroll
+    for (int k = 0; k < kIn; k += 4) {
+      const float4 w = *reinterpret_cast<const float4*>(&w1[o][k]);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (g + G * r < m)
+          z1[r] = chain4(w, *reinterpret_cast<const float4*>(&xs[g + G * r][k]), z1[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) h1[g + G * r][o] = silu(z1[r]);
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < kSliceBatch; r += kGradThreads / (kDeltaPerSample / 4)) {
-      const int q = r + t / (kDeltaPerSample / 4), c = t % (kDeltaPerSample / 4);
-      if (q < m)
-        d4[q][c] = reinterpret_cast<const float4*>(delta + (b + q) * kDeltaPerSample)[c];
+    for (int r = 0; r < R; ++r) z2[r] = b2;
+#pragma unroll 4
+    for (int k = 0; k < kHid; k += 4) {
+      const float4 w = *reinterpret_cast<const float4*>(&w2[o][k]);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        z2[r] = chain4(w, *reinterpret_cast<const float4*>(&h1[g + G * r][k]), z2[r]);
     }
-    if (t < m * kIn) {
-      const int k = t % kIn;
-      reinterpret_cast<float*>(x4[t / kIn])[k] =
-          (x[(b + t / kIn) * kIn + k] - W->in_mean[k]) * W->in_scale[k];
-    }
-    if (t < m) sg[t] = dy[b + t] * os;
+#pragma unroll
+    for (int r = 0; r < R; ++r) h2[g + G * r][o] = silu(z2[r]);
     __syncthreads();
+    if (t < m) {
+      float out = b3;
+#pragma unroll
+      for (int k = 0; k < kHid; k += 4)
+        out = chain4(*reinterpret_cast<const float4*>(&w3[k]),
+                     *reinterpret_cast<const float4*>(&h2[t][k]), out);
+      const float y = os * out + ob;
+      const float res = y - target[b + t];
+      const float w = res > 0.f ? over_w : 1.f;
+      if (GRAD)
+        sg[t] = 2.f * w * res / (float)B * os;
+      else
+        lsample[b + t] = w * res * res;
+    }
+    __syncthreads();
+    if constexpr (GRAD) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (g + G * r < m) dz2[g + G * r][o] = sg[g + G * r] * w3[o] * dsilu(z2[r]);
+      __syncthreads();
+      float acc[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) acc[r] = 0.f;
+#pragma unroll 4
+      for (int k = 0; k < kHid; k += 4) {
+        const float4 w = make_float4(w2[k][o], w2[k + 1][o], w2[k + 2][o], w2[k + 3][o]);
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          acc[r] = chain4(w, *reinterpret_cast<const float4*>(&dz2[g + G * r][k]), acc[r]);
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) dz1[g + G * r][o] = acc[r] * dsilu(z1[r]);
+      __syncthreads();
 #pragma unroll 1
-    for (int r = 0; r < m; ++r) {
-      const float4* h1 = d4[r];
-      const float *dz1 = reinterpret_cast<const float*>(h1 + kHid / 4), *h2 = dz1 + kHid,
-                  *dz2 = h2 + kHid;
-      const float2 go = reinterpret_cast<const float2*>(dz2)[o2];
-      const float4 gk = h1[k4];
-      const float2 gx = reinterpret_cast<const float2*>(x4[r])[k2];
-      const float ao[2] = {go.x, go.y}, ak[4] = {gk.x, gk.y, gk.z, gk.w};
+      for (int r = 0; r < m; ++r) {
+        const float2 go = reinterpret_cast<const float2*>(dz2[r])[o2];
+        const float4 gk = reinterpret_cast<const float4*>(h1[r])[k4];
+        const float2 gx = reinterpret_cast<const float2*>(xs[r])[k2];
+        const float ao[2] = {go.x, go.y}, ak[4] = {gk.x, gk.y, gk.z, gk.w};
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) add_product(a2[i][j], ao[i], ak[j]);
-      add_product(a1[0], dz1[o1], gx.x);
-      add_product(a1[1], dz1[o1], gx.y);
-      if (t < kHid)
-        add_value(av, dz1[t]);
-      else if (t < 2 * kHid)
-        add_value(av, dz2[t - kHid]);
-      else if (t < 3 * kHid)
-        add_product(av, sg[r], h2[t - 2 * kHid]);
-      else if (t == 3 * kHid)
-        add_value(av, sg[r]);
+          for (int j = 0; j < 4; ++j) add_product(a2[i][j], ao[i], ak[j]);
+        add_product(a1[0], dz1[r][o1], gx.x);
+        add_product(a1[1], dz1[r][o1], gx.y);
+        if (t < kHid)
+          add_value(av, dz1[r][t]);
+        else if (t < 2 * kHid)
+          add_value(av, dz2[r][t - kHid]);
+        else if (t < 3 * kHid)
+          add_product(av, sg[r], h2[r][t - 2 * kHid]);
+        else if (t == 3 * kHid)
+          add_value(av, sg[r]);
+      }
+      __syncthreads();
     }
   }
-  float* out = partial + (long long)blockIdx.x * 3 * kPartial;
-  constexpr int w2 = kParamsW1 + kHid;
+  if constexpr (GRAD) {
+    float* out = partial + (long long)blockIdx.x * 3 * kPartial;
+    constexpr int pw2 = kParamsW1 + kHid;
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int q = (w2 + (2 * o2 + i) * kHid) / 4 + k4;
-    const Sum3* v = a2[i];
-    reinterpret_cast<float4*>(out)[q] = make_float4(v[0].h, v[1].h, v[2].h, v[3].h);
-    reinterpret_cast<float4*>(out + kPartial)[q] = make_float4(v[0].m, v[1].m, v[2].m, v[3].m);
-    reinterpret_cast<float4*>(out + 2 * kPartial)[q] = make_float4(v[0].l, v[1].l, v[2].l, v[3].l);
+    for (int i = 0; i < 2; ++i) {
+      const int q = (pw2 + (2 * o2 + i) * kHid) / 4 + k4;
+      const Sum3* v = a2[i];
+      reinterpret_cast<float4*>(out)[q] = make_float4(v[0].h, v[1].h, v[2].h, v[3].h);
+      reinterpret_cast<float4*>(out + kPartial)[q] = make_float4(v[0].m, v[1].m, v[2].m, v[3].m);
+      reinterpret_cast<float4*>(out + 2 * kPartial)[q] = make_float4(v[0].l, v[1].l, v[2].l, v[3].l);
+    }
+    const auto put = [&](int p, const Sum3& v) {
+      out[p] = v.h;
+      out[kPartial + p] = v.m;
+      out[2 * kPartial + p] = v.l;
+    };
+#pragma unroll
+    for (int j = 0; j < 2; ++j) put(o1 * kIn + 2 * k2 + j, a1[j]);
+    if (t < kHid)
+      put(kParamsW1 + t, av);
+    else if (t <= 3 * kHid)  // b2, w3, b3 follow w2
+      put(pw2 + kParamsW2 + t - kHid, av);
   }
-  const auto put = [&](int p, const Sum3& v) {
-    out[p] = v.h;
-    out[kPartial + p] = v.m;
-    out[2 * kPartial + p] = v.l;
-  };
-#pragma unroll
-  for (int j = 0; j < 2; ++j) put(o1 * kIn + 2 * k2 + j, a1[j]);
-  if (t < kHid)
-    put(kParamsW1 + t, av);
-  else if (t <= 3 * kHid)  // b2, w3, b3 follow w2
-    put(w2 + kParamsW2 + t - kHid, av);
 }
 
-// The slices' sums of 32 parameters (warp g adds slices g, g + 8, ... in order,
+// The slices' sums of 32 parameters (warp g adds slices g, g + 16, ... in order,
 // then the warps' sums are added in order), rounded to FP32, and the Adam step.
-__global__ void __launch_bounds__(256)
+// Bound by the latency of the loads: all of a warp's in flight at once up to 144
+// slices (8 warps and 5 slices at a time: 9.4 us, so 6.0; the epoch 26.8 -> 25.0).
+constexpr int kUpdateWarps = 16;
+constexpr int kUpdateLoads = 10;  // slices of a warp loaded together: 160 cover the SMs
+__global__ void __launch_bounds__(32 * kUpdateWarps)
     update_kernel(gb_mlp* W, const float* __restrict__ partial, int slices, gb_mlp* M, gb_mlp* V,
                   float lr, float b1, float b2, float eps, float c1, float c2) {
-  __shared__ Sum3 sums[8][32];
+  __shared__ Sum3 sums[kUpdateWarps][32];
   const int lane = threadIdx.x % 32, g = threadIdx.x / 32;
   const int p = blockIdx.x * 32 + lane;
+  const bool mine = g == 0 && p < kTrainable;
+  float w = 0.f, m = 0.f, u = 0.f;
+  if (mine) {
+    w = *param_ptr(W, p);
+    m = *param_ptr(M, p);
+    u = *param_ptr(V, p);
+  }
   Sum3 v;
   if (p < kTrainable) {
-#pragma unroll 5
-    for (int c = g; c < slices; c += 8) {
-      const float* q = partial + (long long)c * 3 * kPartial + p;
-      add3(v, q[0], q[kPartial], q[2 * kPartial]);
+    constexpr int K = kUpdateLoads;
+    for (int c = g; c < slices; c += K * kUpdateWarps) {
+      float h[K], d[K], l[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const bool on = c + k * kUpdateWarps < slices;
+        const float* q = partial + (long long)(c + k * kUpdateWarps) * 3 * kPartial + p;
+        h[k] = on ? q[0] : 0.f;
+        d[k] = on ? q[kPartial] : 0.f;
+        l[k] = on ? q[2 * kPartial] : 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k) add3(v, h[k], d[k], l[k]);
     }
   }
   sums[g][lane] = v;
   __syncthreads();
-  if (g == 0 && p < kTrainable) {
+  if (mine) {
 #pragma unroll
-    for (int r = 1; r < 8; ++r) add3(v, sums[r][lane].h, sums[r][lane].m, sums[r][lane].l);
-    adam_param(W, __fadd_rn(v.h, __fadd_rn(v.m, v.l)), M, V, p, lr, b1, b2, eps, c1, c2);
+    for (int r = 1; r < kUpdateWarps; ++r)
+      add3(v, sums[r][lane].h, sums[r][lane].m, sums[r][lane].l);
+    adam_param(round3(v), w, m, u, lr, b1, b2, eps, c1, c2);
+    *param_ptr(W, p) = w;
+    *param_ptr(M, p) = m;
+    *param_ptr(V, p) = u;
   }
 }
 
@@ -584,22 +581,19 @@ extern "C" int gb_mlp_train(gb_mlp* W, const float* x, const float* target, int6
   // slices of the gradient sums: one per SM, at least 4 samples each
   const long long per = std::max(4LL, ((long long)B + num_sms() - 1) / num_sms());
   const int slices = (int)((B + per - 1) / per);
-  // one allocation: partial sums, deltas, dy, losses, moments
+  // one allocation: partial sums, losses, moments
   const size_t n_partial = (size_t)slices * 3 * kPartial * sizeof(float);
-  const size_t n_delta = (size_t)B * kDeltaPerSample * sizeof(float);
   const size_t n_sample = (size_t)B * sizeof(float);
   unsigned char* base = nullptr;
   int rc = GB_OK;
-  cudaError_t e = cudaMalloc((void**)&base, n_partial + n_delta + 2 * n_sample +
-                                                2 * sizeof(gb_mlp) + sizeof(float));
+  cudaError_t e = cudaMalloc((void**)&base, n_partial + n_sample + 2 * sizeof(gb_mlp) +
+                                                sizeof(float));
   if (e != cudaSuccess) {
     note_cuda_error(e);
     return GB_ERR_CUDA;
   }
   float* partial = reinterpret_cast<float*>(base);
-  float* delta = reinterpret_cast<float*>(base + n_partial);
-  float* dy = reinterpret_cast<float*>(base + n_partial + n_delta);
-  float* ls = dy + B;
+  float* ls = reinterpret_cast<float*>(base + n_partial);
   gb_mlp* M = reinterpret_cast<gb_mlp*>(ls + B);
   gb_mlp* V = M + 1;
   float* loss = reinterpret_cast<float*>(V + 1);
@@ -607,9 +601,9 @@ extern "C" int gb_mlp_train(gb_mlp* W, const float* x, const float* target, int6
   for (int ep = 1; ep <= epochs && e == cudaSuccess; ++ep) {
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)ep), c2 = 1.f - std::pow(b2, (float)ep);
-    samples_kernel<<<nblk(B, kSamples), 256, 0, s>>>(W, x, target, B, over_w, delta, dy, ls);
-    gradient_kernel<<<(unsigned)slices, kGradThreads, 0, s>>>(W, x, delta, dy, B, per, partial);
-    update_kernel<<<nblk(kTrainable, 32), 256, 0, s>>>(W, partial, slices, M, V, lr, b1,
+    epoch_kernel<true><<<(unsigned)slices, kEpochThreads, 0, s>>>(W, x, target, B, per, over_w,
+                                                                  partial, nullptr);
+    update_kernel<<<nblk(kTrainable, 32), 32 * kUpdateWarps, 0, s>>>(W, partial, slices, M, V, lr, b1,
                                                               b2, 1e-8f, c1, c2);
     e = cudaGetLastError();
   }
@@ -619,7 +613,8 @@ extern "C" int gb_mlp_train(gb_mlp* W, const float* x, const float* target, int6
   }
   if (rc == GB_OK) {
     // the loss of the trained network
-    samples_kernel<<<nblk(B, kSamples), 256, 0, s>>>(W, x, target, B, over_w, delta, dy, ls);
+    epoch_kernel<false><<<(unsigned)slices, kEpochThreads, 0, s>>>(W, x, target, B, per, over_w,
+                                                                   nullptr, ls);
     mean_kernel<<<1, 256, 0, s>>>(ls, B, loss);
     float hl = 0.f;
     e = cudaMemcpyAsync(&hl, loss, sizeof(float), cudaMemcpyDeviceToHost, s);

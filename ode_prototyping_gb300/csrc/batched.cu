@@ -32,9 +32,6 @@
 
 namespace gb {
 
-int launch_norm(const double* v, const double* s, long long n, double* partial, double* out,
-                int take_sqrt, cudaStream_t st);
-
 namespace {
 
 struct BSys {

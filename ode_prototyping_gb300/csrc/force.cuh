@@ -1235,7 +1235,8 @@ struct ForceGeom {
 
 ForceGeom choose_geom(long long n, int precision, const gb_force_tiling* tiling, int exact,
                       bool uniform_masses = true);
+// after: the kernel begins with after_previous
 int launch_cluster(const void* kernel, const ForceGeom& g, size_t smem, cudaStream_t s,
-                   void** args);
+                   void** args, bool after = false);
 
 }  // namespace gb

@@ -54,6 +54,47 @@ struct DevTableau {
 };
 DevTableau make_dev_tableau(const gb_tableau& t);
 
+// ----- programmatic dependent launch ------------------------------------------
+// A kernel launched by launch_after may have its CTAs resident while the kernel
+// before it in the stream still runs, once all of that one's CTAs have called
+// let_next_in (or ended); after_previous, first thing in it, waits until the
+// kernel before it has completed and its writes are visible.  Every pointer the
+// kernel reads or writes through passes through it, so that no access can be
+// scheduled above the wait (a load of a const __restrict__ pointer could be: it
+// counts as invariant).  What it saves is the launch, 1.3 to 2.6 us of a short
+// kernel in a stream: RKF78's twelve stages and update at 600018 elements 211 ->
+// 173 us, a training epoch 25.0 -> 22.5 us, N = 257 FP64 10.25 -> 8.96 us.
+template <class... P>
+__device__ __forceinline__ void after_previous(P&... p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  ((void)[&] { asm volatile("" : "+l"(p)::"memory"); }(), ...);
+}
+__device__ __forceinline__ void let_next_in() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// A captured launch stays an ordinary node: with programmatic edges the graph of
+// an integrator's attempts ran slower (1024 bodies FP64 1940 -> 2061 us).
+inline bool overlaps(cudaStream_t s) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+}
+
+template <class... K, class... A>
+cudaError_t launch_after(void (*kernel)(K...), unsigned grid, unsigned block, cudaStream_t s,
+                         A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(block, 1, 1);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = overlaps(s) ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+
 // ----- exact FP64 arithmetic helpers (no contraction) -----------------------
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }

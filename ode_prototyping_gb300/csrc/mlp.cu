@@ -269,6 +269,8 @@ __global__ void __launch_bounds__(kEpochThreads)
   __shared__ __align__(16) float xs[kBatch][kIn], h1[kBatch][kPad], h2[kBatch][kPad],
       dz1[GRAD ? kBatch : 1][kPad], dz2[GRAD ? kBatch : 1][kPad], w3[kHid];
   __shared__ float sg[kBatch];
+  after_previous(W, x, target, partial, lsample);
+  let_next_in();
   const int t = threadIdx.x, o = t % kHid, g = t / kHid;
   const long long s0 = blockIdx.x * per, s1 = min(B, s0 + per);
 #pragma unroll
@@ -403,6 +405,8 @@ __global__ void __launch_bounds__(32 * kUpdateWarps)
     update_kernel(gb_mlp* W, const float* __restrict__ partial, int slices, gb_mlp* M, gb_mlp* V,
                   float lr, float b1, float b2, float eps, float c1, float c2) {
   __shared__ Sum3 sums[kUpdateWarps][32];
+  after_previous(W, partial, M, V);
+  let_next_in();
   const int lane = threadIdx.x % 32, g = threadIdx.x / 32;
   const int p = blockIdx.x * 32 + lane;
   const bool mine = g == 0 && p < kTrainable;
@@ -601,11 +605,11 @@ extern "C" int gb_mlp_train(gb_mlp* W, const float* x, const float* target, int6
   for (int ep = 1; ep <= epochs && e == cudaSuccess; ++ep) {
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)ep), c2 = 1.f - std::pow(b2, (float)ep);
-    epoch_kernel<true><<<(unsigned)slices, kEpochThreads, 0, s>>>(W, x, target, B, per, over_w,
-                                                                  partial, nullptr);
-    update_kernel<<<nblk(kTrainable, 32), 32 * kUpdateWarps, 0, s>>>(W, partial, slices, M, V, lr, b1,
-                                                              b2, 1e-8f, c1, c2);
-    e = cudaGetLastError();
+    e = launch_after(epoch_kernel<true>, (unsigned)slices, kEpochThreads, s, W, x, target, B, per,
+                     over_w, partial, nullptr);
+    if (e == cudaSuccess)
+      e = launch_after(update_kernel, nblk(kTrainable, 32), 32 * kUpdateWarps, s, W, partial,
+                       slices, M, V, lr, b1, b2, 1e-8f, c1, c2);
   }
   if (e != cudaSuccess) {
     note_cuda_error(e);

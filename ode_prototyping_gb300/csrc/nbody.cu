@@ -22,7 +22,16 @@ namespace {
 
 enum { kModeRhs = 0, kModeAccWrite = 1, kModeAccAdd = 2 };
 
-template <int T, int L>
+// AFTER: the launch overlaps the kernel before it in the stream.  For grids of
+// at most 4 CTAs per SM, whose launches are short (N = 257 FP64 10.25 -> 8.96 us
+// a call, 3001 1846 -> 1807 us for 24 steps of leapfrog; N = 4096 mixed 28.7 -> 24.7
+// us); beyond that the loops run 0.3-0.6 % faster with their pointers left
+// __restrict__ (N = 16384 FP64, 100003 mixed).  A kernel of at most kFewCtas CTAs
+// lets the next one's wait beside it; more of them leave the next kernel's
+// unevenly spread over the SMs (3001: 2088 us for the 24 steps where they may).
+constexpr unsigned kFewCtas = 76;
+constexpr int kAfterCtasPerSm = 4;
+template <int T, int L, bool AFTER = false>
 __global__ void __launch_bounds__(T) rhs_f64_kernel(const double* __restrict__ pos,
                                                     const double* __restrict__ vel,
                                                     double* __restrict__ out_vel,
@@ -33,6 +42,10 @@ __global__ void __launch_bounds__(T) rhs_f64_kernel(const double* __restrict__ p
   constexpr int BI = T / L;
   __shared__ __align__(16) unsigned char sh_raw[f64_smem_bytes<T>()];
   __shared__ double part[BI][3];
+  if constexpr (AFTER) {
+    after_previous(pos, vel, out_vel, out_acc, masses);
+    if (gridDim.x <= kFewCtas) let_next_in();
+  }
   const ClusterInfo ci = cluster_info();
   const long long i0 = ci.itile * BI;
   long long jb, je;
@@ -76,6 +89,8 @@ template <bool PACK>
 __global__ void __cluster_dims__(kCentroidCtas, 1, 1) __launch_bounds__(128)
     centroid_kernel(const double* __restrict__ pos, const double* __restrict__ masses, long long n,
                     double* c_out, PackedBody* out) {
+  after_previous(pos, masses, c_out, out);
+  let_next_in();
   __shared__ double chain[3][128];
   __shared__ double cen[3];
   cg::cluster_group cl = cg::this_cluster();
@@ -132,6 +147,7 @@ __global__ void __cluster_dims__(kCentroidCtas, 1, 1) __launch_bounds__(128)
 
 __global__ void pack_kernel(const double* __restrict__ pos, const double* __restrict__ masses,
                             const double* __restrict__ c, long long n, PackedBody* out) {
+  after_previous(pos, masses, c, out);
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   out[i] = pack_row(pos, masses, c[0], c[1], c[2], i);
@@ -141,11 +157,12 @@ __global__ void pack_kernel(const double* __restrict__ pos, const double* __rest
 // CTAs of 128 threads on an SM (N = 100003 4.62 ms; 4.68 at 8, 4.80 at 10, 4.87
 // at 5, 5.2 at 6 and 7; the same order at 16384 and 65536), the other forms,
 // whose launches are shorter, with what 5 CTAs leave.
-template <int T, int L, int BPT, bool PACKED>
+template <int T, int L, int BPT, bool PACKED, bool AFTER = false>
 __global__ void __launch_bounds__(T, (PACKED && L == 1 && BPT == 1 ? 9 : 5) * 128 / T)
     rhs_mixed_kernel(const PackedBody* __restrict__ packed, const double* __restrict__ vel,
                      double* __restrict__ out_vel, double* __restrict__ out_acc, long long n,
                      float eps2, double mass, int uniform_mass) {
+  if constexpr (AFTER) after_previous(packed, vel, out_vel, out_acc);
   constexpr int BI = (T / L) * BPT;
   constexpr int SH = PACKED ? jp_smem_bytes<T>() : (int)sizeof(PackedBody) * T;
   __shared__ __align__(16) unsigned char sh_raw[SH];
@@ -185,6 +202,36 @@ const void* pick_f64(int L) {
     case 8: return (const void*)rhs_f64_kernel<T, 8>;
     default: return nullptr;
   }
+}
+
+// The kernel whose launch overlaps the one before it, for the geometries that the
+// library picks itself, or null.
+bool may_overlap(const ForceGeom& g) {
+  return g.n_itiles * g.P <= (long long)kAfterCtasPerSm * num_sms();
+}
+const void* pick_f64_after(const ForceGeom& g) {
+  if (g.T != 128 || !may_overlap(g)) return nullptr;
+  switch (g.L) {
+    case 2: return (const void*)rhs_f64_kernel<128, 2, true>;
+    case 4: return (const void*)rhs_f64_kernel<128, 4, true>;
+    case 8: return (const void*)rhs_f64_kernel<128, 8, true>;
+    default: return nullptr;
+  }
+}
+template <int BPT, bool PACKED>
+const void* pick_mixed_after_L(int L) {
+  switch (L) {
+    case 1: return (const void*)rhs_mixed_kernel<128, 1, BPT, PACKED, true>;
+    case 2: return (const void*)rhs_mixed_kernel<128, 2, BPT, PACKED, true>;
+    case 4: return (const void*)rhs_mixed_kernel<128, 4, BPT, PACKED, true>;
+    default: return nullptr;
+  }
+}
+const void* pick_mixed_after(const ForceGeom& g, bool packed) {
+  if (g.T != 128 || !may_overlap(g)) return nullptr;
+  if (packed && g.BPT == 1) return pick_mixed_after_L<1, true>(g.L);
+  if (!packed && g.BPT == 2) return pick_mixed_after_L<2, false>(g.L);
+  return nullptr;
 }
 
 template <int T, int BPT, bool PACKED>
@@ -240,7 +287,8 @@ int run_f64(const double* pos, const double* vel, double* out_vel, double* out_a
                                       : kPairIeee;
   void* args[] = {(void*)&pos, (void*)&vel, (void*)&out_vel, (void*)&out_acc, (void*)&n,
                   (void*)&eps2, (void*)&mass, (void*)&masses, (void*)&mode, (void*)&pair};
-  return launch_cluster(k, g, 0, s, args);
+  const void* ka = pick_f64_after(g);
+  return launch_cluster(ka ? ka : k, g, 0, s, args, ka != nullptr);
 }
 
 }  // namespace
@@ -279,19 +327,21 @@ int rhs_for_start(int prec, const double* x, double* dxdt, long long n, double s
 }
 
 int launch_cluster(const void* kernel, const ForceGeom& g, size_t smem, cudaStream_t s,
-                   void** args) {
+                   void** args, bool after) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(g.n_itiles * g.P), 1, 1);
   cfg.blockDim = dim3((unsigned)g.T, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)g.P;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = after && overlaps(s) ? 2 : 1;
   if (g.P > 8) {
     // clusters above 8 CTAs are opt-in per kernel; the attribute is set on
     // the first (uncaptured) launch and persists
@@ -410,13 +460,11 @@ int mixed_rhs_into(const double* x, double* dxdt, long long n, double softening,
                    const double* masses, PackedBody* packed, double* c,
                    const gb_force_tiling* tiling, cudaStream_t s) {
   if (n <= kFusedPackBodies) {
-    centroid_kernel<true><<<kCentroidCtas, 128, 0, s>>>(x, masses, n, c, packed);
+    GB_CUDA_TRY(launch_after(centroid_kernel<true>, kCentroidCtas, 128, s, x, masses, n, c, packed));
   } else {
-    centroid_kernel<false><<<kCentroidCtas, 128, 0, s>>>(x, nullptr, n, c, nullptr);
-    GB_CUDA_TRY(cudaGetLastError());
-    pack_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(x, masses, c, n, packed);
+    GB_CUDA_TRY(launch_after(centroid_kernel<false>, kCentroidCtas, 128, s, x, nullptr, n, c, nullptr));
+    GB_CUDA_TRY(launch_after(pack_kernel, (unsigned)((n + 255) / 256), 256, s, x, masses, c, n, packed));
   }
-  GB_CUDA_TRY(cudaGetLastError());
   ForceGeom g = choose_geom(n, GB_PREC_MIXED, tiling, 0, masses == nullptr);
   const void* k = nullptr;
   switch (g.T) {
@@ -432,7 +480,8 @@ int mixed_rhs_into(const double* x, double* dxdt, long long n, double softening,
   int uniform = masses ? 0 : 1;
   void* args[] = {(void*)&packed, (void*)&vel,  (void*)&out_vel, (void*)&out_acc,
                   (void*)&n,      (void*)&eps2, (void*)&mass,    (void*)&uniform};
-  return launch_cluster(k, g, 0, s, args);
+  const void* ka = pick_mixed_after(g, use_packed(tiling, g.BPT, masses));
+  return launch_cluster(ka ? ka : k, g, 0, s, args, ka != nullptr);
 }
 }  // namespace gb
 

@@ -177,6 +177,8 @@ __global__ void __launch_bounds__(kBlock) stage_kernel(const __grid_constant__ C
                                                        const double* __restrict__ x0,
                                                        const double* __restrict__ ks,
                                                        double* __restrict__ temp, long long n) {
+  after_previous(x0, ks, temp);
+  let_next_in();
   const long long m = n / V;
   for (long long e = blockIdx.x * (long long)kBlock + threadIdx.x; e < m;
        e += (long long)gridDim.x * kBlock) {
@@ -205,6 +207,8 @@ __global__ void __launch_bounds__(kBlock) update_kernel(const __grid_constant__ 
                                                         const double* __restrict__ ks,
                                                         double* __restrict__ x,
                                                         double* __restrict__ err, long long n) {
+  after_previous(x0, ks, x, err);
+  let_next_in();
   const long long m = n / V;
   for (long long e = blockIdx.x * (long long)kBlock + threadIdx.x; e < m;
        e += (long long)gridDim.x * kBlock) {
@@ -232,6 +236,8 @@ __global__ void __launch_bounds__(kBlock) target_kernel(const double* __restrict
                                                         const double* __restrict__ x,
                                                         const double* __restrict__ x0,
                                                         double* __restrict__ target, long long n) {
+  after_previous(atol, rtol, x, x0, target);
+  let_next_in();
   const long long m = n / V;
   for (long long e = blockIdx.x * (long long)kBlock + threadIdx.x; e < m;
        e += (long long)gridDim.x * kBlock) {
@@ -271,6 +277,8 @@ __global__ void __launch_bounds__(kBlock) sq_partial_kernel(const double* __rest
                                                             const double* __restrict__ s,
                                                             long long n,
                                                             double* __restrict__ partial) {
+  after_previous(v, s, partial);
+  let_next_in();
   __shared__ double sh[kBlock];
   constexpr int U = 4;
   double acc[U] = {0.0, 0.0, 0.0, 0.0};
@@ -301,6 +309,8 @@ __global__ void __launch_bounds__(kBlock) sq_partial_kernel(const double* __rest
 // Sums the partials in block order; out = sqrt(sum / n) or the sum itself.
 __global__ void sq_final_kernel(const double* __restrict__ partial, int nb, long long n,
                                 int take_sqrt, double* out) {
+  after_previous(partial, out);
+  let_next_in();
   __shared__ double sh[kBlock];
   double acc = 0.0;
   for (int i = threadIdx.x; i < nb; i += kBlock) acc = dadd(acc, partial[i]);
@@ -337,7 +347,7 @@ void launch_stage_v(const Coef& cf, double dt, const double* x0, const double* k
   const unsigned g = stream_blocks(n / V);
   switch (cf.n) {
 #define GB_CASE(k) \
-  case k: stage_kernel<k, V><<<g, kBlock, 0, st>>>(cf, dt, x0, ks, temp, n); break;
+  case k: (void)launch_after(stage_kernel<k, V>, g, kBlock, st, cf, dt, x0, ks, temp, n); break;
     GB_TERM_CASES(GB_CASE)
 #undef GB_CASE
     default: break;
@@ -350,7 +360,7 @@ void launch_update_v(const Coef& cf, double dt, const double* x0, const double* 
   const unsigned g = stream_blocks(n / V);
   switch (cf.n) {
 #define GB_CASE(k) \
-  case k: update_kernel<k, V><<<g, kBlock, 0, st>>>(cf, dt, x0, ks, x, err, n); break;
+  case k: (void)launch_after(update_kernel<k, V>, g, kBlock, st, cf, dt, x0, ks, x, err, n); break;
     GB_TERM_CASES(GB_CASE)
 #undef GB_CASE
     default: break;
@@ -362,10 +372,8 @@ void launch_update_v(const Coef& cf, double dt, const double* x0, const double* 
 int launch_norm(const double* v, const double* s, long long n, double* partial, double* out,
                 int take_sqrt, cudaStream_t st) {
   const int nb = norm_blocks(n);
-  sq_partial_kernel<<<nb, kBlock, 0, st>>>(v, s, n, partial);
-  GB_CUDA_TRY(cudaGetLastError());
-  sq_final_kernel<<<1, kBlock, 0, st>>>(partial, nb, n, take_sqrt, out);
-  GB_CUDA_TRY(cudaGetLastError());
+  GB_CUDA_TRY(launch_after(sq_partial_kernel, nb, kBlock, st, v, s, n, partial));
+  GB_CUDA_TRY(launch_after(sq_final_kernel, 1, kBlock, st, partial, nb, n, take_sqrt, out));
   return GB_OK;
 }
 
@@ -592,10 +600,11 @@ extern "C" int gb_rk_error_target_f64(const double* atol, const double* rtol, co
   cudaStream_t st = as_cuda(stream);
   if (n % 2 == 0 && aligned16(atol) && aligned16(rtol) && aligned16(x) && aligned16(x0) &&
       aligned16(target))
-    target_kernel<2><<<stream_blocks(n / 2), kBlock, 0, st>>>(atol, rtol, x, x0, target, n);
+    GB_CUDA_TRY(launch_after(target_kernel<2>, stream_blocks(n / 2), kBlock, st, atol, rtol, x, x0,
+                             target, n));
   else
-    target_kernel<1><<<stream_blocks(n), kBlock, 0, st>>>(atol, rtol, x, x0, target, n);
-  GB_CUDA_TRY(cudaGetLastError());
+    GB_CUDA_TRY(launch_after(target_kernel<1>, stream_blocks(n), kBlock, st, atol, rtol, x, x0,
+                             target, n));
   return GB_OK;
 }
 

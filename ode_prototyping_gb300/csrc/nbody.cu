@@ -24,11 +24,11 @@ enum { kModeRhs = 0, kModeAccWrite = 1, kModeAccAdd = 2 };
 
 // AFTER: the launch overlaps the kernel before it in the stream.  For grids of
 // at most 4 CTAs per SM, whose launches are short (N = 257 FP64 10.25 -> 8.96 us
-// a call, 3001 1846 -> 1807 us for 24 steps of leapfrog; N = 4096 mixed 28.7 -> 24.7
+// a call, 3001 1846 -> 1807 us for 16 steps of leapfrog; N = 4096 mixed 28.7 -> 24.7
 // us); beyond that the loops run 0.3-0.6 % faster with their pointers left
 // __restrict__ (N = 16384 FP64, 100003 mixed).  A kernel of at most kFewCtas CTAs
 // lets the next one's wait beside it; more of them leave the next kernel's
-// unevenly spread over the SMs (3001: 2088 us for the 24 steps where they may).
+// unevenly spread over the SMs (3001: 2088 us for the 16 steps where they may).
 constexpr unsigned kFewCtas = 76;
 constexpr int kAfterCtasPerSm = 4;
 template <int T, int L, bool AFTER = false>

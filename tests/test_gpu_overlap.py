@@ -74,3 +74,19 @@ def test_captured_chain(gb, torch_cuda):
     torch.cuda.synchronize()
     for a, b in zip(want, got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("precision", ["f64", "mixed"])
+@pytest.mark.parametrize("n", [1, 304, 1365, 1366, 3001])
+def test_leapfrog_equals_single_steps(gb, torch_cuda, n, precision):
+    """1365 / 1366 bodies: 16 and 17 CTAs of the drift and kick kernels.  A step at a time starts
+    from a fresh a(x), the same bits as the a(x) kept from the step before."""
+    x0 = gb.to_device(np.random.default_rng(n).standard_normal(6 * n))
+    ode, exe = gb.NBodyODE(n, 0.05, 1.0 / n), gb.Gb300Executor(precision=precision)
+    step = gb.ParallelLeapfrogIntegrator.integrate
+    want = x0
+    for _ in range(6):
+        want, _ = step(want, 0.0, 1 / 64, 1 / 64, ode, None, exe)
+        torch_cuda.cuda.synchronize()
+    got, _ = step(x0, 0.0, 6 / 64, 1 / 64, ode, None, exe)
+    assert torch_cuda.equal(got, want)

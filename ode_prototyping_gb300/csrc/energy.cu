@@ -62,11 +62,12 @@ __device__ __noinline__ double pot_f64(const double* __restrict__ pos, long long
 }
 
 // The same in fixed point on the grid of ex; close pairs in FP64.
-template <bool MASS>
+template <int MASSES>
 __device__ __noinline__ double pot_fx(const double* __restrict__ pos, long long n, long long i0,
                                       long long vb, long long ve, long long span, double eps2,
                                       const double* __restrict__ masses, int ex, int em,
                                       FxBody* rec, const FxRow* tab) {
+  constexpr bool MASS = MASSES != kFxEqual, CLASSES = MASSES == kFxClasses;
   const int b = threadIdx.x;
   const long long i = min(i0 + b, n - 1);
   const Fx96 xi = fx_from_double(pos[3 * i], ex), yi = fx_from_double(pos[3 * i + 1], ex),
@@ -76,43 +77,43 @@ __device__ __noinline__ double pot_fx(const double* __restrict__ pos, long long 
   double near = 0.0;
   for (long long v0 = vb; v0 < ve; v0 += kT) {
     const int cnt = (int)min((long long)kT, ve - v0);
-    __syncthreads();
-    if (b < cnt) {
-      const long long j = (i0 + v0 + b) % n;
-      FxBody r;
-      r.x = fx_from_double(pos[3 * j], ex);
-      r.y = fx_from_double(pos[3 * j + 1], ex);
-      r.z = fx_from_double(pos[3 * j + 2], ex);
-      r.mu_lo = r.mu_hi = 0;
-      r.q = 0;
-      if (MASS) fx_mass(r, masses[j], em);
-      rec[b] = r;
-    }
-    __syncthreads();
-    // partner k counts where 0 <= k - first < span
+    fx_stage<MASSES>(rec, pos, masses, (i0 + v0 + b) % n, cnt, ex, em, kT, b, 0);
+    // the tile's partner k counts where 0 <= k - first < span
     const long long first = b + 1 - v0;
-    for (int c = 0; c < cnt; c += kFxChunk) {
-      const int end = min(cnt, c + kFxChunk);
+    for (int c = 0, end; c < cnt; c = end) {
+      end = min(cnt, c + kFxChunk);
+      int run = cnt, cls = 0;
+      if (CLASSES) {
+        run = fx_tag_end(rec[c].tag);
+        cls = fx_tag_class(rec[c].tag);
+        end = min(end, run);
+      }
+      const bool light = CLASSES && cls == kFxClassFp64;
       unsigned mask = 0;
       FxAcc a = {};
 #pragma unroll 2
       for (int k = c; k < end; ++k) {
-        const bool on = (unsigned long long)(k - first) < (unsigned long long)span;
+        const int at = CLASSES ? fx_tag_index(rec[k].tag) : k;
+        const bool on = (unsigned long long)(at - first) < (unsigned long long)span;
         const int norm = fx_term_pot<MASS>(rec[k], xi, yi, zi, eps2f, tab, on, a);
-        mask = (mask << 1) | (on && norm > kFxMaxK ? 1u : 0u);
+        mask = (mask << 1) | (on && (light || norm > kFxMaxK) ? 1u : 0u);
       }
-      fx_fold(tot, a);
+      if (!light) fx_fold(tot, a);
       while (mask) {  // close pairs
         const int k = end - 32 + __clz(mask);
         mask &= ~(0x80000000u >> __clz(mask));
-        const long long j = (i0 + v0 + k) % n;
+        const long long j = (i0 + v0 + (CLASSES ? fx_tag_index(rec[k].tag) : k)) % n;
         const double dx = pos[3 * j] - pos[3 * i], dy = pos[3 * j + 1] - pos[3 * i + 1],
                      dz = pos[3 * j + 2] - pos[3 * i + 2];
         near += (MASS ? masses[j] : 1.0) / sqrt(dx * dx + dy * dy + dz * dz + eps2);
       }
+      if (CLASSES && end == run) {  // the class's sum in the tile
+        near += fx_to_double(tot, fx_out_exp_pot(ex) + fx_class_exp(em, cls) + 3);
+        tot = 0;
+      }
     }
   }
-  return fx_to_double(tot, fx_out_exp_pot(ex) + (MASS ? em + 3 : 0)) + near;
+  return fx_to_double(tot, fx_out_exp_pot(ex) + (MASS ? fx_class_exp(em, 0) + 3 : 0)) + near;
 }
 
 __global__ void __launch_bounds__(kT, kCtasPerSm)
@@ -138,12 +139,15 @@ __global__ void __launch_bounds__(kT, kCtasPerSm)
   FxBody* rec = reinterpret_cast<FxBody*>(sh_raw);
   FxRow* tab = reinterpret_cast<FxRow*>(rec + kT);
   int ex, em;
+  bool classes;
   if (fx_grid(pos, n, min(i, n - 1), (i0 + vb) % n, min(n, ve - vb), eps2, masses,
-              reinterpret_cast<int*>(tab + kFxRows), kT, threadIdx.x, 0, &ex, &em)) {
+              reinterpret_cast<int*>(tab + kFxRows), kT, threadIdx.x, 0, &ex, &em, &classes)) {
     if (threadIdx.x < kFxRows) tab[threadIdx.x] = fx_row(threadIdx.x, eps2, ex);
     part[threadIdx.x] =
-        masses ? pot_fx<true>(pos, n, i0, vb, ve, span, eps2, masses, ex, em, rec, tab)
-               : pot_fx<false>(pos, n, i0, vb, ve, span, eps2, nullptr, ex, 0, rec, tab);
+        !masses ? pot_fx<kFxEqual>(pos, n, i0, vb, ve, span, eps2, nullptr, ex, 0, rec, tab)
+        : !classes
+            ? pot_fx<kFxOneClass>(pos, n, i0, vb, ve, span, eps2, masses, ex, em, rec, tab)
+            : pot_fx<kFxClasses>(pos, n, i0, vb, ve, span, eps2, masses, ex, em, rec, tab);
   } else {
     part[threadIdx.x] = pot_f64(pos, n, i0, vb, ve, span, eps2, masses,
                                 reinterpret_cast<double*>(sh_raw));

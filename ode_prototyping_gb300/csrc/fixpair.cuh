@@ -43,6 +43,12 @@ namespace gb {
 
 constexpr int kFxMaxK = 13;       // largest normalisation inside the window
 constexpr int kFxRows = kFxMaxK + 2;  // table rows (the last: weight 0)
+// with per-body masses, whose weight is 4^k times up to 8
+constexpr int kFxMaxKMass = 11;
+template <bool MASS>
+constexpr int fx_max_k() {
+  return MASS ? kFxMaxKMass : kFxMaxK;
+}
 
 struct Fx96 {  // two's complement, w0 least significant
   uint32_t w0, w1, w2;
@@ -182,10 +188,10 @@ GB_HD Fx96 fx_sub(const Fx96& a, const Fx96& b) {
   return r;
 }
 
-// Normalisation of a difference from the high words, clamped to kFxMaxK + 1:
+// Normalisation of a difference from the high words, clamped to max_k + 1:
 // R 4^k in [2^60 (1 - 2^-8), 2^62 (1 - 2^-9)], so that every component's high
 // word stays below 2^31 (the high words, truncated, know r to 2^-13 at k = 13).
-GB_HD int fx_norm(const Fx96& dx, const Fx96& dy, const Fx96& dz, float eps2f) {
+GB_HD int fx_norm(const Fx96& dx, const Fx96& dy, const Fx96& dz, float eps2f, int max_k) {
   const float fx = (float)(int32_t)dx.w2, fy = (float)(int32_t)dy.w2, fz = (float)(int32_t)dz.w2;
 #ifdef __CUDA_ARCH__
   const float f = __fmaf_rn(fx, fx, __fmaf_rn(fy, fy, __fmaf_rn(fz, fz, eps2f)));
@@ -193,7 +199,7 @@ GB_HD int fx_norm(const Fx96& dx, const Fx96& dy, const Fx96& dz, float eps2f) {
   const float f = fx * fx + fy * fy + fz * fz + eps2f;
 #endif
   const int k = (int)((0x5e7fffffu - 0x8000u - fx_float_bits(f)) >> 24);
-  return k < kFxMaxK + 1 ? k : kFxMaxK + 1;
+  return k < max_k + 1 ? k : max_k + 1;
 }
 
 struct FxDiff {  // a normalised component: (h 2^31 + l), 0 <= l < 2^31
@@ -327,14 +333,29 @@ GB_HD FxRow fx_row(int k, double eps2, int ex) {
   return FxRow{(uint32_t)e, (uint32_t)(e >> 32), k <= kFxMaxK ? 1u << (2 * k) : 0u, 0u};
 }
 
-// A partner's record.  Per-body masses: mass = mu 2^(em + q - 61) with mu in
-// [2^61, 2^62), q <= 0, em the largest mass's exponent; mu = 0 for a mass of 0.
+// A partner's record.  Per-body masses come in classes of four binary orders,
+// class c the exponents em - 4 c - 3 ... em - 4 c with em the largest mass's:
+// mass = mu 2^(eb + q - 61), mu in [2^61, 2^62), eb the class's lowest exponent
+// and 0 <= q <= 3, mu = 0 for a mass of 0.  Every class has sums of its own
+// (fx_class_exp), so a term keeps its bits however light its partner is: the
+// heaviest body feels only the others.
 struct alignas(16) FxBody {
   Fx96 x, y, z;
   uint32_t mu_lo, mu_hi;
-  int32_t q;
+  uint32_t tag;  // q, class, index in the tile, end of the class's run of records
 };
 
+constexpr int kFxClassFp64 = 255;  // masses below 2^-300: terms in FP64
+GB_HD uint32_t fx_tag(int q, int cls, int index, int end) {
+  return (uint32_t)(q | cls << 2 | index << 10 | end << 18);
+}
+GB_HD int fx_tag_q(uint32_t t) { return (int)(t & 3); }
+GB_HD int fx_tag_class(uint32_t t) { return (int)(t >> 2 & 255); }
+GB_HD int fx_tag_index(uint32_t t) { return (int)(t >> 10 & 255); }
+GB_HD int fx_tag_end(uint32_t t) { return (int)(t >> 18); }
+GB_HD int fx_class_exp(int em, int cls) { return em - 4 * cls - 3; }
+
+// Mantissa and tag (class and q) of a mass; em - 300 exponents at most.
 GB_HD void fx_mass(FxBody& b, double mass, int em) {
 #ifdef __CUDA_ARCH__
   const uint64_t bits = (uint64_t)__double_as_longlong(mass);
@@ -342,31 +363,30 @@ GB_HD void fx_mass(FxBody& b, double mass, int em) {
   uint64_t bits;
   memcpy(&bits, &mass, 8);
 #endif
-  const int e = (int)((bits >> 52) & 0x7ff);
-  const uint64_t mu = e ? ((bits & 0xfffffffffffffull) | (1ull << 52)) << 9 : 0;
+  const int e = (int)((bits >> 52) & 0x7ff) - 1023;
+  const bool normal = e >= -300;
+  const uint64_t mu = normal ? ((bits & 0xfffffffffffffull) | (1ull << 52)) << 9 : 0;
   b.mu_lo = fx_lo(mu);
   b.mu_hi = fx_hi(mu);
-  b.q = e ? e - 1023 - em : 0;
+  const int down = normal ? em - e : 0;
+  b.tag = fx_tag(normal ? 3 - (down & 3) : 0,
+                 normal ? down >> 2 : bits << 1 ? kFxClassFp64 : 0, 0, 0);
 }
 
-// One term of the accelerations into the three sums; returns its
-// normalisation (kFxMaxK + 1: not added).  With masses the weight is 4^k 2^q:
-// what is below 1 shifts S right, which drops only bits below the heaviest
-// body's at the largest distance.
+// One term of the accelerations into the three sums; returns its normalisation
+// (above fx_max_k: not added).  With masses the weight is 4^k 2^q.
 template <bool MASS>
 GB_HD int fx_term(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& zi, float eps2f,
                   const FxRow* tab, FxAcc (&a)[3]) {
   const Fx96 ux = fx_sub(j.x, xi), uy = fx_sub(j.y, yi), uz = fx_sub(j.z, zi);
-  const int k = fx_norm(ux, uy, uz, eps2f);
+  const int k = fx_norm(ux, uy, uz, eps2f, fx_max_k<MASS>());
   const FxRow row = tab[k];
   const FxDiff dx = fx_scale(ux, k), dy = fx_scale(uy, k), dz = fx_scale(uz, k);
   uint64_t s = fx_rinv3(fx_r2(dx, dy, dz, fx_pair(row.e_lo, row.e_hi)));
   uint32_t p = row.p;
   if (MASS) {
-    s = fx_mul_hi(s << 2, fx_pair(j.mu_lo, j.mu_hi));  // S mass 2^(-em - q - 1)
-    const int t = 2 * k + j.q;
-    if (t < 0) s = t > -63 ? (s + (1ull << (-t - 1))) >> -t : 0;
-    p = k <= kFxMaxK ? 1u << (t > 0 ? t : 0) : 0u;
+    s = fx_mul_hi(s << 2, fx_pair(j.mu_lo, j.mu_hi));  // S mass 2^(-eb - q - 1)
+    p = k <= kFxMaxKMass ? p << fx_tag_q(j.tag) : 0u;
   }
   const int32_t sh = (int32_t)(s >> 31), sl = (int32_t)((uint32_t)s & 0x7fffffffu);
   fx_add(a[0], sh, sl, dx, p);
@@ -381,18 +401,14 @@ template <bool MASS>
 GB_HD int fx_term_pot(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& zi, float eps2f,
                       const FxRow* tab, bool on, FxAcc& a) {
   const Fx96 ux = fx_sub(j.x, xi), uy = fx_sub(j.y, yi), uz = fx_sub(j.z, zi);
-  const int k = fx_norm(ux, uy, uz, eps2f);
+  const int k = fx_norm(ux, uy, uz, eps2f, kFxMaxK);
   const FxRow row = tab[k];
   const FxDiff dx = fx_scale(ux, k), dy = fx_scale(uy, k), dz = fx_scale(uz, k);
   uint64_t y = fx_rinv1(fx_r2(dx, dy, dz, fx_pair(row.e_lo, row.e_hi)));
   int t = k;
   if (MASS) {
-    y = fx_mul_hi(y, fx_pair(j.mu_lo, j.mu_hi));  // y mass 2^(-em - q - 3)
-    t += j.q;
-    if (t < 0) {
-      y = t > -63 ? (y + (1ull << (-t - 1))) >> -t : 0;
-      t = 0;
-    }
+    y = fx_mul_hi(y, fx_pair(j.mu_lo, j.mu_hi));  // y mass 2^(-eb - q - 3)
+    t += fx_tag_q(j.tag);
   }
   const uint32_t p = on && k <= kFxMaxK ? 1u << t : 0u;
   a.h = (long long)fx_mad(fx_hi(y), p, (uint64_t)a.h);
@@ -401,8 +417,8 @@ GB_HD int fx_term_pot(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx9
 }
 
 // exponent of a term's unit: sum 2^(fx_out_exp(ex)) is the sum of d / r^3, and
-// sum 2^(fx_out_exp(ex) + em + 1) that of mass d / r^3; of the potential:
-// 1 / r, and with em + 3 mass / r
+// sum 2^(fx_out_exp(ex) + eb + 1) that of mass d / r^3; of the potential:
+// 1 / r, and with eb + 3 mass / r
 GB_HD int fx_out_exp(int ex) { return -60 - 2 * ex; }
 GB_HD int fx_out_exp_pot(int ex) { return -63 - ex; }
 

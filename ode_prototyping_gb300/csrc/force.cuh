@@ -162,7 +162,7 @@ struct WarpGroup {
 template <int T>
 constexpr int f64_smem_bytes() {
   // partner records (at least the 32 T bytes of the FP64 loop), table, reduction
-  return ((int)sizeof(FxBody) * T + (int)sizeof(FxRow) * kFxRows + 28 * (T / 32) + 15) / 16 * 16;
+  return ((int)sizeof(FxBody) * T + (int)sizeof(FxRow) * kFxRows + 32 * (T / 32) + 15) / 16 * 16;
 }
 
 // Pair terms of the FP64 loops.
@@ -197,12 +197,15 @@ __device__ __forceinline__ void add_pair_f64(const double* pos, long long i, lon
   }
 }
 
-// The partners of one lane's chunk (j0 + u L, u < steps) whose bits are set in
-// `mask` (bit steps - 1 - u) in FP64, lanes side by side: as many rounds as the
-// warp's lane with most of them, which is returned.  The whole warp calls it.
-static __device__ __noinline__ int fx_chunk_f64(unsigned mask, int steps, long long j0, int L,
-                                                const double* pos, long long i, double eps2,
-                                                const double* masses, bool ieee, double* s) {
+// The partners of one lane's chunk (records p0 + u L of the tile from j0 on,
+// u < steps) whose bits are set in `mask` (bit steps - 1 - u) in FP64, lanes side
+// by side: as many rounds as the warp's lane with most of them, which is
+// returned.  sorted: the records, where they are not in the order of the
+// bodies, else null.  The whole warp calls it.
+static __device__ __noinline__ int fx_chunk_f64(unsigned mask, int steps, long long j0, int p0,
+                                                int L, const FxBody* sorted, const double* pos,
+                                                long long i, double eps2, const double* masses,
+                                                bool ieee, double* s) {
   int rounds = 0;
 #pragma unroll 1
   while (__any_sync(0xffffffffu, mask != 0)) {
@@ -210,7 +213,9 @@ static __device__ __noinline__ int fx_chunk_f64(unsigned mask, int steps, long l
     if (mask) {
       const int u = steps - 32 + __clz(mask);
       mask &= ~(0x80000000u >> __clz(mask));
-      add_pair_f64(pos, i, j0 + (long long)u * L, eps2, masses, ieee, s);
+      const int p = p0 + u * L;
+      const long long j = j0 + (sorted ? fx_tag_index(sorted[p].tag) : p);
+      if (j != i) add_pair_f64(pos, i, j, eps2, masses, ieee, s);
     }
   }
   return rounds;
@@ -222,15 +227,60 @@ __device__ __forceinline__ void group_bar(int bar, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(threads) : "memory");
 }
 
+// Masses of a group's partners: all equal, per body within one class (fixpair.cuh),
+// per body of several classes.
+enum { kFxEqual = 0, kFxOneClass = 1, kFxClasses = 2 };
+
+// A tile's records: threads tid < cnt, of a group of T, each bring partner j.
+// With several classes the records are put in the order of their classes, the
+// heaviest first, each with the end of its class's run (a thread counts the
+// records before its own: 128 reads of the same word by all, 3 to 7 % of the
+// tile's pairs).
+template <int MASSES>
+__device__ __forceinline__ void fx_stage(FxBody* rec, const double* __restrict__ pos,
+                                         const double* __restrict__ masses, long long j, int cnt,
+                                         int ex, int em, int T, int tid, int bar) {
+  group_bar(bar, T);  // the tile before is read
+  FxBody r;
+  if (tid < cnt) {
+    r.x = fx_from_double(pos[3 * j], ex);
+    r.y = fx_from_double(pos[3 * j + 1], ex);
+    r.z = fx_from_double(pos[3 * j + 2], ex);
+    r.mu_lo = r.mu_hi = r.tag = 0;
+    if (MASSES != kFxEqual) fx_mass(r, masses[j], em);
+  }
+  int at = tid;
+  if (MASSES == kFxClasses) {
+    const int cls = tid < cnt ? fx_tag_class(r.tag) : 0;
+    if (tid < cnt) rec[tid].tag = (uint32_t)cls;
+    group_bar(bar, T);
+    if (tid < cnt) {
+      int before = 0, end = 0;
+#pragma unroll 4
+      for (int v = 0; v < cnt; ++v) {
+        const int c = (int)rec[v].tag;
+        before += c < cls || (c == cls && v < tid);
+        end += c <= cls;
+      }
+      at = before;
+      r.tag |= fx_tag(0, 0, tid, end);
+    }
+    group_bar(bar, T);
+  }
+  if (tid < cnt) rec[at] = r;
+  group_bar(bar, T);
+}
+
 // The tiles of one CTA or group.  Not inlined, and the geometry (T threads, L
 // lanes) a run-time value: the loop is long enough for the call, and a copy of
 // it in each of the FP64 kernels would make them slow to build.
-template <bool MASS>
+template <int MASSES>
 __device__ __noinline__ void force_fx_tiles(const double* __restrict__ pos, long long n,
                                             long long i0, long long jb, long long je, double eps2,
                                             const double* __restrict__ masses, int ex, int em,
                                             bool ieee, int T, int L, int tid, int bar,
                                             FxBody* rec, const FxRow* tab, double (*part)[3]) {
+  constexpr bool MASS = MASSES != kFxEqual, CLASSES = MASSES == kFxClasses;
   const int b = tid / L;
   const int l = tid % L;
   const long long i = i0 + b;
@@ -245,50 +295,64 @@ __device__ __noinline__ void force_fx_tiles(const double* __restrict__ pos, long
   __int128 tot[3] = {};
   double near[3] = {};
   bool in_f64 = false, any_near = false;  // uniform in the warp
+  int terms = 0, slow = 0;                // a lane's terms, and those of them in FP64
   for (long long j0 = jb; j0 < je; j0 += T) {
     const int cnt = (int)min((long long)T, je - j0);
-    group_bar(bar, T);
-    if (tid < cnt) {
-      const long long j = j0 + tid;
-      FxBody r;
-      r.x = fx_from_double(pos[3 * j], ex);
-      r.y = fx_from_double(pos[3 * j + 1], ex);
-      r.z = fx_from_double(pos[3 * j + 2], ex);
-      r.mu_lo = r.mu_hi = 0;
-      r.q = 0;
-      if (MASS) fx_mass(r, masses[j], em);
-      rec[tid] = r;
-    }
-    group_bar(bar, T);
-    for (int c0 = l; c0 - l < cnt; c0 += kFxChunk * L) {
-      const int end = min(cnt, c0 + kFxChunk * L);
+    fx_stage<MASSES>(rec, pos, masses, j0 + tid, cnt, ex, em, T, tid, bar);
+    for (int base = 0, end; base < cnt; base = end) {
+      end = min(cnt, base + kFxChunk * L);
+      int run = cnt, cls = 0;
+      if (CLASSES) {
+        run = fx_tag_end(rec[base].tag);
+        cls = fx_tag_class(rec[base].tag);
+        end = min(end, run);
+      }
+      const int c0 = base + l;
       const int steps = c0 < end ? (end - c0 + L - 1) / L : 0;
-      unsigned mask = in_f64 && steps ? 0xffffffffu >> (32 - steps) : 0u;
-      if (!in_f64) {
+      const bool light = CLASSES && cls == kFxClassFp64;
+      unsigned mask = (in_f64 || light) && steps ? 0xffffffffu >> (32 - steps) : 0u;
+      if (!in_f64 && !light) {
         FxAcc a[3] = {};
         // unrolled twice: 1.59 ms at N = 16384 against 1.72 ms (1) and 1.73 ms (4)
 #pragma unroll 2
         for (int jj = c0; jj < end; jj += L) {
           const int k = fx_term<MASS>(rec[jj], xi, yi, zi, eps2f, tab, a);
-          mask = __funnelshift_l((unsigned)(kFxMaxK - k), mask, 1);  // 1 when k > kFxMaxK
+          mask = __funnelshift_l((unsigned)(fx_max_k<MASS>() - k), mask, 1);  // 1 when k is above
         }
 #pragma unroll
         for (int d = 0; d < 3; ++d) fx_fold(tot[d], a[d]);
       }
+      int rounds = 0;
       if (__any_sync(0xffffffffu, mask != 0)) {
         if (!valid) mask = 0;
         const long long self = i - j0 - c0;  // not the body itself
-        if (self >= 0 && self < (long long)steps * L && self % L == 0)
+        if (!CLASSES && self >= 0 && self < (long long)steps * L && self % L == 0)
           mask &= ~(1u << (steps - 1 - (int)self / L));
-        const int rounds = fx_chunk_f64(mask, steps, j0 + c0, L, pos, i, eps2, masses, ieee, near);
-        // an FP64 term costs 5 fixed-point ones: where a lane needs more than 4
-        // in 5 of its terms in FP64, the others' are not worth their time
-        in_f64 = in_f64 || rounds > kFxChunk * 4 / 5;
+        rounds = fx_chunk_f64(mask, steps, j0, c0, L, CLASSES ? rec : nullptr, pos, i, eps2,
+                              masses, ieee, near);
         any_near = any_near || rounds > 0;
+      }
+      // an FP64 term costs 5 fixed-point ones: where a lane needs more than 4 in 5
+      // of a chunk's terms in FP64, the others' are not worth their time
+      if (!light) {
+        terms += (end - base + L - 1) / L;
+        slow += rounds;
+        if (terms >= kFxChunk) {
+          in_f64 = in_f64 || slow > terms * 4 / 5;
+          terms = slow = 0;
+        }
+      }
+      if (CLASSES && end == run) {  // the class's sums in the tile
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          near[d] = dadd(near[d], fx_to_double(tot[d], fx_out_exp(ex) + fx_class_exp(em, cls) + 1));
+          tot[d] = 0;
+        }
+        any_near = true;
       }
     }
   }
-  const int sc = fx_out_exp(ex) + (MASS ? em + 1 : 0);
+  const int sc = fx_out_exp(ex) + (MASS ? fx_class_exp(em, 0) + 1 : 0);
   for (int off = L / 2; off >= 1; off /= 2) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -321,8 +385,8 @@ __device__ __forceinline__ double key_bound(int key, bool upper) {
 }
 
 // The grid of a group's own body i and of the `count` partners from jb on
-// (modulo n): exponents ex and, with masses, em; red holds 7 words a warp.
-// Returns false, uniformly in the group, when there is no grid: a coordinate
+// (modulo n): exponents ex and, with masses, em, and whether the masses are of
+// more than one class; red holds 8 words a warp.  Returns false, uniformly in the group, when there is no grid: a coordinate
 // that is not finite, bodies all within a sixteenth of the softening,
 // exponents beyond 2^+-300, or a mass that is negative, not finite or all of
 // them zero.
@@ -330,10 +394,10 @@ static __device__ __noinline__ bool fx_grid(const double* __restrict__ pos, long
                                             long long i, long long jb, long long count,
                                             double eps2, const double* __restrict__ masses,
                                             int* red, int T, int tid, int bar, int* ex_out,
-                                            int* em_out) {
+                                            int* em_out, bool* classes_out) {
   const int nw = T / 32;
   int lo[3], hi[3];
-  unsigned mm = 0;
+  unsigned mm = 0, ml = 0xffffffffu;
 #pragma unroll
   for (int c = 0; c < 3; ++c) lo[c] = hi[c] = order_key(pos[3 * i + c]);
 #pragma unroll 4
@@ -351,33 +415,38 @@ static __device__ __noinline__ bool fx_grid(const double* __restrict__ pos, long
 #pragma unroll 4
     for (long long v = tid; v < count; v += T) {
       const long long j = jb + v < n ? jb + v : jb + v - n;
-      mm = max(mm, (unsigned)__double2hiint(masses[j]));
+      const unsigned m = (unsigned)__double2hiint(masses[j]);
+      mm = max(mm, m);
+      if (m | (unsigned)__double2loint(masses[j])) ml = min(ml, m);
     }
   }
   mm = __reduce_max_sync(0xffffffffu, mm);
+  ml = __reduce_min_sync(0xffffffffu, ml);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     lo[c] = __reduce_min_sync(0xffffffffu, lo[c]);
     hi[c] = __reduce_max_sync(0xffffffffu, hi[c]);
   }
   if ((tid & 31) == 0) {
-    int* r = red + 7 * (tid / 32);
+    int* r = red + 8 * (tid / 32);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       r[c] = lo[c];
       r[3 + c] = hi[c];
     }
     r[6] = (int)mm;
+    r[7] = (int)ml;
   }
   group_bar(bar, T);
   for (int w = 0; w < nw; ++w) {
-    const int* r = red + 7 * w;
+    const int* r = red + 8 * w;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       lo[c] = min(lo[c], r[c]);
       hi[c] = max(hi[c], r[3 + c]);
     }
     mm = max(mm, (unsigned)r[6]);
+    ml = min(ml, (unsigned)r[7]);
   }
   constexpr int kInf = 0x7ff00000;
   int xe = 0;
@@ -398,6 +467,7 @@ static __device__ __noinline__ bool fx_grid(const double* __restrict__ pos, long
   if (ex < -300 || ex > 300 || (masses && (em < -300 || em > 300))) return false;
   *ex_out = ex;
   *em_out = em;
+  *classes_out = masses && (int)(ml >> 20) < (int)(mm >> 20) - 3;
   return true;
 }
 
@@ -413,16 +483,20 @@ static __device__ __noinline__ bool force_fx_group(const double* __restrict__ po
   FxRow* tab = reinterpret_cast<FxRow*>(rec + T);
   int* red = reinterpret_cast<int*>(tab + kFxRows);
   int ex, em;
+  bool classes;
   if (!fx_grid(pos, n, min(i0 + tid / L, n - 1), jb, je - jb, eps2, masses, red, T, tid, bar, &ex,
-               &em))
+               &em, &classes))
     return false;
   if (tid < kFxRows) tab[tid] = fx_row(tid, eps2, ex);
-  if (masses)
-    force_fx_tiles<true>(pos, n, i0, jb, je, eps2, masses, ex, em, ieee, T, L, tid, bar, rec, tab,
-                         part);
+  if (!masses)
+    force_fx_tiles<kFxEqual>(pos, n, i0, jb, je, eps2, nullptr, ex, 0, ieee, T, L, tid, bar, rec,
+                             tab, part);
+  else if (!classes)
+    force_fx_tiles<kFxOneClass>(pos, n, i0, jb, je, eps2, masses, ex, em, ieee, T, L, tid, bar,
+                                rec, tab, part);
   else
-    force_fx_tiles<false>(pos, n, i0, jb, je, eps2, nullptr, ex, 0, ieee, T, L, tid, bar, rec,
-                          tab, part);
+    force_fx_tiles<kFxClasses>(pos, n, i0, jb, je, eps2, masses, ex, em, ieee, T, L, tid, bar,
+                               rec, tab, part);
   return true;
 }
 

@@ -115,6 +115,14 @@ constexpr int batch_smem_bytes() {
                              : (TG <= 128 ? jp_smem_bytes<TG>() : (int)sizeof(PackedBody) * TG);
 }
 
+// Of a CTA of T threads that runs one unit or G of them side by side: a group's
+// staging has parts that do not shrink with it (FP64: the softening table), so G
+// of T / G threads may need more than one of T.
+template <int PREC, int T, int G>
+constexpr int batch_cta_smem_bytes() {
+  return std::max(batch_smem_bytes<PREC, T>(), G * batch_smem_bytes<PREC, T / G>());
+}
+
 // One unit (system, i-tile) of one stage, run by TG threads (the whole CTA,
 // or one warp group of it): the tile's accelerations against every body of
 // its system, then the shared stage epilogue for the tile's bodies.
@@ -212,7 +220,7 @@ __global__ void __launch_bounds__(T, PREC == GB_PREC_F64 ? 4 * 128 / T : 1)
   static_assert(G == 1 || (T / G >= 32 && T <= 128 && (T / G / L) * BPT >= 1),
                 "systems per CTA: warp groups of the packed loop");
   constexpr int BI = (T / L) * BPT;
-  constexpr int SMEM_BODY_BYTES = batch_smem_bytes<PREC, T>();
+  constexpr int SMEM_BODY_BYTES = batch_cta_smem_bytes<PREC, T, G>();
   __shared__ __align__(16) unsigned char sh_raw[SMEM_BODY_BYTES];
   __shared__ double part[BI][3];
   __shared__ double red[T];
@@ -333,7 +341,7 @@ __global__ void __launch_bounds__(T)
     batch_rhs_kernel(const __grid_constant__ BatchParams P, const double* __restrict__ x,
                      const PackedBody* __restrict__ packed, double* __restrict__ out) {
   constexpr int BI = (T / L) * BPT;
-  __shared__ __align__(16) unsigned char sh_raw[batch_smem_bytes<PREC, T>()];
+  __shared__ __align__(16) unsigned char sh_raw[batch_cta_smem_bytes<PREC, T, G>()];
   __shared__ double part[BI][3];
   for (long long w = blockIdx.x; w < P.n_work; w += gridDim.x) {
     const int2 item = P.work[w];

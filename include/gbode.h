@@ -117,11 +117,14 @@ typedef struct {
                             (per-body masses run the scalar loop) */
   int32_t f64_pair;      /* FP64 pair term: 0 = the entry point's default, 1 = fixed-point
                             terms on the integer pipes (each within 2^-55 of its size, the
-                            sums of a CTA exact), with r^-3 from a Newton-refined reciprocal
-                            square root in FP64 (a few ulp per term) for pairs closer than
-                            about 2^-12 of the system's extent and where fixed point does
-                            not apply (coordinates that are not finite, exponents beyond
-                            2^+-300, negative masses, an extent far below the softening),
+                            sums of a CTA exact; a component whose terms are far smaller than
+                            the whole terms has its sum with more words or in FP64), with
+                            r^-3 from a Newton-refined reciprocal square root in FP64 (a few
+                            ulp per term) for pairs closer than about 2^-12 of the system's
+                            extent (2^-10 with masses), masses below 2^-300, and where fixed
+                            point does not apply (coordinates that are not finite, exponents
+                            beyond 2^+-300, negative masses, an extent far below the
+                            softening, one far below another),
                             2 = the reference's operation order (IEEE sqrt and divisions,
                             NBodyODE.hpp:89-98).  The integrator's FP64 stages default to 1
                             (exact mode: 2).  The standalone right-hand sides default to 2

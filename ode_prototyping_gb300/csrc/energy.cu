@@ -140,8 +140,9 @@ __global__ void __launch_bounds__(kT, kCtasPerSm)
   FxRow* tab = reinterpret_cast<FxRow*>(rec + kT);
   int ex, em;
   bool classes;
+  FxShape shape;
   if (fx_grid(pos, n, min(i, n - 1), (i0 + vb) % n, min(n, ve - vb), eps2, masses,
-              reinterpret_cast<int*>(tab + kFxRows), kT, threadIdx.x, 0, &ex, &em, &classes)) {
+              reinterpret_cast<int*>(tab + kFxRows), kT, threadIdx.x, 0, &ex, &em, &classes, &shape)) {
     if (threadIdx.x < kFxRows) tab[threadIdx.x] = fx_row(threadIdx.x, eps2, ex);
     part[threadIdx.x] =
         !masses ? pot_fx<kFxEqual>(pos, n, i0, vb, ve, span, eps2, nullptr, ex, 0, rec, tab)

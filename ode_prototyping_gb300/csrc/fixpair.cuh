@@ -6,9 +6,8 @@
 // 18 of them even with a refined reciprocal square root.  Here the whole term
 // is fixed point: positions are 96-bit integers on a grid common to the bodies
 // a CTA reads, so the difference of two is exact; r^2, its reciprocal square
-// root, r^-3 and the products keep 57 bits or more; and the sums are integers,
-// exact and independent of the order.  36 IMAD.WIDE and about 75 simple
-// instructions per term.
+// root and r^-3 keep 57 bits or more; and the sums are integers, exact and
+// independent of the order.  33 IMAD.WIDE per term.
 //
 // Scales.  The grid is U = 2^(Ex - 94) with |x_j - x_i| < 2^Ex in every
 // component and eps < 2^(Ex - 1); coordinates are taken modulo 2^96 U, so only
@@ -19,15 +18,18 @@
 // sums' window: they get weight 0 here and are added by the caller in FP64.
 //
 // Error: d is exact where a coordinate's last bit is a multiple of U (every
-// coordinate above 2^-41 2^Ex) and enters with 62 bits; R and the Newton
-// residual hold 2^-58.  A term is within 2^-55 of its size (0.04 2^-53 rms; a
-// term in FP64: 1.3 2^-53 rms, up to 5 2^-53).
+// coordinate above 2^-41 2^Ex); R and the Newton residual hold 2^-58.  A term is
+// within 2^-55 of its size (0.04 2^-53 rms; a term in FP64: 1.3 2^-53 rms, up to
+// 5 2^-53).  Its components are products of two words' precision, 2^-57 of the
+// term and not of the component; the sizes of a sum's terms and of their
+// components say where that is not enough (kFxNarrow, kFxThin), and those sums
+// are taken with three words or in FP64, so that every component is as good as
+// its FP64 sum.
 //
-// Measured at N = 16384 (right-hand side): 1.6 ms against 22.3 ms for the FP64
+// Measured at N = 16384 (right-hand side): 1.65 ms against 22.3 ms for the FP64
 // loop in the reference's operation order and 12 ms with the refined
-// reciprocal square root; about 111 instructions and 220 cycles of a
-// sub-partition per 32 terms, the multiply-add pipe (4 cycles for an IMAD.WIDE)
-// 80 % busy.
+// reciprocal square root (1.60 ms with two words and no look at the components,
+// 1.92 ms with three words everywhere).
 #pragma once
 
 #include <cstdint>
@@ -54,17 +56,22 @@ struct Fx96 {  // two's complement, w0 least significant
   uint32_t w0, w1, w2;
 };
 
-// row k of the softening table: eps^2 at normalisation k, the weight 4^k
+// row k of the softening table: eps^2 at normalisation k, the weight 4^k twice
 struct alignas(16) FxRow {
   uint32_t e_lo, e_hi;
   uint32_t p;
-  uint32_t pad;
+  float pf;
 };
 
-struct FxAcc {  // sum of the terms, weight 2^32, 1 and 2
+struct FxAcc {  // sum of the terms, weight 2^64, 1 and 2^32
   long long h;
   unsigned long long l;
-  long long m;
+  unsigned long long m;
+};
+
+struct FxTot {  // sum of FxAcc, 160 bits two's complement
+  unsigned __int128 l;
+  int32_t h;
 };
 
 // 32 x 32 -> 64 bit products and words, each one instruction.  In PTX: from C
@@ -144,6 +151,24 @@ GB_HD uint32_t fx_float_bits(float f) {
 #endif
 }
 
+GB_HD float fx_abs(float v) {
+#ifdef __CUDA_ARCH__
+  return fabsf(v);
+#else
+  return __builtin_fabsf(v);
+#endif
+}
+
+GB_HD float fx_float_of(uint32_t u) {
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(u);
+#else
+  float f;
+  memcpy(&f, &u, 4);
+  return f;
+#endif
+}
+
 // v in units of U = 2^(ex - 94) modulo 2^96, truncated (exact when v is a
 // multiple of U).
 GB_HD Fx96 fx_from_double(double v, int ex) {
@@ -202,33 +227,44 @@ GB_HD int fx_norm(const Fx96& dx, const Fx96& dy, const Fx96& dz, float eps2f, i
   return k < max_k + 1 ? k : max_k + 1;
 }
 
-struct FxDiff {  // a normalised component: (h 2^31 + l), 0 <= l < 2^31
+// A normalised component, h 2^32 + l + ll 2^-32.  The middle word is signed, so
+// that its products with a signed word are single instructions.
+struct FxDiff {
   int32_t h, l;
+  uint32_t ll;
 };
 
 GB_HD FxDiff fx_scale(const Fx96& d, int k) {
-  return FxDiff{(int32_t)fx_shl(d.w1, d.w2, k), (int32_t)(fx_shl(d.w0, d.w1, k) >> 1)};
+  const uint32_t w1 = fx_shl(d.w0, d.w1, k);
+  return FxDiff{(int32_t)(fx_shl(d.w1, d.w2, k) + (w1 >> 31)), (int32_t)w1, d.w0 << k};
 }
 
 // R = (|d|^2 + eps^2) 4^k; the table's eps^2 carries the mean of what is dropped.
 GB_HD uint64_t fx_r2(const FxDiff& x, const FxDiff& y, const FxDiff& z, uint64_t eps2) {
   int64_t a = fx_mads(z.h, z.h, fx_mads(y.h, y.h, fx_mads(x.h, x.h, (int64_t)eps2)));
   const int64_t b = fx_mads(z.h, z.l, fx_mads(y.h, y.l, fx_muls(x.h, x.l)));
-  return (uint64_t)fx_mads((int32_t)fx_hi((uint64_t)b), 4, a);
+  return (uint64_t)fx_mads((int32_t)fx_hi((uint64_t)b), 2, a);
 }
 
 // Y <= 2^61 / sqrt(R), within 2^-19.9 of it from below: 24 bits from the SFU's
 // reciprocal square root (relative error <= 2^-22.9), scaled down by 5 2^-24
 // so that the residual 1 - R Y^2 / 2^122 is positive.
-GB_HD uint32_t fx_rsqrt_seed(uint64_t r) {
+GB_HD float fx_rsqrt_seed_float(uint64_t r) {
   const float rh = (float)fx_hi(r);
   constexpr float kScale = 35184372088832.0f * (1.0f - 5.0f / 16777216.0f);
 #ifdef __CUDA_ARCH__
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(rh));
-  return __float2uint_rz(__fmul_rn(y, kScale));
+  return __fmul_rn(y, kScale);
 #else
-  return (uint32_t)((float)(1.0 / __builtin_sqrt((double)rh)) * kScale);
+  return (float)(1.0 / __builtin_sqrt((double)rh)) * kScale;
+#endif
+}
+GB_HD uint32_t fx_rsqrt_seed(float y) {
+#ifdef __CUDA_ARCH__
+  return __float2uint_rz(y);
+#else
+  return (uint32_t)y;
 #endif
 }
 
@@ -255,36 +291,56 @@ GB_HD uint64_t fx_mul_hi(uint64_t a, uint64_t b) {
   return fx_mad(fx_hi(a), fx_hi(b), fx_pair(fx_hi(m), 0));
 }
 
-// S = 2^151 R^(-3/2) = Y^3 (1 - e)^(-3/2) (in [2^58, 2^61]).
-GB_HD uint64_t fx_rinv3(uint64_t r) {
-  const uint32_t y = fx_rsqrt_seed(r);
+// S = 2^151 R^(-3/2) = Y^3 (1 - e)^(-3/2) (in [2^58, 2^61]); yf = Y.
+GB_HD uint64_t fx_rinv3(uint64_t r, float& yf) {
+  yf = fx_rsqrt_seed_float(r);
+  const uint32_t y = fx_rsqrt_seed(yf);
   const uint64_t q = fx_mul(y, y);
   return fx_mul_hi(fx_refine(y, fx_residual(r, q), 96u, 30u), q);
 }
 
 // 2^93 R^(-1/2) = Y (1 - e)^(-1/2) 2^32 (in [2^62, 2^63]).
 GB_HD uint64_t fx_rinv1(uint64_t r) {
-  const uint32_t y = fx_rsqrt_seed(r);
+  const uint32_t y = fx_rsqrt_seed(fx_rsqrt_seed_float(r));
   return fx_refine(y, fx_residual(r, fx_mul(y, y)), 32u, 6u);
 }
 
-// Adds weight p times the component S (h 2^31 + l) / 2^62.
-GB_HD void fx_add(FxAcc& a, int32_t sh, int32_t sl, const FxDiff& d, uint32_t p) {
-  const uint64_t hh = (uint64_t)fx_muls(sh, d.h);
-  const uint64_t m = (uint64_t)fx_mads(sl, d.h, fx_mads(sh, d.l, 1ll << 31));
-  a.h = fx_mads((int32_t)fx_hi(hh), (int32_t)p, a.h);
-  a.l = fx_mad(fx_lo(hh), p, a.l);
-  a.m = fx_mads((int32_t)fx_hi(m), (int32_t)p, a.m);
+// Adds weight p times the component V = S (h 2^32 + l + ll 2^-32) / 2^32, of which
+// a term has 2^89 to 2^91.  With S split like the component, the words' carries go
+// through the multiply-adds' addends.  Two words, within 0.8 2^32 (2^-57 of the
+// term), or, WIDE, three, within 2: the parts that two drop are all that a
+// component far smaller than the distance has.
+template <bool WIDE>
+GB_HD void fx_add(FxAcc& a, uint64_t s, const FxDiff& d, uint32_t p) {
+  const int32_t sl = (int32_t)fx_lo(s), sh = (int32_t)(fx_hi(s) + (fx_lo(s) >> 31));
+  int64_t low = 1ll << 31;
+  if (WIDE) low = (int32_t)fx_hi((uint64_t)fx_mads(sl, d.l, (int64_t)fx_mul((uint32_t)sh, d.ll)));
+  const int64_t m = fx_mads(sl, d.h, fx_mads(sh, d.l, low));
+  const uint64_t h = (uint64_t)fx_mads(sh, d.h, (int32_t)fx_hi((uint64_t)m));
+  a.h = fx_mads((int32_t)fx_hi(h), (int32_t)p, a.h);
+  a.m = fx_mad(fx_lo(h), p, a.m);
+  if (WIDE) a.l = fx_mad(fx_lo((uint64_t)m), p, a.l);
 }
 
-// Terms added between two folds: a.l stays below 2^63 (2^32 2^26 a term).
+// Terms added between two folds: a.l and a.m stay below 2^63 (2^32 2^26 a term).
 constexpr int kFxChunk = 32;
 
 GB_HD void fx_fold(__int128& tot, FxAcc& a) {
-  tot += ((__int128)a.h << 32) + (__int128)a.l + ((__int128)a.m << 1);
+  tot += ((__int128)a.h << 64) + ((__int128)a.m << 32) + (__int128)a.l;
   a.h = 0;
   a.l = 0;
   a.m = 0;
+}
+
+// A term is below 2^118 in size, a fold of 32 below 2^123: 2^36 folds.
+GB_HD void fx_tot_add(FxTot& t, unsigned __int128 l, int32_t h) {
+  t.l += l;
+  t.h += h + (t.l < l ? 1 : 0);
+}
+GB_HD void fx_fold(FxTot& tot, FxAcc& a) {
+  __int128 v = 0;
+  fx_fold(v, a);
+  fx_tot_add(tot, (unsigned __int128)v, v < 0 ? -1 : 0);
 }
 
 // v 2^sc to the nearest double (|v| < 2^126, the result's exponent in range).
@@ -316,6 +372,12 @@ GB_HD double fx_to_double(__int128 v, int sc) {
 #endif
 }
 
+GB_HD double fx_to_double(const FxTot& t, int sc) {
+  if (t.h == ((__int128)t.l < 0 ? -1 : 0)) return fx_to_double((__int128)t.l, sc);
+  const __int128 v = (__int128)((unsigned __int128)(uint32_t)t.h << 96 | t.l >> 32);
+  return fx_to_double(v | ((uint32_t)t.l != 0 ? 1 : 0), sc + 32);
+}
+
 // Row k of the softening table on the grid of ex: eps^2 in units of (2^64 U)^2
 // times 4^k, truncated (the 2 is the mean of what fx_r2 drops), 4^k as the
 // weight.  A row whose eps^2 does not fit is never read: R would exceed 2^62.
@@ -330,7 +392,8 @@ GB_HD FxRow fx_row(int k, double eps2, int ex) {
   const uint64_t m = ee ? (bits & 0xfffffffffffffull) | (1ull << 52) : 0;
   const int sh = ee - 1075 + 2 * (30 - ex + k);
   const uint64_t e = (sh > 9 ? 1ull << 62 : sh >= 0 ? m << sh : sh > -64 ? m >> -sh : 0) + 2;
-  return FxRow{(uint32_t)e, (uint32_t)(e >> 32), k <= kFxMaxK ? 1u << (2 * k) : 0u, 0u};
+  return FxRow{(uint32_t)e, (uint32_t)(e >> 32), k <= kFxMaxK ? 1u << (2 * k) : 0u,
+               k <= kFxMaxK ? (float)(1u << (2 * k)) : 0.0f};
 }
 
 // A partner's record.  Per-body masses come in classes of four binary orders,
@@ -373,29 +436,63 @@ GB_HD void fx_mass(FxBody& b, double mass, int em) {
                  normal ? down >> 2 : bits << 1 ? kFxClassFp64 : 0, 0, 0);
 }
 
-// One term of the accelerations into the three sums; returns its normalisation
-// (above fx_max_k: not added).  With masses the weight is 4^k 2^q.
-template <bool MASS>
+// Sizes of the terms added, in FP32: m at least the sum of their sizes (as
+// S |d| <= 2^151 / R), c[3] the sums of their components' sizes; units of 2^29
+// of V's.
+struct FxSize {
+  float m, c[3];
+};
+
+// One term of the accelerations into the three sums and its sizes into z (the
+// components' with two words only).  Returns its normalisation (above fx_max_k:
+// not added).  With masses the weight is 4^k 2^q.
+template <bool MASS, bool WIDE>
 GB_HD int fx_term(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& zi, float eps2f,
-                  const FxRow* tab, FxAcc (&a)[3]) {
+                  const FxRow* tab, FxAcc (&a)[3], FxSize& z) {
   const Fx96 ux = fx_sub(j.x, xi), uy = fx_sub(j.y, yi), uz = fx_sub(j.z, zi);
   const int k = fx_norm(ux, uy, uz, eps2f, fx_max_k<MASS>());
   const FxRow row = tab[k];
   const FxDiff dx = fx_scale(ux, k), dy = fx_scale(uy, k), dz = fx_scale(uz, k);
-  uint64_t s = fx_rinv3(fx_r2(dx, dy, dz, fx_pair(row.e_lo, row.e_hi)));
+  float yf;
+  uint64_t s = fx_rinv3(fx_r2(dx, dy, dz, fx_pair(row.e_lo, row.e_hi)), yf);
   uint32_t p = row.p;
+  float pf = row.pf;
   if (MASS) {
     s = fx_mul_hi(s << 2, fx_pair(j.mu_lo, j.mu_hi));  // S mass 2^(-eb - q - 1)
     p = k <= kFxMaxKMass ? p << fx_tag_q(j.tag) : 0u;
+    pf = k <= kFxMaxKMass ? fx_float_of(fx_float_bits(pf) + ((uint32_t)fx_tag_q(j.tag) << 23)) : 0.0f;
   }
-  const int32_t sh = (int32_t)(s >> 31), sl = (int32_t)((uint32_t)s & 0x7fffffffu);
-  fx_add(a[0], sh, sl, dx, p);
-  fx_add(a[1], sh, sl, dy, p);
-  fx_add(a[2], sh, sl, dz, p);
+  const float t = pf * (yf * yf);
+  z.m += t;
+  if (!WIDE) {
+    // |h| = |high word| 2^k, and S = Y^3 2^-32; half of it for what MASS takes off S
+    const float w = t * yf * fx_float_of((uint32_t)(127 - 61 - (MASS ? 1 : 0) + k) << 23);
+    z.c[0] += w * fx_abs((float)(int32_t)ux.w2);
+    z.c[1] += w * fx_abs((float)(int32_t)uy.w2);
+    z.c[2] += w * fx_abs((float)(int32_t)uz.w2);
+  }
+  fx_add<WIDE>(a[0], s, dx, p);
+  fx_add<WIDE>(a[1], s, dy, p);
+  fx_add<WIDE>(a[2], s, dz, p);
   return k;
 }
 
-// One term of the potential, [mass] / sqrt(|d|^2 + eps^2), into a.h and a.l;
+// What a body's term with itself adds to z.m (its components are zero).
+template <bool MASS>
+GB_HD float fx_self_size(float eps2f, const FxRow* tab, int q) {
+  const int k = fx_norm(Fx96{}, Fx96{}, Fx96{}, eps2f, fx_max_k<MASS>());
+  if (k > fx_max_k<MASS>()) return 0.0f;
+  const float yf = fx_rsqrt_seed_float(fx_pair(tab[k].e_lo, tab[k].e_hi));
+  return tab[k].pf * (float)(1 << q) * (yf * yf);
+}
+template <bool MASS>
+GB_HD int fx_term(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& zi, float eps2f,
+                  const FxRow* tab, FxAcc (&a)[3]) {
+  FxSize z = {};
+  return fx_term<MASS, false>(j, xi, yi, zi, eps2f, tab, a, z);
+}
+
+// One term of the potential, [mass] / sqrt(|d|^2 + eps^2), into a.m and a.l;
 // with weight 0 where `on` is false.
 template <bool MASS>
 GB_HD int fx_term_pot(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& zi, float eps2f,
@@ -411,15 +508,24 @@ GB_HD int fx_term_pot(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx9
     t += fx_tag_q(j.tag);
   }
   const uint32_t p = on && k <= kFxMaxK ? 1u << t : 0u;
-  a.h = (long long)fx_mad(fx_hi(y), p, (uint64_t)a.h);
+  a.m = fx_mad(fx_hi(y), p, a.m);
   a.l = fx_mad(fx_lo(y), p, a.l);
   return k;
 }
 
+// Two words serve a component whose terms' sizes come to more than 2^-kFxNarrow of
+// all the terms' together: V's error, 2^-57 of a term at most and 2^-59 in the
+// mean, is then that of a term in FP64 or less (5 and 1.3 2^-53).  Three words
+// serve one whose sum is above 2^-kFxThin of the terms' sizes: V's 2 units and
+// the coordinates' last bits, 2^-80 of a term at most, are then within 2^-54 of
+// it.  A sum below that (of a body in a plane, nearly) is taken in FP64.
+constexpr int kFxNarrow = 6;
+constexpr int kFxThin = 26;
+
 // exponent of a term's unit: sum 2^(fx_out_exp(ex)) is the sum of d / r^3, and
 // sum 2^(fx_out_exp(ex) + eb + 1) that of mass d / r^3; of the potential:
 // 1 / r, and with eb + 3 mass / r
-GB_HD int fx_out_exp(int ex) { return -60 - 2 * ex; }
+GB_HD int fx_out_exp(int ex) { return -91 - 2 * ex; }
 GB_HD int fx_out_exp_pot(int ex) { return -63 - ex; }
 
 // eps^2 in units of (2^64 U)^2

@@ -162,7 +162,7 @@ struct WarpGroup {
 template <int T>
 constexpr int f64_smem_bytes() {
   // partner records (at least the 32 T bytes of the FP64 loop), table, reduction
-  return ((int)sizeof(FxBody) * T + (int)sizeof(FxRow) * kFxRows + 32 * (T / 32) + 15) / 16 * 16;
+  return ((int)sizeof(FxBody) * T + (int)sizeof(FxRow) * kFxRows + 36 * (T / 32) + 15) / 16 * 16;
 }
 
 // Pair terms of the FP64 loops.
@@ -227,6 +227,14 @@ __device__ __forceinline__ void group_bar(int bar, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(threads) : "memory");
 }
 
+// t += the total of the lane `off` above (a whole warp's call)
+__device__ __forceinline__ void fx_tot_add_lane(FxTot& t, int off) {
+  const unsigned long long lo = __shfl_down_sync(0xffffffffu, (unsigned long long)t.l, off);
+  const unsigned long long mi = __shfl_down_sync(0xffffffffu, (unsigned long long)(t.l >> 64), off);
+  const int hi = __shfl_down_sync(0xffffffffu, t.h, off);
+  fx_tot_add(t, (unsigned __int128)mi << 64 | lo, hi);
+}
+
 // Masses of a group's partners: all equal, per body within one class (fixpair.cuh),
 // per body of several classes.
 enum { kFxEqual = 0, kFxOneClass = 1, kFxClasses = 2 };
@@ -274,11 +282,14 @@ __device__ __forceinline__ void fx_stage(FxBody* rec, const double* __restrict__
 // The tiles of one CTA or group.  Not inlined, and the geometry (T threads, L
 // lanes) a run-time value: the loop is long enough for the call, and a copy of
 // it in each of the FP64 kernels would make them slow to build.
+//
+// Returns whether the body of the thread's lanes (on its first lane) has a
+// component that the sums, of two words (fx_add), have too little of.
 template <int MASSES>
-__device__ __noinline__ void force_fx_tiles(const double* __restrict__ pos, long long n,
+__device__ __noinline__ bool force_fx_tiles(const double* __restrict__ pos, long long n,
                                             long long i0, long long jb, long long je, double eps2,
                                             const double* __restrict__ masses, int ex, int em,
-                                            bool ieee, int T, int L, int tid, int bar,
+                                            int flat, bool ieee, int T, int L, int tid, int bar,
                                             FxBody* rec, const FxRow* tab, double (*part)[3]) {
   constexpr bool MASS = MASSES != kFxEqual, CLASSES = MASSES == kFxClasses;
   const int b = tid / L;
@@ -292,13 +303,20 @@ __device__ __noinline__ void force_fx_tiles(const double* __restrict__ pos, long
     zi = fx_from_double(pos[3 * i + 2], ex);
   }
   const float eps2f = fx_eps2f(eps2, ex);
-  __int128 tot[3] = {};
+  FxTot tot[3] = {};
+  FxSize size = {};  // of the terms, in the heaviest class's units
   double near[3] = {};
   bool in_f64 = false, any_near = false;  // uniform in the warp
   int terms = 0, slow = 0;                // a lane's terms, and those of them in FP64
   for (long long j0 = jb; j0 < je; j0 += T) {
     const int cnt = (int)min((long long)T, je - j0);
     fx_stage<MASSES>(rec, pos, masses, j0 + tid, cnt, ex, em, T, tid, bar);
+    int own = i >= j0 && i - j0 < cnt ? (int)(i - j0) : -1;  // the body's own record
+    if (CLASSES && own >= 0) {
+      int p = 0;
+      while (fx_tag_index(rec[p].tag) != own) ++p;
+      own = p;
+    }
     for (int base = 0, end; base < cnt; base = end) {
       end = min(cnt, base + kFxChunk * L);
       int run = cnt, cls = 0;
@@ -313,21 +331,31 @@ __device__ __noinline__ void force_fx_tiles(const double* __restrict__ pos, long
       unsigned mask = (in_f64 || light) && steps ? 0xffffffffu >> (32 - steps) : 0u;
       if (!in_f64 && !light) {
         FxAcc a[3] = {};
+        FxSize z = {};
         // unrolled twice: 1.59 ms at N = 16384 against 1.72 ms (1) and 1.73 ms (4)
 #pragma unroll 2
         for (int jj = c0; jj < end; jj += L) {
-          const int k = fx_term<MASS>(rec[jj], xi, yi, zi, eps2f, tab, a);
+          const int k = fx_term<MASS, false>(rec[jj], xi, yi, zi, eps2f, tab, a, z);
           mask = __funnelshift_l((unsigned)(fx_max_k<MASS>() - k), mask, 1);  // 1 when k is above
         }
+        if (own >= base && own < end && (own - base) % L == l) {
+          // without the body itself, whose part may be far above the others': as
+          // much as the rounding of their sum with it
+          const float self = fx_self_size<MASS>(eps2f, tab, MASS ? fx_tag_q(rec[own].tag) : 0);
+          z.m = fmaxf(z.m - self, 0.0f) + self * 0x1p-18f;
+        }
+        const float w = CLASSES ? scalbnf(1.0f, -4 * cls) : 1.0f;
+        size.m += w * z.m;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) size.c[d] += w * z.c[d];
 #pragma unroll
         for (int d = 0; d < 3; ++d) fx_fold(tot[d], a[d]);
       }
       int rounds = 0;
       if (__any_sync(0xffffffffu, mask != 0)) {
         if (!valid) mask = 0;
-        const long long self = i - j0 - c0;  // not the body itself
-        if (!CLASSES && self >= 0 && self < (long long)steps * L && self % L == 0)
-          mask &= ~(1u << (steps - 1 - (int)self / L));
+        if (own >= base && own < end && (own - base) % L == l)  // not the body itself
+          mask &= ~(1u << (steps - 1 - (own - c0) / L));
         rounds = fx_chunk_f64(mask, steps, j0, c0, L, CLASSES ? rec : nullptr, pos, i, eps2,
                               masses, ieee, near);
         any_near = any_near || rounds > 0;
@@ -346,7 +374,7 @@ __device__ __noinline__ void force_fx_tiles(const double* __restrict__ pos, long
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
           near[d] = dadd(near[d], fx_to_double(tot[d], fx_out_exp(ex) + fx_class_exp(em, cls) + 1));
-          tot[d] = 0;
+          tot[d] = FxTot{};
         }
         any_near = true;
       }
@@ -356,20 +384,122 @@ __device__ __noinline__ void force_fx_tiles(const double* __restrict__ pos, long
   for (int off = L / 2; off >= 1; off /= 2) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      const unsigned long long lo =
-          __shfl_down_sync(0xffffffffu, (unsigned long long)tot[d], off);
-      const unsigned long long hi =
-          __shfl_down_sync(0xffffffffu, (unsigned long long)(tot[d] >> 64), off);
-      tot[d] += (__int128)(((unsigned __int128)hi << 64) | lo);
+      fx_tot_add_lane(tot[d], off);
       if (any_near) near[d] = dadd(near[d], __shfl_down_sync(0xffffffffu, near[d], off));
     }
+    size.m += __shfl_down_sync(0xffffffffu, size.m, off);
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      size.c[d] += __shfl_down_sync(0xffffffffu, size.c[d], off);
+  }
+  double v[3];
+  bool thin = false;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    v[d] = fx_to_double(tot[d], sc);
+    if (any_near) v[d] = dadd(v[d], near[d]);
+    thin = thin || (!(flat >> d & 1) && size.c[d] * (1 << kFxNarrow) < size.m);
+  }
+  if (any_near && thin) {  // the terms in FP64 count as well
+    const double least =
+        dmul((double)size.m, __hiloint2double((1023 + sc + 29 - kFxNarrow) << 20, 0));
+    thin = false;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      thin = thin || (!(flat >> d & 1) && size.c[d] * (1 << kFxNarrow) < size.m &&
+                      !(fabs(near[d]) >= least));
   }
   if (l == 0) {
 #pragma unroll
+    for (int d = 0; d < 3; ++d) part[b][d] = v[d];
+  }
+  return thin && l == 0 && valid;
+}
+
+// The sums of the bodies i of the lanes in `lanes` (bits) over the partners from
+// jb to je, each with three words (fx_add; 42 IMAD.WIDE a term against 33) or, where
+// they have too little of a component, in FP64: one body after the other, the
+// partners over the warp's lanes, so that they depend on nothing else that the
+// warp runs.  The whole warp calls it.
+static __device__ __noinline__ void fx_bodies_wide(unsigned lanes, const double* __restrict__ pos,
+                                                   long long i, long long jb, long long je,
+                                                   double eps2, const double* __restrict__ masses,
+                                                   bool classes, int ex, int em, int flat,
+                                                   bool ieee, const FxRow* tab, double* sum) {
+  const int lane = threadIdx.x & 31;
+  const float eps2f = fx_eps2f(eps2, ex);
+#pragma unroll 1
+  for (; lanes; lanes &= lanes - 1) {
+    const int src = __ffs(lanes) - 1;
+    const long long ib = __shfl_sync(0xffffffffu, i, src);
+    const Fx96 xi = fx_from_double(pos[3 * ib], ex), yi = fx_from_double(pos[3 * ib + 1], ex),
+               zi = fx_from_double(pos[3 * ib + 2], ex);
+    FxTot tot[3] = {};
+    FxSize size = {};
+    double v[3] = {};
+    int terms = 0;
+    FxAcc a[3] = {};
+#pragma unroll 1
+    for (long long j = jb + lane; j < je; j += 32) {
+      if (j == ib) continue;
+      FxBody r;
+      r.x = fx_from_double(pos[3 * j], ex);
+      r.y = fx_from_double(pos[3 * j + 1], ex);
+      r.z = fx_from_double(pos[3 * j + 2], ex);
+      r.mu_lo = r.mu_hi = r.tag = 0;
+      if (masses) fx_mass(r, masses[j], em);
+      const int cls = fx_tag_class(r.tag);
+      FxSize z = {};
+      const bool near =
+          cls == kFxClassFp64 ||
+          (masses ? fx_term<true, true>(r, xi, yi, zi, eps2f, tab, a, z) > fx_max_k<true>()
+                  : fx_term<false, true>(r, xi, yi, zi, eps2f, tab, a, z) > fx_max_k<false>());
+      if (near) {
+        add_pair_f64(pos, ib, j, eps2, masses, ieee, v);
+        continue;
+      }
+      size.m += classes ? scalbnf(z.m, -4 * cls) : z.m;
+      if (classes) {
+        const int sc = fx_out_exp(ex) + fx_class_exp(em, cls) + 1;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          FxTot t = {};
+          fx_fold(t, a[d]);
+          v[d] = dadd(v[d], fx_to_double(t, sc));
+        }
+      } else if (++terms == kFxChunk) {
+        terms = 0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) fx_fold(tot[d], a[d]);
+      }
+    }
+    const int sc = fx_out_exp(ex) + (masses ? fx_class_exp(em, 0) + 1 : 0);
+#pragma unroll
     for (int d = 0; d < 3; ++d) {
-      double v = fx_to_double(tot[d], sc);
-      if (any_near) v = dadd(v, near[d]);
-      part[b][d] = v;
+      fx_fold(tot[d], a[d]);
+#pragma unroll
+      for (int off = 16; off >= 1; off /= 2) fx_tot_add_lane(tot[d], off);
+      v[d] = dadd(fx_to_double(tot[d], sc), lane_reduce<32>(v[d]));
+    }
+#pragma unroll
+    for (int off = 16; off >= 1; off /= 2) size.m += __shfl_down_sync(0xffffffffu, size.m, off);
+    const double least =
+        dmul((double)size.m, __hiloint2double((1023 + sc + 29 - kFxThin) << 20, 0));
+    bool thin = false;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) thin = thin || (!(flat >> d & 1) && fabs(v[d]) < least);
+    if (__shfl_sync(0xffffffffu, (int)thin, 0)) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) v[d] = 0.0;
+      for (long long j = jb + lane; j < je; j += 32)
+        if (j != ib) add_pair_f64(pos, ib, j, eps2, masses, ieee, v);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) v[d] = lane_reduce<32>(v[d]);
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double t = __shfl_sync(0xffffffffu, v[d], 0);
+      if (lane == src) sum[d] = t;
     }
   }
 }
@@ -384,32 +514,52 @@ __device__ __forceinline__ double key_bound(int key, bool upper) {
   return __hiloint2double(h, (h < 0) != upper ? -1 : 0);  // outwards over the low word
 }
 
+// What the extents say of the accelerations' components: along the axes of
+// `flat` (bits) the bodies have one coordinate; wide: another axis is so short
+// that three words are called for from the start (kFxNarrow), thin: so short that
+// most bodies' sums would be in FP64 as well (kFxThin).
+struct FxShape {
+  int flat;
+  bool wide, thin;
+};
+
 // The grid of a group's own body i and of the `count` partners from jb on
-// (modulo n): exponents ex and, with masses, em, and whether the masses are of
-// more than one class; red holds 8 words a warp.  Returns false, uniformly in the group, when there is no grid: a coordinate
-// that is not finite, bodies all within a sixteenth of the softening,
-// exponents beyond 2^+-300, or a mass that is negative, not finite or all of
-// them zero.
+// (modulo n): exponents ex and, with masses, em, whether the masses are of more
+// than one class, and the shape; red holds 9 words a warp.  Returns false,
+// uniformly in the group, when there is no grid: a coordinate that is not
+// finite, bodies all within a sixteenth of the softening, exponents beyond
+// 2^+-300, or a mass that is negative, not finite or all of them zero.
 static __device__ __noinline__ bool fx_grid(const double* __restrict__ pos, long long n,
                                             long long i, long long jb, long long count,
                                             double eps2, const double* __restrict__ masses,
                                             int* red, int T, int tid, int bar, int* ex_out,
-                                            int* em_out, bool* classes_out) {
+                                            int* em_out, bool* classes_out, FxShape* shape_out) {
+  if (count == 0) return false;
   const int nw = T / 32;
   int lo[3], hi[3];
+  int ref[3], other = 0;  // axes with a low word that is not the first partner's
   unsigned mm = 0, ml = 0xffffffffu;
+  int off[3] = {};
 #pragma unroll
-  for (int c = 0; c < 3; ++c) lo[c] = hi[c] = order_key(pos[3 * i + c]);
+  for (int c = 0; c < 3; ++c) {
+    lo[c] = hi[c] = order_key(pos[3 * i + c]);
+    ref[c] = __double2loint(pos[3 * jb + c]);
+    off[c] = __double2loint(pos[3 * i + c]) ^ ref[c];
+  }
 #pragma unroll 4
   for (long long v = tid; v < count; v += T) {
     const long long j = jb + v < n ? jb + v : jb + v - n;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const int k = order_key(pos[3 * j + c]);
+      const double x = pos[3 * j + c];
+      const int k = order_key(x);
       lo[c] = min(lo[c], k);
       hi[c] = max(hi[c], k);
+      off[c] |= __double2loint(x) ^ ref[c];
     }
   }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) other |= off[c] ? 1 << c : 0;
   if (masses) {
     // a negative mass reads as a large unsigned word
 #pragma unroll 4
@@ -422,13 +572,14 @@ static __device__ __noinline__ bool fx_grid(const double* __restrict__ pos, long
   }
   mm = __reduce_max_sync(0xffffffffu, mm);
   ml = __reduce_min_sync(0xffffffffu, ml);
+  other = __reduce_or_sync(0xffffffffu, other);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     lo[c] = __reduce_min_sync(0xffffffffu, lo[c]);
     hi[c] = __reduce_max_sync(0xffffffffu, hi[c]);
   }
   if ((tid & 31) == 0) {
-    int* r = red + 8 * (tid / 32);
+    int* r = red + 9 * (tid / 32);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       r[c] = lo[c];
@@ -436,10 +587,11 @@ static __device__ __noinline__ bool fx_grid(const double* __restrict__ pos, long
     }
     r[6] = (int)mm;
     r[7] = (int)ml;
+    r[8] = other;
   }
   group_bar(bar, T);
   for (int w = 0; w < nw; ++w) {
-    const int* r = red + 8 * w;
+    const int* r = red + 9 * w;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       lo[c] = min(lo[c], r[c]);
@@ -447,26 +599,36 @@ static __device__ __noinline__ bool fx_grid(const double* __restrict__ pos, long
     }
     mm = max(mm, (unsigned)r[6]);
     ml = min(ml, (unsigned)r[7]);
+    other |= r[8];
   }
   constexpr int kInf = 0x7ff00000;
-  int xe = 0;
+  int xe[3], flat = 0;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     if (hi[c] >= kInf || lo[c] <= ~kInf) return false;
     const double ext = key_bound(hi[c], true) - key_bound(lo[c], false);
-    xe = max(xe, __double2hiint(ext) >> 20);
+    xe[c] = __double2hiint(ext) >> 20;
+    if (hi[c] == lo[c] && !(other >> c & 1)) flat |= 1 << c;
   }
-  int ex = xe - 1022;  // the extents are below 2^ex
+  int ex = max(xe[0], max(xe[1], xe[2])) - 1022;  // the extents are below 2^ex
   const int e2 = (__double2hiint(eps2) >> 20) & 0x7ff;
   if (e2) {
     const int ee = ((e2 - 1023) >> 1) + 1;  // eps < 2^ee
     if (ex < ee - 4) return false;
     ex = max(ex, ee + 1);
   }
+  bool wide = false, thin = false;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    if (flat >> c & 1) continue;
+    wide = wide || xe[c] - 1022 < ex - kFxNarrow;
+    thin = thin || xe[c] - 1022 < ex - kFxThin + 2;
+  }
   const int em = (int)(mm >> 20) - 1023;  // 2^em <= the largest mass < 2^(em + 1)
   if (ex < -300 || ex > 300 || (masses && (em < -300 || em > 300))) return false;
   *ex_out = ex;
   *em_out = em;
+  *shape_out = FxShape{flat, wide, thin};
   *classes_out = masses && (int)(ml >> 20) < (int)(mm >> 20) - 3;
   return true;
 }
@@ -482,21 +644,39 @@ static __device__ __noinline__ bool force_fx_group(const double* __restrict__ po
   FxBody* rec = reinterpret_cast<FxBody*>(smem);
   FxRow* tab = reinterpret_cast<FxRow*>(rec + T);
   int* red = reinterpret_cast<int*>(tab + kFxRows);
+  // no more than a term for each lane: FP64 takes less than the grid
+  if (je - jb <= L) return false;
   int ex, em;
   bool classes;
+  FxShape shape;
   if (!fx_grid(pos, n, min(i0 + tid / L, n - 1), jb, je - jb, eps2, masses, red, T, tid, bar, &ex,
-               &em, &classes))
+               &em, &classes, &shape) ||
+      shape.thin)
     return false;
+  const int flat = shape.flat;
   if (tid < kFxRows) tab[tid] = fx_row(tid, eps2, ex);
-  if (!masses)
-    force_fx_tiles<kFxEqual>(pos, n, i0, jb, je, eps2, nullptr, ex, 0, ieee, T, L, tid, bar, rec,
-                             tab, part);
+  const long long i = i0 + tid / L;
+  bool thin = tid % L == 0 && i < n;
+  if (shape.wide)
+    group_bar(bar, T);  // the table is there
+  else if (!masses)
+    thin = force_fx_tiles<kFxEqual>(pos, n, i0, jb, je, eps2, nullptr, ex, 0, flat, ieee, T, L, tid,
+                                    bar, rec, tab, part);
   else if (!classes)
-    force_fx_tiles<kFxOneClass>(pos, n, i0, jb, je, eps2, masses, ex, em, ieee, T, L, tid, bar,
-                                rec, tab, part);
+    thin = force_fx_tiles<kFxOneClass>(pos, n, i0, jb, je, eps2, masses, ex, em, flat, ieee, T, L,
+                                       tid, bar, rec, tab, part);
   else
-    force_fx_tiles<kFxClasses>(pos, n, i0, jb, je, eps2, masses, ex, em, ieee, T, L, tid, bar,
-                               rec, tab, part);
+    thin = force_fx_tiles<kFxClasses>(pos, n, i0, jb, je, eps2, masses, ex, em, flat, ieee, T, L,
+                                      tid, bar, rec, tab, part);
+  const unsigned lanes = __ballot_sync(0xffffffffu, thin);
+  if (lanes) {
+    double v[3];
+    fx_bodies_wide(lanes, pos, i, jb, je, eps2, masses, classes, ex, em, flat, ieee, tab, v);
+    if (thin) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) part[tid / L][d] = v[d];
+    }
+  }
   return true;
 }
 

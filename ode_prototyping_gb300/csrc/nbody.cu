@@ -31,8 +31,10 @@ enum { kModeRhs = 0, kModeAccWrite = 1, kModeAccAdd = 2 };
 // unevenly spread over the SMs (3001: 2088 us for the 16 steps where they may).
 constexpr unsigned kFewCtas = 76;
 constexpr int kAfterCtasPerSm = 4;
+// Registers for 4 CTAs of 128 threads on an SM (N = 16384 1.66 ms, 1.88 at 5; 162
+// registers and 3 CTAs where the compiler is left to itself, 13 % slower).
 template <int T, int L, bool AFTER = false>
-__global__ void __launch_bounds__(T) rhs_f64_kernel(const double* __restrict__ pos,
+__global__ void __launch_bounds__(T, 4 * 128 / T) rhs_f64_kernel(const double* __restrict__ pos,
                                                     const double* __restrict__ vel,
                                                     double* __restrict__ out_vel,
                                                     double* __restrict__ out_acc, long long n,

@@ -312,7 +312,8 @@ typedef struct {
                                  tableau allows it (bit-identical results) */
   int32_t exact;              /* serial-order forces and norm (reference bit pattern) */
   int32_t attempts_per_sync;  /* attempts per graph replay (0 = 16); the host waits for one
-                                 replay at a time, in FP64 without recording for up to 8 */
+                                 replay at a time, in FP64 without recording for up to 8
+                                 where they take no longer than one in FP64 terms */
   int32_t record;             /* deliver every accepted state to the save callback */
   int64_t max_attempts;       /* 0 = unlimited (the reference has no bound) */
   double host_wait_timeout_s; /* bound on one host wait (0 = 600 s) */

@@ -1554,22 +1554,31 @@ extern "C" int gb_integrator_advance(gb_integrator it, int64_t max_attempts, gb_
   if (!it || !it->started) return GB_ERR_INVALID_ARGUMENT;
   const long long start_attempts = it->hctrl->n_attempts;
   // One replay per host wait, or, where FP64 stages run on fixed-point pair
-  // terms (a replay takes a seventh of the time it took in FP64, so a wait
-  // stays as long as it was) and nobody takes states, as many as the steps
-  // left at the present step size fill, at most 8: replays past the end would
-  // be launches that only find the run done.
+  // terms and nobody takes states, as many as the steps left at the present step
+  // size fill (replays past the end would be launches that only find the run
+  // done), at most 8 and no more than take, by the longest replay so far, the
+  // time of one replay of FP64 terms (12 ms a right-hand side at N = 16384): a
+  // system that the fixed point does not suit takes that time for a replay, and
+  // is waited for one at a time.
+  constexpr double kPairF64 = 4.4e-11;  // seconds
   const bool several = it->params.f64_pair == kPairFixedFast &&
                        it->opts.precision == GB_PREC_F64 && !save && !it->opts.record &&
                        max_attempts <= 0;
+  const double in_f64 = kPairF64 * (double)it->n * (double)it->n * it->S * it->A;
+  double longest = 0.0;  // seconds of a replay in this call
   while (!it->hctrl->done) {
     if (max_attempts > 0 && it->hctrl->n_attempts - start_attempts >= max_attempts) break;
     int replays = 1;
-    if (several && it->hctrl->n_attempts > 0) {
-      const double left = (it->hctrl->tf - it->hctrl->t) / (it->hctrl->dt * it->A);
-      replays = left >= 8.0 ? 8 : std::max(1, (int)left);
+    if (several && longest > 0.0) {
+      const double left = std::min((it->hctrl->tf - it->hctrl->t) / (it->hctrl->dt * it->A),
+                                   in_f64 / longest);
+      replays = left >= 8.0 ? 8 : left >= 1.0 ? (int)left : 1;
     }
+    const auto t0 = std::chrono::steady_clock::now();
     for (int r = 0; r < replays; ++r) GB_CUDA_TRY(cudaGraphLaunch(it->exec, it->stream));
     GB_TRY(read_ctrl(it));
+    longest = std::max(longest, std::chrono::duration<double>(
+                                    std::chrono::steady_clock::now() - t0).count() / replays);
     GB_TRY(drain(it, save, user));
   }
   GB_TRY(drain(it, save, user));

@@ -108,12 +108,12 @@ __device__ __noinline__ double pot_fx(const double* __restrict__ pos, long long 
         near += (MASS ? masses[j] : 1.0) / sqrt(dx * dx + dy * dy + dz * dz + eps2);
       }
       if (CLASSES && end == run) {  // the class's sum in the tile
-        near += fx_to_double(tot, fx_out_exp_pot(ex) + fx_class_exp(em, cls) + 3);
+        near += fx_to_double(tot, fx_out_exp_pot(ex) + fx_class_exp(em, cls) + 2);
         tot = 0;
       }
     }
   }
-  return fx_to_double(tot, fx_out_exp_pot(ex) + (MASS ? fx_class_exp(em, 0) + 3 : 0)) + near;
+  return fx_to_double(tot, fx_out_exp_pot(ex) + (MASS ? fx_class_exp(em, 0) + 2 : 0)) + near;
 }
 
 __global__ void __launch_bounds__(kT, kCtasPerSm)

@@ -305,10 +305,10 @@ GB_HD uint64_t fx_rinv1(uint64_t r) {
   return fx_refine(y, fx_residual(r, fx_mul(y, y)), 32u, 6u);
 }
 
-// Adds weight p times the component V = S (h 2^32 + l + ll 2^-32) / 2^32, of which
-// a term has 2^89 to 2^91.  With S split like the component, the words' carries go
-// through the multiply-adds' addends.  Two words, within 0.8 2^32 (2^-57 of the
-// term), or, WIDE, three, within 2: the parts that two drop are all that a
+// Adds weight p times the component V = 2 S (h 2^32 + l + ll 2^-32) / 2^32, of
+// which a term has 2^90 to 2^92; s = 2 S.  With S split like the component, the words' carries go
+// through the multiply-adds' addends.  Two words, within 0.8 2^32 (2^-58 of the
+// term, 2^-60 in the mean), or, WIDE, three, within 2: the parts that two drop are all that a
 // component far smaller than the distance has.
 template <bool WIDE>
 GB_HD void fx_add(FxAcc& a, uint64_t s, const FxDiff& d, uint32_t p) {
@@ -332,7 +332,7 @@ GB_HD void fx_fold(__int128& tot, FxAcc& a) {
   a.m = 0;
 }
 
-// A term is below 2^118 in size, a fold of 32 below 2^123: 2^36 folds.
+// A term is below 2^118 in size, a fold of 32 below 2^123: 2^36 folds in 160 bits.
 GB_HD void fx_tot_add(FxTot& t, unsigned __int128 l, int32_t h) {
   t.l += l;
   t.h += h + (t.l < l ? 1 : 0);
@@ -398,7 +398,7 @@ GB_HD FxRow fx_row(int k, double eps2, int ex) {
 
 // A partner's record.  Per-body masses come in classes of four binary orders,
 // class c the exponents em - 4 c - 3 ... em - 4 c with em the largest mass's:
-// mass = mu 2^(eb + q - 61), mu in [2^61, 2^62), eb the class's lowest exponent
+// mass = mu 2^(eb + q - 62), mu in [2^62, 2^63), eb the class's lowest exponent
 // and 0 <= q <= 3, mu = 0 for a mass of 0.  Every class has sums of its own
 // (fx_class_exp), so a term keeps its bits however light its partner is: the
 // heaviest body feels only the others.
@@ -428,7 +428,7 @@ GB_HD void fx_mass(FxBody& b, double mass, int em) {
 #endif
   const int e = (int)((bits >> 52) & 0x7ff) - 1023;
   const bool normal = e >= -300;
-  const uint64_t mu = normal ? ((bits & 0xfffffffffffffull) | (1ull << 52)) << 9 : 0;
+  const uint64_t mu = normal ? ((bits & 0xfffffffffffffull) | (1ull << 52)) << 10 : 0;
   b.mu_lo = fx_lo(mu);
   b.mu_hi = fx_hi(mu);
   const int down = normal ? em - e : 0;
@@ -437,7 +437,7 @@ GB_HD void fx_mass(FxBody& b, double mass, int em) {
 }
 
 // Sizes of the terms added, in FP32: m at least the sum of their sizes (as
-// S |d| <= 2^151 / R), c[3] the sums of their components' sizes; units of 2^29
+// S |d| <= 2^151 / R), c[3] the sums of their components' sizes; units of 2^30
 // of V's.
 struct FxSize {
   float m, c[3];
@@ -454,19 +454,21 @@ GB_HD int fx_term(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& z
   const FxRow row = tab[k];
   const FxDiff dx = fx_scale(ux, k), dy = fx_scale(uy, k), dz = fx_scale(uz, k);
   float yf;
-  uint64_t s = fx_rinv3(fx_r2(dx, dy, dz, fx_pair(row.e_lo, row.e_hi)), yf);
+  uint64_t s = fx_rinv3(fx_r2(dx, dy, dz, fx_pair(row.e_lo, row.e_hi)), yf) << 1;
   uint32_t p = row.p;
   float pf = row.pf;
   if (MASS) {
-    s = fx_mul_hi(s << 2, fx_pair(j.mu_lo, j.mu_hi));  // S mass 2^(-eb - q - 1)
+    s = fx_mul_hi(s << 1, fx_pair(j.mu_lo, j.mu_hi));  // 2 S mass 2^(-eb - q - 1)
     p = k <= kFxMaxKMass ? p << fx_tag_q(j.tag) : 0u;
-    pf = k <= kFxMaxKMass ? fx_float_of(fx_float_bits(pf) + ((uint32_t)fx_tag_q(j.tag) << 23)) : 0.0f;
+    // times half the mantissa, of mu's 31 bits in the high word, and 2^q
+    const uint32_t half = (j.mu_hi >> 7 & 0x7fffffu) | (uint32_t)(126 + fx_tag_q(j.tag)) << 23;
+    pf = k <= kFxMaxKMass && j.mu_hi ? pf * fx_float_of(half) : 0.0f;
   }
   const float t = pf * (yf * yf);
   z.m += t;
   if (!WIDE) {
-    // |h| = |high word| 2^k, and S = Y^3 2^-32; half of it for what MASS takes off S
-    const float w = t * yf * fx_float_of((uint32_t)(127 - 61 - (MASS ? 1 : 0) + k) << 23);
+    // |h| = |high word| 2^k, and S = Y^3 2^-32
+    const float w = t * yf * fx_float_of((uint32_t)(127 - 61 + k) << 23);
     z.c[0] += w * fx_abs((float)(int32_t)ux.w2);
     z.c[1] += w * fx_abs((float)(int32_t)uy.w2);
     z.c[2] += w * fx_abs((float)(int32_t)uz.w2);
@@ -479,11 +481,16 @@ GB_HD int fx_term(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& z
 
 // What a body's term with itself adds to z.m (its components are zero).
 template <bool MASS>
-GB_HD float fx_self_size(float eps2f, const FxRow* tab, int q) {
+GB_HD float fx_self_size(float eps2f, const FxRow* tab, const FxBody& j) {
   const int k = fx_norm(Fx96{}, Fx96{}, Fx96{}, eps2f, fx_max_k<MASS>());
   if (k > fx_max_k<MASS>()) return 0.0f;
   const float yf = fx_rsqrt_seed_float(fx_pair(tab[k].e_lo, tab[k].e_hi));
-  return tab[k].pf * (float)(1 << q) * (yf * yf);
+  float pf = tab[k].pf;
+  if (MASS)
+    pf = j.mu_hi ? pf * fx_float_of((j.mu_hi >> 7 & 0x7fffffu) |
+                                    (uint32_t)(126 + fx_tag_q(j.tag)) << 23)
+                 : 0.0f;
+  return pf * (yf * yf);
 }
 template <bool MASS>
 GB_HD int fx_term(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& zi, float eps2f,
@@ -504,7 +511,7 @@ GB_HD int fx_term_pot(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx9
   uint64_t y = fx_rinv1(fx_r2(dx, dy, dz, fx_pair(row.e_lo, row.e_hi)));
   int t = k;
   if (MASS) {
-    y = fx_mul_hi(y, fx_pair(j.mu_lo, j.mu_hi));  // y mass 2^(-eb - q - 3)
+    y = fx_mul_hi(y, fx_pair(j.mu_lo, j.mu_hi));  // y mass 2^(-eb - q - 2)
     t += fx_tag_q(j.tag);
   }
   const uint32_t p = on && k <= kFxMaxK ? 1u << t : 0u;
@@ -514,18 +521,18 @@ GB_HD int fx_term_pot(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx9
 }
 
 // Two words serve a component whose terms' sizes come to more than 2^-kFxNarrow of
-// all the terms' together: V's error, 2^-57 of a term at most and 2^-59 in the
-// mean, is then that of a term in FP64 or less (5 and 1.3 2^-53).  Three words
+// all the terms' together: V's error, 2^-58 of a term at most and 2^-60 in the
+// mean, is then that of a term in FP64 (5 and 1.3 2^-53).  Three words
 // serve one whose sum is above 2^-kFxThin of the terms' sizes: V's 2 units and
 // the coordinates' last bits, 2^-80 of a term at most, are then within 2^-54 of
 // it.  A sum below that (of a body in a plane, nearly) is taken in FP64.
-constexpr int kFxNarrow = 6;
+constexpr int kFxNarrow = 8;
 constexpr int kFxThin = 26;
 
 // exponent of a term's unit: sum 2^(fx_out_exp(ex)) is the sum of d / r^3, and
 // sum 2^(fx_out_exp(ex) + eb + 1) that of mass d / r^3; of the potential:
-// 1 / r, and with eb + 3 mass / r
-GB_HD int fx_out_exp(int ex) { return -91 - 2 * ex; }
+// 1 / r, and with eb + 2 mass / r
+GB_HD int fx_out_exp(int ex) { return -92 - 2 * ex; }
 GB_HD int fx_out_exp_pot(int ex) { return -63 - ex; }
 
 // eps^2 in units of (2^64 U)^2

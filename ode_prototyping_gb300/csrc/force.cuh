@@ -341,7 +341,7 @@ __device__ __noinline__ bool force_fx_tiles(const double* __restrict__ pos, long
         if (own >= base && own < end && (own - base) % L == l) {
           // without the body itself, whose part may be far above the others': as
           // much as the rounding of their sum with it
-          const float self = fx_self_size<MASS>(eps2f, tab, MASS ? fx_tag_q(rec[own].tag) : 0);
+          const float self = fx_self_size<MASS>(eps2f, tab, rec[own]);
           z.m = fmaxf(z.m - self, 0.0f) + self * 0x1p-18f;
         }
         const float w = CLASSES ? scalbnf(1.0f, -4 * cls) : 1.0f;
@@ -402,7 +402,7 @@ __device__ __noinline__ bool force_fx_tiles(const double* __restrict__ pos, long
   }
   if (any_near && thin) {  // the terms in FP64 count as well
     const double least =
-        dmul((double)size.m, __hiloint2double((1023 + sc + 29 - kFxNarrow) << 20, 0));
+        dmul((double)size.m, __hiloint2double((1023 + sc + 30 - kFxNarrow) << 20, 0));
     thin = false;
 #pragma unroll
     for (int d = 0; d < 3; ++d)
@@ -438,6 +438,7 @@ static __device__ __noinline__ void fx_bodies_wide(unsigned lanes, const double*
     FxSize size = {};
     double v[3] = {};
     int terms = 0;
+    bool in_f64 = classes;
     FxAcc a[3] = {};
 #pragma unroll 1
     for (long long j = jb + lane; j < je; j += 32) {
@@ -456,6 +457,7 @@ static __device__ __noinline__ void fx_bodies_wide(unsigned lanes, const double*
                   : fx_term<false, true>(r, xi, yi, zi, eps2f, tab, a, z) > fx_max_k<false>());
       if (near) {
         add_pair_f64(pos, ib, j, eps2, masses, ieee, v);
+        in_f64 = true;
         continue;
       }
       size.m += classes ? scalbnf(z.m, -4 * cls) : z.m;
@@ -474,20 +476,24 @@ static __device__ __noinline__ void fx_bodies_wide(unsigned lanes, const double*
       }
     }
     const int sc = fx_out_exp(ex) + (masses ? fx_class_exp(em, 0) + 1 : 0);
+    const bool any_f64 = __any_sync(0xffffffffu, in_f64);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       fx_fold(tot[d], a[d]);
 #pragma unroll
       for (int off = 16; off >= 1; off /= 2) fx_tot_add_lane(tot[d], off);
-      v[d] = dadd(fx_to_double(tot[d], sc), lane_reduce<32>(v[d]));
+      const double t = fx_to_double(tot[d], sc);
+      v[d] = any_f64 ? dadd(t, lane_reduce<32>(v[d])) : t;
     }
 #pragma unroll
     for (int off = 16; off >= 1; off /= 2) size.m += __shfl_down_sync(0xffffffffu, size.m, off);
-    const double least =
-        dmul((double)size.m, __hiloint2double((1023 + sc + 29 - kFxThin) << 20, 0));
+    // exponents: of a component, and of 2^-kFxThin of the sizes
+    const int least = (int)(fx_float_bits(size.m) >> 23) - 127 + sc + 30 - kFxThin;
     bool thin = false;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) thin = thin || (!(flat >> d & 1) && fabs(v[d]) < least);
+    for (int d = 0; d < 3; ++d)
+      thin = thin || (size.m > 0.0f && !(flat >> d & 1) &&
+                      (__double2hiint(v[d]) >> 20 & 0x7ff) - 1023 <= least);
     if (__shfl_sync(0xffffffffu, (int)thin, 0)) {
 #pragma unroll
       for (int d = 0; d < 3; ++d) v[d] = 0.0;

@@ -49,7 +49,7 @@ int main() {
               FxAcc an[3] = {};
               fx_term<false, false>(j, x, y, z, e2, tab, an, zn);
               if (zn.m != zw.m) return 5;
-              const Q size = ldexpl((Q)zw.m, fx_out_exp(0) + 29);
+              const Q size = ldexpl((Q)zw.m, fx_out_exp(0) + 30);
               const Q s = 1 / (r2 * sqrtl(r2));
               const Q dist = sqrtl(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
               if (s * dist > size * 1.0001L) return 1;
@@ -62,7 +62,7 @@ int main() {
                   continue;
                 }
                 if (zn.c[c] * (1 << kFxNarrow) >= zn.m) {
-                  if (fabsl(ldexpl((Q)zn.c[c], fx_out_exp(0) + 29) / (s * fabsl(d[c])) - 1) > 0.01) return 6;
+                  if (fabsl(ldexpl((Q)zn.c[c], fx_out_exp(0) + 30) / (s * fabsl(d[c])) - 1) > 0.01) return 6;
                   __int128 t2 = 0;
                   fx_fold(t2, an[c]);
                   const Q got = ldexpl((Q)t2, fx_out_exp(0));

@@ -17,7 +17,7 @@ int main() {
   for (int em : {0, 3, -299, 300})
     for (int down = 0; down <= 84; ++down)
       for (int lg = 0; lg >= -13; --lg)
-        for (int t = 0; t < 20; ++t) {
+        for (int t = 0; t < 200; ++t) {
           const double mass = std::ldexp(1.0 + 0.5 * (1.0 + U(g)), em - down);
           double xi[3], xj[3], u[3], nn = 0.0;
           for (double& v : u) nn += (v = U(g)) * v;
@@ -60,7 +60,7 @@ int main() {
           if (fx_term_pot<true>(j, x, y, z, e2, tab, true, p) <= kFxMaxK) {
             __int128 tot = 0;
             fx_fold(tot, p);
-            const Q got = ldexpl((Q)tot, fx_out_exp_pot(0) + fx_class_exp(em, cls) + 3);
+            const Q got = ldexpl((Q)tot, fx_out_exp_pot(0) + fx_class_exp(em, cls) + 2);
             const Q ref = mass / sqrtl(r2);
             worst_pot = std::fmax(worst_pot, (double)fabsl(got / ref - 1) * 0x1p53);
           }

@@ -168,16 +168,19 @@ constexpr int f64_smem_bytes() {
 // Pair terms of the FP64 loops.
 enum { kPairIeee = 0, kPairFast = 1, kPairFixedFast = 2, kPairFixedIeee = 3 };
 
-// One partner's term in FP64, added to s.
+// One partner's term in FP64, added to s.  MASS is known to the compiler: with a
+// test of the pointer it multiplied by the mass or by 1 (7 % of the FP64 pipe's
+// time).
+template <bool MASS>
 __device__ __forceinline__ void add_pair_f64(const double* pos, long long i, long long j,
                                              double eps2, const double* masses, bool ieee,
                                              double* s) {
-  const double mj = masses ? masses[j] : 1.0;
+  const double mj = MASS ? masses[j] : 1.0;
   if (ieee) {
     double ax, ay, az;
     pair_term_f64(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], pos[3 * j], pos[3 * j + 1],
                   pos[3 * j + 2], eps2, ax, ay, az);
-    if (masses) {
+    if (MASS) {
       ax = dmul(ax, mj);
       ay = dmul(ay, mj);
       az = dmul(az, mj);
@@ -190,7 +193,7 @@ __device__ __forceinline__ void add_pair_f64(const double* pos, long long i, lon
     const double dy = pos[3 * j + 1] - pos[3 * i + 1];
     const double dz = pos[3 * j + 2] - pos[3 * i + 2];
     double r3 = rinv3_f64(fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))));
-    if (masses) r3 *= mj;
+    if (MASS) r3 *= mj;
     s[0] = fma(dx, r3, s[0]);
     s[1] = fma(dy, r3, s[1]);
     s[2] = fma(dz, r3, s[2]);
@@ -202,6 +205,7 @@ __device__ __forceinline__ void add_pair_f64(const double* pos, long long i, lon
 // by side: as many rounds as the warp's lane with most of them, which is
 // returned.  sorted: the records, where they are not in the order of the
 // bodies, else null.  The whole warp calls it.
+template <bool MASS>
 static __device__ __noinline__ int fx_chunk_f64(unsigned mask, int steps, long long j0, int p0,
                                                 int L, const FxBody* sorted, const double* pos,
                                                 long long i, double eps2, const double* masses,
@@ -215,7 +219,7 @@ static __device__ __noinline__ int fx_chunk_f64(unsigned mask, int steps, long l
       mask &= ~(0x80000000u >> __clz(mask));
       const int p = p0 + u * L;
       const long long j = j0 + (sorted ? fx_tag_index(sorted[p].tag) : p);
-      if (j != i) add_pair_f64(pos, i, j, eps2, masses, ieee, s);
+      if (j != i) add_pair_f64<MASS>(pos, i, j, eps2, masses, ieee, s);
     }
   }
   return rounds;
@@ -290,7 +294,8 @@ __device__ __noinline__ bool force_fx_tiles(const double* __restrict__ pos, long
                                             long long i0, long long jb, long long je, double eps2,
                                             const double* __restrict__ masses, int ex, int em,
                                             int flat, bool ieee, int T, int L, int tid, int bar,
-                                            FxBody* rec, const FxRow* tab, double (*part)[3]) {
+                                            FxBody* rec, const FxRow* tab, double (*part)[3],
+                                            bool in_f64) {
   constexpr bool MASS = MASSES != kFxEqual, CLASSES = MASSES == kFxClasses;
   const int b = tid / L;
   const int l = tid % L;
@@ -306,8 +311,8 @@ __device__ __noinline__ bool force_fx_tiles(const double* __restrict__ pos, long
   FxTot tot[3] = {};
   FxSize size = {};  // of the terms, in the heaviest class's units
   double near[3] = {};
-  bool in_f64 = false, any_near = false;  // uniform in the warp
-  int terms = 0, slow = 0;                // a lane's terms, and those of them in FP64
+  bool any_near = false;  // uniform in the warp, as in_f64: all terms in FP64
+  int terms = 0, slow = 0;  // a lane's terms, and those of them in FP64
   for (long long j0 = jb; j0 < je; j0 += T) {
     const int cnt = (int)min((long long)T, je - j0);
     fx_stage<MASSES>(rec, pos, masses, j0 + tid, cnt, ex, em, T, tid, bar);
@@ -356,7 +361,7 @@ __device__ __noinline__ bool force_fx_tiles(const double* __restrict__ pos, long
         if (!valid) mask = 0;
         if (own >= base && own < end && (own - base) % L == l)  // not the body itself
           mask &= ~(1u << (steps - 1 - (own - c0) / L));
-        rounds = fx_chunk_f64(mask, steps, j0, c0, L, CLASSES ? rec : nullptr, pos, i, eps2,
+        rounds = fx_chunk_f64<MASS>(mask, steps, j0, c0, L, CLASSES ? rec : nullptr, pos, i, eps2,
                               masses, ieee, near);
         any_near = any_near || rounds > 0;
       }
@@ -438,28 +443,40 @@ static __device__ __noinline__ void fx_bodies_wide(unsigned lanes, const double*
     FxSize size = {};
     double v[3] = {};
     int terms = 0;
-    bool in_f64 = classes;
+    bool any_f64 = classes;  // uniform in the warp
     FxAcc a[3] = {};
 #pragma unroll 1
-    for (long long j = jb + lane; j < je; j += 32) {
-      if (j == ib) continue;
+    for (long long j0 = jb; j0 < je; j0 += 32) {
+      const long long j = j0 + lane;
+      const bool on = j < je && j != ib;
+      const long long jr = on ? j : ib;
       FxBody r;
-      r.x = fx_from_double(pos[3 * j], ex);
-      r.y = fx_from_double(pos[3 * j + 1], ex);
-      r.z = fx_from_double(pos[3 * j + 2], ex);
+      r.x = fx_from_double(pos[3 * jr], ex);
+      r.y = fx_from_double(pos[3 * jr + 1], ex);
+      r.z = fx_from_double(pos[3 * jr + 2], ex);
       r.mu_lo = r.mu_hi = r.tag = 0;
-      if (masses) fx_mass(r, masses[j], em);
+      if (masses) fx_mass(r, masses[jr], em);
       const int cls = fx_tag_class(r.tag);
       FxSize z = {};
-      const bool near =
-          cls == kFxClassFp64 ||
-          (masses ? fx_term<true, true>(r, xi, yi, zi, eps2f, tab, a, z) > fx_max_k<true>()
-                  : fx_term<false, true>(r, xi, yi, zi, eps2f, tab, a, z) > fx_max_k<false>());
-      if (near) {
-        add_pair_f64(pos, ib, j, eps2, masses, ieee, v);
-        in_f64 = true;
+      // one lane's pair in FP64 takes the warp as long as all lanes'
+      const int max_k = masses ? kFxMaxKMass : kFxMaxK;
+      if (__any_sync(0xffffffffu, on && (cls == kFxClassFp64 ||
+                                         fx_norm(fx_sub(r.x, xi), fx_sub(r.y, yi),
+                                                 fx_sub(r.z, zi), eps2f, max_k) > max_k))) {
+        if (on) {
+          if (masses)
+            add_pair_f64<true>(pos, ib, j, eps2, masses, ieee, v);
+          else
+            add_pair_f64<false>(pos, ib, j, eps2, nullptr, ieee, v);
+        }
+        any_f64 = true;
         continue;
       }
+      if (!on) continue;
+      if (masses)
+        fx_term<true, true>(r, xi, yi, zi, eps2f, tab, a, z);
+      else
+        fx_term<false, true>(r, xi, yi, zi, eps2f, tab, a, z);
       size.m += classes ? scalbnf(z.m, -4 * cls) : z.m;
       if (classes) {
         const int sc = fx_out_exp(ex) + fx_class_exp(em, cls) + 1;
@@ -476,7 +493,6 @@ static __device__ __noinline__ void fx_bodies_wide(unsigned lanes, const double*
       }
     }
     const int sc = fx_out_exp(ex) + (masses ? fx_class_exp(em, 0) + 1 : 0);
-    const bool any_f64 = __any_sync(0xffffffffu, in_f64);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       fx_fold(tot[d], a[d]);
@@ -497,8 +513,13 @@ static __device__ __noinline__ void fx_bodies_wide(unsigned lanes, const double*
     if (__shfl_sync(0xffffffffu, (int)thin, 0)) {
 #pragma unroll
       for (int d = 0; d < 3; ++d) v[d] = 0.0;
-      for (long long j = jb + lane; j < je; j += 32)
-        if (j != ib) add_pair_f64(pos, ib, j, eps2, masses, ieee, v);
+      if (masses) {
+        for (long long j = jb + lane; j < je; j += 32)
+          if (j != ib) add_pair_f64<true>(pos, ib, j, eps2, masses, ieee, v);
+      } else {
+        for (long long j = jb + lane; j < je; j += 32)
+          if (j != ib) add_pair_f64<false>(pos, ib, j, eps2, nullptr, ieee, v);
+      }
 #pragma unroll
       for (int d = 0; d < 3; ++d) v[d] = lane_reduce<32>(v[d]);
     }
@@ -524,10 +545,23 @@ __device__ __forceinline__ double key_bound(int key, bool upper) {
 // `flat` (bits) the bodies have one coordinate; wide: another axis is so short
 // that three words are called for from the start (kFxNarrow), thin: so short that
 // most bodies' sums would be in FP64 as well (kFxThin).
+// near, of the warp's bodies: 7 in 8 of a sample of pairs are below the window (with
+// wide, whose lanes wait for the one that has such a pair, 1 in 8), so it takes
+// all terms in FP64 from the start: the count in the tiles comes after 32 terms of
+// a lane, all it has at N = 1024 (one body at 1e5 radii 115 -> 109 us, in FP64 alone
+// 104).
 struct FxShape {
   int flat;
-  bool wide, thin;
+  bool wide, thin, near;
 };
+
+// A coordinate in units of 2^ex from its high word, |v| < 2^(ex + 64).
+__device__ __forceinline__ float fx_coarse(int hi, int ex) {
+  const int e = (hi >> 20 & 0x7ff) - 1023 - ex + 127;
+  return e > 0 && e < 192
+             ? __int_as_float((hi & 0x80000000) | e << 23 | (hi & 0xfffff) << 3)
+             : 0.0f;
+}
 
 // The grid of a group's own body i and of the `count` partners from jb on
 // (modulo n): exponents ex and, with masses, em, whether the masses are of more
@@ -542,12 +576,13 @@ static __device__ __noinline__ bool fx_grid(const double* __restrict__ pos, long
                                             int* em_out, bool* classes_out, FxShape* shape_out) {
   if (count == 0) return false;
   const int nw = T / 32;
-  int lo[3], hi[3];
+  int lo[3], hi[3], xi[3], xj[3] = {};
   int ref[3], other = 0;  // axes with a low word that is not the first partner's
   unsigned mm = 0, ml = 0xffffffffu;
   int off[3] = {};
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
+    xi[c] = __double2hiint(pos[3 * i + c]);
     lo[c] = hi[c] = order_key(pos[3 * i + c]);
     ref[c] = __double2loint(pos[3 * jb + c]);
     off[c] = __double2loint(pos[3 * i + c]) ^ ref[c];
@@ -562,6 +597,7 @@ static __device__ __noinline__ bool fx_grid(const double* __restrict__ pos, long
       lo[c] = min(lo[c], k);
       hi[c] = max(hi[c], k);
       off[c] |= __double2loint(x) ^ ref[c];
+      xj[c] = __double2hiint(x);
     }
   }
 #pragma unroll
@@ -634,7 +670,18 @@ static __device__ __noinline__ bool fx_grid(const double* __restrict__ pos, long
   if (ex < -300 || ex > 300 || (masses && (em < -300 || em > 300))) return false;
   *ex_out = ex;
   *em_out = em;
-  *shape_out = FxShape{flat, wide, thin};
+  float r2 = fx_eps2f(eps2, ex) * 0x1p-60f;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const float d = fx_coarse(xj[c], ex) - fx_coarse(xi[c], ex);
+    r2 += d * d;
+  }
+  const int k = masses ? kFxMaxKMass : kFxMaxK;
+  const unsigned have = __ballot_sync(0xffffffffu, tid < count);
+  const unsigned below = __ballot_sync(
+      0xffffffffu, tid < count && r2 < __int_as_float((127 - 2 * k) << 23));
+  const bool near = __popc(have) >= 16 && 8 * __popc(below) >= (wide ? 1 : 7) * __popc(have);
+  *shape_out = FxShape{flat, wide, thin, near};
   *classes_out = masses && (int)(ml >> 20) < (int)(mm >> 20) - 3;
   return true;
 }
@@ -663,17 +710,21 @@ static __device__ __noinline__ bool force_fx_group(const double* __restrict__ po
   if (tid < kFxRows) tab[tid] = fx_row(tid, eps2, ex);
   const long long i = i0 + tid / L;
   bool thin = tid % L == 0 && i < n;
-  if (shape.wide)
-    group_bar(bar, T);  // the table is there
-  else if (!masses)
+  if (shape.wide) {
+    // these sums take one body after the other; FP64 terms are better taken together
+    if ((tid & 31) == 0) red[tid / 32] = shape.near;
+    group_bar(bar, T);  // and the table is there
+    for (int w = 0; w < T / 32; ++w)
+      if (red[w]) return false;
+  } else if (!masses)
     thin = force_fx_tiles<kFxEqual>(pos, n, i0, jb, je, eps2, nullptr, ex, 0, flat, ieee, T, L, tid,
-                                    bar, rec, tab, part);
+                                    bar, rec, tab, part, shape.near);
   else if (!classes)
     thin = force_fx_tiles<kFxOneClass>(pos, n, i0, jb, je, eps2, masses, ex, em, flat, ieee, T, L,
-                                       tid, bar, rec, tab, part);
+                                       tid, bar, rec, tab, part, shape.near);
   else
     thin = force_fx_tiles<kFxClasses>(pos, n, i0, jb, je, eps2, masses, ex, em, flat, ieee, T, L,
-                                      tid, bar, rec, tab, part);
+                                      tid, bar, rec, tab, part, shape.near);
   const unsigned lanes = __ballot_sync(0xffffffffu, thin);
   if (lanes) {
     double v[3];
@@ -684,6 +735,72 @@ static __device__ __noinline__ bool force_fx_group(const double* __restrict__ po
     }
   }
   return true;
+}
+
+// The FP64 terms of one CTA or group, a lane's partners in ascending order.  Not
+// inlined and for masses or none (add_pair_f64): in some of the kernels the
+// compiler had multiplied by a mass of 1 (N = 1024 103 -> 110 us).
+template <bool MASS>
+static __device__ __noinline__ void force_f64_tiles(const double* __restrict__ pos, long long n,
+                                                    long long i0, long long jb, long long je,
+                                                    double eps2,
+                                                    const double* __restrict__ masses, bool ieee,
+                                                    double* sh_pos, int T, int L, int tid, int bar,
+                                                    double* sum) {
+  double* sh_m = sh_pos + 3 * T;
+  const int l = tid % L;
+  const long long i = i0 + tid / L;
+  double xi = 0.0, yi = 0.0, zi = 0.0;
+  if (i < n) {
+    xi = pos[3 * i];
+    yi = pos[3 * i + 1];
+    zi = pos[3 * i + 2];
+  }
+  double sx = 0.0, sy = 0.0, sz = 0.0;
+  for (long long j0 = jb; j0 < je; j0 += T) {
+    const int cnt = (int)min((long long)T, je - j0);
+    group_bar(bar, T);
+    for (int k = tid; k < 3 * cnt; k += T) sh_pos[k] = pos[3 * j0 + k];
+    if (MASS)
+      for (int k = tid; k < cnt; k += T) sh_m[k] = masses[j0 + k];
+    group_bar(bar, T);
+    if (i >= n) continue;
+    if (!ieee) {
+      // N = 16384 13.2 ms without the unrolling
+#pragma unroll 4
+      for (int jj = l; jj < cnt; jj += L) {
+        if (j0 + jj == i) continue;
+        const double dx = sh_pos[3 * jj] - xi;
+        const double dy = sh_pos[3 * jj + 1] - yi;
+        const double dz = sh_pos[3 * jj + 2] - zi;
+        double r3 = rinv3_f64(fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))));
+        if (MASS) r3 *= sh_m[jj];
+        sx = fma(dx, r3, sx);
+        sy = fma(dy, r3, sy);
+        sz = fma(dz, r3, sz);
+      }
+    } else {
+      for (int jj = l; jj < cnt; jj += L) {
+        const long long j = j0 + jj;
+        if (j == i) continue;
+        double ax, ay, az;
+        pair_term_f64(xi, yi, zi, sh_pos[3 * jj], sh_pos[3 * jj + 1], sh_pos[3 * jj + 2], eps2,
+                      ax, ay, az);
+        if (MASS) {
+          const double mj = sh_m[jj];
+          ax = dmul(ax, mj);
+          ay = dmul(ay, mj);
+          az = dmul(az, mj);
+        }
+        sx = dadd(sx, ax);
+        sy = dadd(sy, ay);
+        sz = dadd(sz, az);
+      }
+    }
+  }
+  sum[0] = sx;
+  sum[1] = sy;
+  sum[2] = sz;
 }
 
 // ---------------------------------------------------------------------------
@@ -703,73 +820,25 @@ __device__ __forceinline__ void force_f64_cta(const double* __restrict__ pos, lo
                                               double eps2, const double* __restrict__ masses,
                                               unsigned char* smem, double (*part)[3], int pair,
                                               const G& grp = G{}) {
-  constexpr int BI = T / L;
   const bool ieee = pair == kPairIeee || pair == kPairFixedIeee;
   if (pair >= kPairFixedFast &&
       force_fx_group(pos, n, i0, jb, je, eps2, masses, ieee, smem, part, T, L, (int)grp.tid(),
                      grp.id()))
     return;
-  double* sh_pos = reinterpret_cast<double*>(smem);
-  double* sh_m = sh_pos + 3 * T;
-  const unsigned tid = grp.tid();
-  const int b = tid / L;
-  const int l = tid % L;
-  const long long i = i0 + b;
-  double xi = 0.0, yi = 0.0, zi = 0.0;
-  if (i < n) {
-    xi = pos[3 * i];
-    yi = pos[3 * i + 1];
-    zi = pos[3 * i + 2];
-  }
-  double sx = 0.0, sy = 0.0, sz = 0.0;
-  for (long long j0 = jb; j0 < je; j0 += T) {
-    const int cnt = (int)min((long long)T, je - j0);
-    grp.sync();
-    for (int k = tid; k < 3 * cnt; k += T) sh_pos[k] = pos[3 * j0 + k];
-    if (masses)
-      for (int k = tid; k < cnt; k += T) sh_m[k] = masses[j0 + k];
-    grp.sync();
-    if (i >= n) continue;
-    if (!ieee) {
-      for (int jj = l; jj < cnt; jj += L) {
-        if (j0 + jj == i) continue;
-        const double dx = sh_pos[3 * jj] - xi;
-        const double dy = sh_pos[3 * jj + 1] - yi;
-        const double dz = sh_pos[3 * jj + 2] - zi;
-        double r3 = rinv3_f64(fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))));
-        if (masses) r3 *= sh_m[jj];
-        sx = fma(dx, r3, sx);
-        sy = fma(dy, r3, sy);
-        sz = fma(dz, r3, sz);
-      }
-    } else {
-      for (int jj = l; jj < cnt; jj += L) {
-        const long long j = j0 + jj;
-        if (j == i) continue;
-        double ax, ay, az;
-        pair_term_f64(xi, yi, zi, sh_pos[3 * jj], sh_pos[3 * jj + 1], sh_pos[3 * jj + 2], eps2,
-                      ax, ay, az);
-        if (masses) {
-          const double mj = sh_m[jj];
-          ax = dmul(ax, mj);
-          ay = dmul(ay, mj);
-          az = dmul(az, mj);
-        }
-        sx = dadd(sx, ax);
-        sy = dadd(sy, ay);
-        sz = dadd(sz, az);
-      }
-    }
-  }
-  sx = lane_reduce<L>(sx);
-  sy = lane_reduce<L>(sy);
-  sz = lane_reduce<L>(sz);
+  double s[3];
+  if (masses)
+    force_f64_tiles<true>(pos, n, i0, jb, je, eps2, masses, ieee, reinterpret_cast<double*>(smem),
+                          T, L, (int)grp.tid(), grp.id(), s);
+  else
+    force_f64_tiles<false>(pos, n, i0, jb, je, eps2, nullptr, ieee,
+                           reinterpret_cast<double*>(smem), T, L, (int)grp.tid(), grp.id(), s);
+  const int b = grp.tid() / L, l = grp.tid() % L;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) s[d] = lane_reduce<L>(s[d]);
   if (l == 0) {
-    part[b][0] = sx;
-    part[b][1] = sy;
-    part[b][2] = sz;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) part[b][d] = s[d];
   }
-  (void)BI;
 }
 
 // ---------------------------------------------------------------------------

@@ -422,10 +422,15 @@ __global__ void batch_elem_kernel(const BatchParams P, int mode, const double* _
   }
 }
 
-// Per-system RMS norm of v / s in a fixed order: a cluster of 4 CTAs per
-// system, thread sums, a tree per CTA, then the CTAs in rank order.  Bound by
-// the FP64 pipe (an IEEE division, a multiply and an add an element): one warp
-// per system left a 4096-body system 280 us on one sub-partition.
+// Per-system RMS norm of v / s in a fixed order.  Bound by the FP64 pipe (an IEEE
+// division, a multiply and an add an element).  A system of more than
+// kWarpNormBodies: a cluster of 4 CTAs, thread sums, a tree per CTA, then the CTAs
+// in rank order (one warp left a 4096-body system 280 us on one sub-partition).
+// Up to that, 252 elements: a warp, of which four share a CTA, as the cluster's
+// launch alone takes longer (2000 systems of 16 to 32 bodies, a start of the
+// batch in mixed precision: 468 us with clusters, 306 so).  Which of the two is by
+// the system's own size, so its norm does not depend on the others.
+constexpr long long kWarpNormBodies = 42;
 constexpr int kNormCtas = 4, kNormThreads = 256;
 __global__ void __cluster_dims__(kNormCtas, 1, 1) __launch_bounds__(kNormThreads)
     batch_norm_kernel(const BatchParams P, const double* __restrict__ v,
@@ -434,6 +439,7 @@ __global__ void __cluster_dims__(kNormCtas, 1, 1) __launch_bounds__(kNormThreads
   __shared__ double part;
   const int k = blockIdx.x / kNormCtas, rank = blockIdx.x % kNormCtas;
   const BSys sy = P.sys[k];
+  if (sy.n <= kWarpNormBodies) return;  // the whole cluster
   const long long nv = 6 * sy.n;
   double acc = 0.0;
   for (long long e = rank * kNormThreads + threadIdx.x; e < nv; e += kNormCtas * kNormThreads) {
@@ -450,6 +456,23 @@ __global__ void __cluster_dims__(kNormCtas, 1, 1) __launch_bounds__(kNormThreads
     out[3 * k + slot] = sqrt(t / (double)nv);
   }
   cl.sync();
+}
+__global__ void __launch_bounds__(128)
+    batch_norm_warp_kernel(const BatchParams P, const double* __restrict__ v,
+                           const double* __restrict__ s, double* __restrict__ out, int slot) {
+  const int k = blockIdx.x * 4 + threadIdx.x / 32, lane = threadIdx.x % 32;
+  if (k >= P.n_sys) return;
+  const BSys sy = P.sys[k];
+  if (sy.n > kWarpNormBodies) return;
+  const long long nv = 6 * sy.n;
+  double acc = 0.0;
+  for (long long e = lane; e < nv; e += 32) {
+    const double q = __ddiv_rn(v[sy.var_off + e], s[sy.var_off + e]);
+    acc = dadd(acc, dmul(q, q));
+  }
+#pragma unroll
+  for (int off = 16; off >= 1; off /= 2) acc = dadd(acc, __shfl_xor_sync(0xffffffffu, acc, off));
+  if (lane == 0) out[3 * k + slot] = sqrt(acc / (double)nv);
 }
 
 // The systems' current states, one after the other.
@@ -722,6 +745,22 @@ int set_geometry(gb_batch_s* b, int T, int L, int BPT, int G, int grid) {
   return GB_OK;
 }
 
+// CTAs of 256 threads for the element-wise kernels: up to 4 a system, as many as the
+// largest one fills.
+dim3 elem_grid(const gb_batch_s* b) {
+  const long long n = *std::max_element(b->n.begin(), b->n.end());
+  return dim3((unsigned)b->n_sys, (unsigned)std::min<long long>(4, (6 * n + 255) / 256));
+}
+
+void launch_norms(gb_batch_s* b, const double* v, const double* s, int slot) {
+  const auto [lo, hi] = std::minmax_element(b->n.begin(), b->n.end());
+  if (*hi > kWarpNormBodies)
+    batch_norm_kernel<<<b->n_sys * kNormCtas, kNormThreads, 0, b->stream>>>(b->P, v, s, b->dscal,
+                                                                           slot);
+  if (*lo <= kWarpNormBodies)
+    batch_norm_warp_kernel<<<(b->n_sys + 3) / 4, 128, 0, b->stream>>>(b->P, v, s, b->dscal, slot);
+}
+
 int launch_stage(gb_batch_s* b, int s) {
   void* args[] = {(void*)&b->tab, (void*)&b->P, (void*)&s};
   GB_CUDA_TRY(cudaLaunchKernel(b->k.stage, dim3(b->grid), dim3(b->T), args, 0, b->stream));
@@ -955,16 +994,16 @@ extern "C" int gb_batch_start(gb_batch b, const double* x0, const double* t0, co
   double* x1 = b->Y + tv;
   double* f0 = b->ks;
   double* df = b->ks + tv;
-  batch_elem_kernel<<<dim3(ns, 4), 256, 0, s>>>(P, 0, b->ring, nullptr, tg, nullptr);
+  batch_elem_kernel<<<elem_grid(b), 256, 0, s>>>(P, 0, b->ring, nullptr, tg, nullptr);
   GB_TRY(launch_rhs(b, b->ring, b->PX, f0));
-  batch_norm_kernel<<<ns * kNormCtas, kNormThreads, 0, s>>>(P, b->ring, tg, b->dscal, 0);
-  batch_norm_kernel<<<ns * kNormCtas, kNormThreads, 0, s>>>(P, f0, tg, b->dscal, 1);
-  batch_elem_kernel<<<dim3(ns, 4), 256, 0, s>>>(P, 1, b->ring, f0, x1, b->dscal);
+  launch_norms(b, b->ring, tg, 0);
+  launch_norms(b, f0, tg, 1);
+  batch_elem_kernel<<<elem_grid(b), 256, 0, s>>>(P, 1, b->ring, f0, x1, b->dscal);
   if (b->opts.precision == GB_PREC_MIXED)
     batch_pack_kernel<<<(unsigned)((tb + 255) / 256), 256, 0, s>>>(P, x1, b->PY);
   GB_TRY(launch_rhs(b, x1, b->PY, df));
-  batch_elem_kernel<<<dim3(ns, 4), 256, 0, s>>>(P, 2, nullptr, f0, df, nullptr);
-  batch_norm_kernel<<<ns * kNormCtas, kNormThreads, 0, s>>>(P, df, tg, b->dscal, 2);
+  batch_elem_kernel<<<elem_grid(b), 256, 0, s>>>(P, 2, nullptr, f0, df, nullptr);
+  launch_norms(b, df, tg, 2);
   const int q = std::min(b->htab.p, b->htab.pt);
   const double safety = std::pow(0.38, 1.0 / (1.0 + q));
   batch_init_ctrl_kernel<<<(ns + 127) / 128, 128, 0, s>>>(P, b->dscal, b->tv, b->tv + ns,
@@ -1047,7 +1086,7 @@ extern "C" int gb_batch_state(gb_batch b, double* x_dev, double* t_host) {
   if (!b || !b->started) return GB_ERR_INVALID_ARGUMENT;
   GB_TRY(read_ctrl(b));
   if (x_dev) {
-    batch_state_kernel<<<dim3(b->n_sys, 4), 256, 0, b->stream>>>(b->P, x_dev);
+    batch_state_kernel<<<elem_grid(b), 256, 0, b->stream>>>(b->P, x_dev);
     GB_CUDA_TRY(cudaGetLastError());
   }
   if (t_host)

@@ -22,7 +22,7 @@
 // within 2^-55 of its size (0.04 2^-53 rms; a term in FP64: 1.3 2^-53 rms, up to
 // 5 2^-53).  Its components are products of two words' precision, 2^-57 of the
 // term and not of the component; the sizes of a sum's terms and of their
-// components say where that is not enough (kFxNarrow, kFxThin), and those sums
+// components say where that is not enough (kFxEnough, kFxThin), and those sums
 // are taken with three words or in FP64, so that every component is as good as
 // its FP64 sum.
 //
@@ -56,7 +56,7 @@ struct Fx96 {  // two's complement, w0 least significant
   uint32_t w0, w1, w2;
 };
 
-// row k of the softening table: eps^2 at normalisation k, the weight 4^k twice
+// row k of the softening table: eps^2 at normalisation k, the weight 4^k, 8^k 2^-62
 struct alignas(16) FxRow {
   uint32_t e_lo, e_hi;
   uint32_t p;
@@ -393,7 +393,7 @@ GB_HD FxRow fx_row(int k, double eps2, int ex) {
   const int sh = ee - 1075 + 2 * (30 - ex + k);
   const uint64_t e = (sh > 9 ? 1ull << 62 : sh >= 0 ? m << sh : sh > -64 ? m >> -sh : 0) + 2;
   return FxRow{(uint32_t)e, (uint32_t)(e >> 32), k <= kFxMaxK ? 1u << (2 * k) : 0u,
-               k <= kFxMaxK ? (float)(1u << (2 * k)) : 0.0f};
+               k <= kFxMaxK ? fx_float_of((uint32_t)(127 - 62 + 3 * k) << 23) : 0.0f};
 }
 
 // A partner's record.  Per-body masses come in classes of four binary orders,
@@ -436,16 +436,19 @@ GB_HD void fx_mass(FxBody& b, double mass, int em) {
                  normal ? down >> 2 : bits << 1 ? kFxClassFp64 : 0, 0, 0);
 }
 
-// Sizes of the terms added, in FP32: m at least the sum of their sizes (as
-// S |d| <= 2^151 / R), c[3] the sums of their components' sizes; units of 2^30
-// of V's.
+// Sizes of the terms added.  Two words: the sum p of the weights (V is within
+// 0.8 2^32 p), and in FP32 the sums c[3] of the components' sizes, in units of
+// 2^31 of V's, with masses without their mantissas (at least half of it).  Three
+// words: m, at least the sum of the terms' sizes (as S |d| <= 2^151 / R), in units
+// of 2^30.
 struct FxSize {
-  float m, c[3];
+  uint32_t p;  // of kFxChunk terms
+  float c[3], m;
 };
 
-// One term of the accelerations into the three sums and its sizes into z (the
-// components' with two words only).  Returns its normalisation (above fx_max_k:
-// not added).  With masses the weight is 4^k 2^q.
+// One term of the accelerations into the three sums and its sizes into z.
+// Returns its normalisation (above fx_max_k: not added).  With masses the weight
+// is 4^k 2^q.
 template <bool MASS, bool WIDE>
 GB_HD int fx_term(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& zi, float eps2f,
                   const FxRow* tab, FxAcc (&a)[3], FxSize& z) {
@@ -459,16 +462,17 @@ GB_HD int fx_term(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& z
   float pf = row.pf;
   if (MASS) {
     s = fx_mul_hi(s << 1, fx_pair(j.mu_lo, j.mu_hi));  // 2 S mass 2^(-eb - q - 1)
-    p = k <= kFxMaxKMass ? p << fx_tag_q(j.tag) : 0u;
-    // times half the mantissa, of mu's 31 bits in the high word, and 2^q
-    const uint32_t half = (j.mu_hi >> 7 & 0x7fffffu) | (uint32_t)(126 + fx_tag_q(j.tag)) << 23;
-    pf = k <= kFxMaxKMass && j.mu_hi ? pf * fx_float_of(half) : 0.0f;
+    const bool on = k <= kFxMaxKMass && j.mu_hi != 0;
+    p = on ? p << fx_tag_q(j.tag) : 0u;
+    if (!WIDE)
+      pf = on ? fx_float_of(fx_float_bits(pf) + ((uint32_t)fx_tag_q(j.tag) << 23)) : 0.0f;
   }
-  const float t = pf * (yf * yf);
-  z.m += t;
-  if (!WIDE) {
+  if (WIDE) {
+    z.m += (float)p * (yf * yf);
+  } else {
+    z.p += p;
     // |h| = |high word| 2^k, and S = Y^3 2^-32
-    const float w = t * yf * fx_float_of((uint32_t)(127 - 61 + k) << 23);
+    const float w = pf * yf * (yf * yf);
     z.c[0] += w * fx_abs((float)(int32_t)ux.w2);
     z.c[1] += w * fx_abs((float)(int32_t)uy.w2);
     z.c[2] += w * fx_abs((float)(int32_t)uz.w2);
@@ -479,18 +483,12 @@ GB_HD int fx_term(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& z
   return k;
 }
 
-// What a body's term with itself adds to z.m (its components are zero).
+// What a body's term with itself adds to z.p (its components are zero).
 template <bool MASS>
-GB_HD float fx_self_size(float eps2f, const FxRow* tab, const FxBody& j) {
+GB_HD uint32_t fx_self_weight(float eps2f, const FxRow* tab, const FxBody& j) {
   const int k = fx_norm(Fx96{}, Fx96{}, Fx96{}, eps2f, fx_max_k<MASS>());
-  if (k > fx_max_k<MASS>()) return 0.0f;
-  const float yf = fx_rsqrt_seed_float(fx_pair(tab[k].e_lo, tab[k].e_hi));
-  float pf = tab[k].pf;
-  if (MASS)
-    pf = j.mu_hi ? pf * fx_float_of((j.mu_hi >> 7 & 0x7fffffu) |
-                                    (uint32_t)(126 + fx_tag_q(j.tag)) << 23)
-                 : 0.0f;
-  return pf * (yf * yf);
+  if (k > fx_max_k<MASS>()) return 0u;
+  return !MASS ? tab[k].p : j.mu_hi ? tab[k].p << fx_tag_q(j.tag) : 0u;
 }
 template <bool MASS>
 GB_HD int fx_term(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx96& zi, float eps2f,
@@ -520,14 +518,16 @@ GB_HD int fx_term_pot(const FxBody& j, const Fx96& xi, const Fx96& yi, const Fx9
   return k;
 }
 
-// Two words serve a component whose terms' sizes come to more than 2^-kFxNarrow of
-// all the terms' together: V's error, 2^-58 of a term at most and 2^-60 in the
-// mean, is then that of a term in FP64 (5 and 1.3 2^-53).  Three words
-// serve one whose sum is above 2^-kFxThin of the terms' sizes: V's 2 units and
-// the coordinates' last bits, 2^-80 of a term at most, are then within 2^-54 of
-// it.  A sum below that (of a body in a plane, nearly) is taken in FP64.
-constexpr int kFxNarrow = 8;
+// Two words serve a component whose terms' sizes come to 2^kFxEnough times the
+// weights or more, 2^-8 to 2^-10 of the terms: V's error, 0.8 2^32 of a weight at
+// most and 0.3 2^32 in the mean, is then 6 2^-53 and 2 2^-53 of it, as that of a
+// term in FP64 (5 and 1.3 2^-53).  Three words serve one whose sum is above
+// 2^-kFxThin of the terms' sizes: V's 2 units and the coordinates' last bits,
+// 2^-80 of a term at most, are then within 2^-54 of it.  A sum below that (of a
+// body in a plane, nearly) is taken in FP64.
+constexpr int kFxEnough = 82;
 constexpr int kFxThin = 26;
+constexpr int kFxShort = 8;  // an axis 2^-kFxShort of the longest: three words
 
 // exponent of a term's unit: sum 2^(fx_out_exp(ex)) is the sum of d / r^3, and
 // sum 2^(fx_out_exp(ex) + eb + 1) that of mass d / r^3; of the potential:

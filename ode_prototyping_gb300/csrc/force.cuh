@@ -309,7 +309,7 @@ __device__ __noinline__ bool force_fx_tiles(const double* __restrict__ pos, long
   }
   const float eps2f = fx_eps2f(eps2, ex);
   FxTot tot[3] = {};
-  FxSize size = {};  // of the terms, in the heaviest class's units
+  float weight = 0.0f, size[3] = {};  // of the terms, in the heaviest class's units
   double near[3] = {};
   bool any_near = false;  // uniform in the warp, as in_f64: all terms in FP64
   int terms = 0, slow = 0;  // a lane's terms, and those of them in FP64
@@ -343,16 +343,12 @@ __device__ __noinline__ bool force_fx_tiles(const double* __restrict__ pos, long
           const int k = fx_term<MASS, false>(rec[jj], xi, yi, zi, eps2f, tab, a, z);
           mask = __funnelshift_l((unsigned)(fx_max_k<MASS>() - k), mask, 1);  // 1 when k is above
         }
-        if (own >= base && own < end && (own - base) % L == l) {
-          // without the body itself, whose part may be far above the others': as
-          // much as the rounding of their sum with it
-          const float self = fx_self_size<MASS>(eps2f, tab, rec[own]);
-          z.m = fmaxf(z.m - self, 0.0f) + self * 0x1p-18f;
-        }
+        if (own >= base && own < end && (own - base) % L == l)
+          z.p -= fx_self_weight<MASS>(eps2f, tab, rec[own]);
         const float w = CLASSES ? scalbnf(1.0f, -4 * cls) : 1.0f;
-        size.m += w * z.m;
+        weight += w * (float)z.p;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) size.c[d] += w * z.c[d];
+        for (int d = 0; d < 3; ++d) size[d] += w * z.c[d];
 #pragma unroll
         for (int d = 0; d < 3; ++d) fx_fold(tot[d], a[d]);
       }
@@ -392,27 +388,26 @@ __device__ __noinline__ bool force_fx_tiles(const double* __restrict__ pos, long
       fx_tot_add_lane(tot[d], off);
       if (any_near) near[d] = dadd(near[d], __shfl_down_sync(0xffffffffu, near[d], off));
     }
-    size.m += __shfl_down_sync(0xffffffffu, size.m, off);
+    weight += __shfl_down_sync(0xffffffffu, weight, off);
 #pragma unroll
-    for (int d = 0; d < 3; ++d)
-      size.c[d] += __shfl_down_sync(0xffffffffu, size.c[d], off);
+    for (int d = 0; d < 3; ++d) size[d] += __shfl_down_sync(0xffffffffu, size[d], off);
   }
   double v[3];
   bool thin = false;
+  const float enough = weight * __int_as_float((127 + kFxEnough - 31) << 23);
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     v[d] = fx_to_double(tot[d], sc);
     if (any_near) v[d] = dadd(v[d], near[d]);
-    thin = thin || (!(flat >> d & 1) && size.c[d] * (1 << kFxNarrow) < size.m);
+    thin = thin || (!(flat >> d & 1) && size[d] < enough);
   }
   if (any_near && thin) {  // the terms in FP64 count as well
     const double least =
-        dmul((double)size.m, __hiloint2double((1023 + sc + 30 - kFxNarrow) << 20, 0));
+        dmul((double)weight, __hiloint2double((1023 + sc + kFxEnough) << 20, 0));
     thin = false;
 #pragma unroll
     for (int d = 0; d < 3; ++d)
-      thin = thin || (!(flat >> d & 1) && size.c[d] * (1 << kFxNarrow) < size.m &&
-                      !(fabs(near[d]) >= least));
+      thin = thin || (!(flat >> d & 1) && size[d] < enough && !(fabs(near[d]) >= least));
   }
   if (l == 0) {
 #pragma unroll
@@ -440,7 +435,7 @@ static __device__ __noinline__ void fx_bodies_wide(unsigned lanes, const double*
     const Fx96 xi = fx_from_double(pos[3 * ib], ex), yi = fx_from_double(pos[3 * ib + 1], ex),
                zi = fx_from_double(pos[3 * ib + 2], ex);
     FxTot tot[3] = {};
-    FxSize size = {};
+    float size = 0.0f;  // of the terms
     double v[3] = {};
     int terms = 0;
     bool any_f64 = classes;  // uniform in the warp
@@ -477,7 +472,7 @@ static __device__ __noinline__ void fx_bodies_wide(unsigned lanes, const double*
         fx_term<true, true>(r, xi, yi, zi, eps2f, tab, a, z);
       else
         fx_term<false, true>(r, xi, yi, zi, eps2f, tab, a, z);
-      size.m += classes ? scalbnf(z.m, -4 * cls) : z.m;
+      size += classes ? scalbnf(z.m, -4 * cls) : z.m;
       if (classes) {
         const int sc = fx_out_exp(ex) + fx_class_exp(em, cls) + 1;
 #pragma unroll
@@ -502,13 +497,13 @@ static __device__ __noinline__ void fx_bodies_wide(unsigned lanes, const double*
       v[d] = any_f64 ? dadd(t, lane_reduce<32>(v[d])) : t;
     }
 #pragma unroll
-    for (int off = 16; off >= 1; off /= 2) size.m += __shfl_down_sync(0xffffffffu, size.m, off);
+    for (int off = 16; off >= 1; off /= 2) size += __shfl_down_sync(0xffffffffu, size, off);
     // exponents: of a component, and of 2^-kFxThin of the sizes
-    const int least = (int)(fx_float_bits(size.m) >> 23) - 127 + sc + 30 - kFxThin;
+    const int least = (int)(fx_float_bits(size) >> 23) - 127 + sc + 30 - kFxThin;
     bool thin = false;
 #pragma unroll
     for (int d = 0; d < 3; ++d)
-      thin = thin || (size.m > 0.0f && !(flat >> d & 1) &&
+      thin = thin || (size > 0.0f && !(flat >> d & 1) &&
                       (__double2hiint(v[d]) >> 20 & 0x7ff) - 1023 <= least);
     if (__shfl_sync(0xffffffffu, (int)thin, 0)) {
 #pragma unroll
@@ -543,7 +538,7 @@ __device__ __forceinline__ double key_bound(int key, bool upper) {
 
 // What the extents say of the accelerations' components: along the axes of
 // `flat` (bits) the bodies have one coordinate; wide: another axis is so short
-// that three words are called for from the start (kFxNarrow), thin: so short that
+// that three words are called for from the start (kFxShort), thin: so short that
 // most bodies' sums would be in FP64 as well (kFxThin).
 // near, of the warp's bodies: 7 in 8 of a sample of pairs are below the window (with
 // wide, whose lanes wait for the one that has such a pair, 1 in 8), so it takes
@@ -663,7 +658,7 @@ static __device__ __noinline__ bool fx_grid(const double* __restrict__ pos, long
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     if (flat >> c & 1) continue;
-    wide = wide || xe[c] - 1022 < ex - kFxNarrow;
+    wide = wide || xe[c] - 1022 < ex - kFxShort;
     thin = thin || xe[c] - 1022 < ex - kFxThin + 2;
   }
   const int em = (int)(mm >> 20) - 1023;  // 2^em <= the largest mass < 2^(em + 1)

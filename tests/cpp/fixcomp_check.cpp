@@ -3,7 +3,7 @@
 // 2^-40, near the origin (coordinates off the grid) and away from it. Prints the largest error of a
 // component above 2^-kFxThin of the bound of the term's size, in units of 2^-53 of itself, and how
 // many were above and below; a term above its bound, or a bound more than twice it without
-// softening, fails; the same with two words for components above 2^-kFxNarrow. Then the 160-bit total.
+// softening, fails; the same with two words for components above 2^kFxEnough weights. Then the 160-bit total.
 #include <cmath>
 #include <cstdio>
 #include <random>
@@ -48,7 +48,6 @@ int main() {
               if (fx_term<false, true>(j, x, y, z, e2, tab, a, zw) > kFxMaxK) continue;
               FxAcc an[3] = {};
               fx_term<false, false>(j, x, y, z, e2, tab, an, zn);
-              if (zn.m != zw.m) return 5;
               const Q size = ldexpl((Q)zw.m, fx_out_exp(0) + 30);
               const Q s = 1 / (r2 * sqrtl(r2));
               const Q dist = sqrtl(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
@@ -61,8 +60,8 @@ int main() {
                   if (tot != 0) return 3;
                   continue;
                 }
-                if (zn.c[c] * (1 << kFxNarrow) >= zn.m) {
-                  if (fabsl(ldexpl((Q)zn.c[c], fx_out_exp(0) + 30) / (s * fabsl(d[c])) - 1) > 0.01) return 6;
+                if (zn.c[c] >= ldexpf((float)zn.p, kFxEnough - 31)) {
+                  if (fabsl(ldexpl((Q)zn.c[c], fx_out_exp(0) + 31) / (s * fabsl(d[c])) - 1) > 0.01) return 6;
                   __int128 t2 = 0;
                   fx_fold(t2, an[c]);
                   const Q got = ldexpl((Q)t2, fx_out_exp(0));

@@ -18,5 +18,5 @@ def test_components_within_2_to_minus_53(tmp_path):
     out = r.stdout.split()
     assert r.returncode == 0 and out[4] == "ok", (r.returncode, out)
     assert float(out[0]) <= 0.75 and int(out[1]) > 100000 and int(out[2]) > 10000, out
-    # two words: 2^-58 of the term is 8 units of 2^-53 of a component 2^-8 of it
+    # two words: 0.8 2^32 of a weight is 6.4 units of 2^-53 of 2^82 weights, the term half a unit
     assert float(out[3]) <= 8.75, out

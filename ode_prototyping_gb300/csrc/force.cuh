@@ -140,7 +140,8 @@ struct WarpGroup {
   __device__ __forceinline__ unsigned tid() const { return t; }
   __device__ __forceinline__ int id() const { return bar; }
   __device__ __forceinline__ void sync() const {
-    // immediate ids, so the kernel reserves barriers 0..4 only
+    // immediate ids, so that this reserves barriers 0..4 only (group_bar, in the
+    // FP64 kernels, has its id at run time and reserves all 16)
     switch (bar) {
       case 1: asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory"); break;
       case 2: asm volatile("bar.sync 2, %0;" ::"n"(T) : "memory"); break;

@@ -88,7 +88,7 @@ struct FusedParams {
   const double* cref;  // reference point for hi/lo packing
   double* partials;    // n_parts: per (i-tile, cluster rank) scaled-square sums
   double* sq;          // n_var (exact mode)
-  double* aux;         // n_parts (max |a| partials)
+  double* aux;         // n_parts (max |a|^2 partials)
   StepLog* log;        // log_capacity records or null
   long long log_capacity;
   const void* mlp;     // device MLP weights (learned controller) or null

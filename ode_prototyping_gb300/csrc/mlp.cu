@@ -9,9 +9,9 @@
 //              thread per parameter sums its gradient over the batch in
 //              sample order (deterministic, no atomics);
 //   adam     : one thread per parameter.
-// A training epoch (gb_mlp_train) is three kernels, deterministic as well:
-// samples (forward, loss and deltas, a thread per output), gradients (sums over
-// a slice of the samples) and update (the slices' sums in order, then Adam).
+// A training epoch (gb_mlp_train) is two kernels, deterministic as well: epoch
+// (forward, loss, deltas and gradient sums of a slice of the samples) and update
+// (the slices' sums in order, then Adam).
 // Inference in the controller uses BF16-rounded weights with FP32
 // accumulation (mlp.cuh); gb_mlp_infer_bf16 exposes the same arithmetic.
 #include <algorithm>
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(kEpochThreads)
 
 // The slices' sums of 32 parameters (warp g adds slices g, g + 16, ... in order,
 // then the warps' sums are added in order), rounded to FP32, and the Adam step.
-// Bound by the latency of the loads: all of a warp's in flight at once up to 144
+// Bound by the latency of the loads: all of a warp's in flight at once up to 160
 // slices (8 warps and 5 slices at a time: 9.4 us, so 6.0; the epoch 26.8 -> 25.0).
 constexpr int kUpdateWarps = 16;
 constexpr int kUpdateLoads = 10;  // slices of a warp loaded together: 160 cover the SMs

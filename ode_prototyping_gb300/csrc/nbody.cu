@@ -26,8 +26,8 @@ enum { kModeRhs = 0, kModeAccWrite = 1, kModeAccAdd = 2 };
 // at most 4 CTAs per SM, whose launches are short (N = 257 FP64 10.25 -> 8.96 us
 // a call, 3001 1846 -> 1807 us for 16 steps of leapfrog; N = 4096 mixed 28.7 -> 24.7
 // us); beyond that the loops run 0.3-0.6 % faster with their pointers left
-// __restrict__ (N = 16384 FP64, 100003 mixed).  A kernel of at most kFewCtas CTAs
-// lets the next one's wait beside it; more of them leave the next kernel's
+// __restrict__ (N = 16384 FP64, 100003 mixed).  A kernel of at most kFewCtas CTAs,
+// half the SMs, lets the next one's wait beside it; more of them leave the next kernel's
 // unevenly spread over the SMs (3001: 2088 us for the 16 steps where they may).
 constexpr unsigned kFewCtas = 76;
 constexpr int kAfterCtasPerSm = 4;
@@ -156,8 +156,9 @@ __global__ void pack_kernel(const double* __restrict__ pos, const double* __rest
 }
 
 // Registers: the one-lane packed loop (large systems) runs fastest with 56, 9
-// CTAs of 128 threads on an SM (N = 100003 4.62 ms; 4.68 at 8, 4.80 at 10, 4.87
-// at 5, 5.2 at 6 and 7; the same order at 16384 and 65536), the other forms,
+// CTAs of 128 threads on an SM (N = 100003 4.79 ms, 4.88 with those of 5; in one
+// sweep, ms: 4.62 at 9, 4.68 at 8, 4.80 at 10, 4.87 at 5, 5.2 at 6 and 7; the same
+// order at 16384 and 65536), the other forms,
 // whose launches are shorter, with what 5 CTAs leave.
 template <int T, int L, int BPT, bool PACKED, bool AFTER = false>
 __global__ void __launch_bounds__(T, (PACKED && L == 1 && BPT == 1 ? 9 : 5) * 128 / T)
@@ -371,10 +372,10 @@ ForceGeom choose_geom(long long n, int precision, const gb_force_tiling* tiling,
     g.P = 1;
   } else if (precision == GB_PREC_F64) {
     if (n >= 4096) {
-      // 8 cluster ranks and lanes for about 2048 CTAs of 128 threads: the
-      // FP64-pipe-bound pair loop then balances across the SMs (measured per
-      // stage: N = 16384 23.9 ms at 8 x 2 against 25.5 ms at 4 x 1; N = 4096
-      // 1.51 ms at 8 x 8 against 1.60 ms at 8 x 2)
+      // 8 cluster ranks and lanes for about 2048 CTAs of 128 threads, so that
+      // the pair loop balances across the SMs.  Chosen with FP64 terms (a stage,
+      // ms: N = 16384 23.9 at 8 x 2 against 25.5 at 4 x 1; 4096 1.51 at 8 x 8
+      // against 1.60 at 8 x 2) and kept for the fixed-point terms (1.67 and 0.137).
       int L = 1;
       while (L < 8 && (long long)L * 2 * n <= 32768) L *= 2;
       g.P = 8;

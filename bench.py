@@ -962,9 +962,10 @@ def run_other_workload(args):
         # error, error target, scaled norm.  Two ceilings per kernel: HBM
         # (algorithmic bytes = every vector element read or written once,
         # against the measured copy bandwidth) and the FP64 pipe (the IEEE
-        # multiply and add per coefficient that bit-for-bit parity needs; a
-        # division counted as ~9 FP64 instructions of a Newton-Raphson
-        # sequence; GB300: 1.25 TFLOP/s = 0.625e12 FP64 instructions/s).
+        # additions that bit-for-bit parity needs -- the products by constants
+        # are formed on the integer pipes; a division counted as ~9 FP64
+        # instructions of a Newton-Raphson sequence; GB300: 1.25 TFLOP/s =
+        # 0.625e12 FP64 instructions/s).
         import ctypes as C
         pk, src = peaks()
         fp64_ips = FP64_TFLOPS_NOMINAL * 1e12 / 2
@@ -987,10 +988,10 @@ def run_other_workload(args):
         cases = []
         for s in range(1, S):
             nnz = sum(1 for j in range(s) if t.a[s - 1][j] != 0.0)
-            cases.append((f"rk_stage_{s}", 8 * nv * (nnz + 2), nv * (2 * nnz + 2),
+            cases.append((f"rk_stage_{s}", 8 * nv * (nnz + 2), nv * (nnz + 1),
                           lambda s=s: gb.rk_stage(t, s, 1e-3, x0, ks, out, nv, stream)))
         cases.append(("rk_update_state_and_error", 8 * nv * (nb_u + 3),
-                      nv * (2 * nb_b + 2 * nb_d + 3),
+                      nv * (nb_b + nb_d + 1),
                       lambda: gb.rk_update(t, 1e-3, x0, ks, x, err, nv, stream)))
         cases.append(("rk_error_target", 8 * nv * 5, nv * 2,
                       lambda: gb.rk_error_target(atol, rtol, x, x0, tg, nv, stream)))

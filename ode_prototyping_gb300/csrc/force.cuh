@@ -808,19 +808,21 @@ static __device__ __noinline__ void force_f64_tiles(const double* __restrict__ p
 // multiply-add accumulation.  kPairFixed...: the fixed-point terms, and one of
 // the two where they do not apply.  With L lanes, lane l takes the partners
 // j = l (mod L) in ascending order whatever T is, so the sums do not depend on
-// the group size.
+// the group size.  FX false: the first two only, in 32 T bytes.
 // ---------------------------------------------------------------------------
-template <int T, int L, class G = WholeCta>
+template <int T, int L, bool FX = true, class G = WholeCta>
 __device__ __forceinline__ void force_f64_cta(const double* __restrict__ pos, long long n,
                                               long long i0, long long jb, long long je,
                                               double eps2, const double* __restrict__ masses,
                                               unsigned char* smem, double (*part)[3], int pair,
                                               const G& grp = G{}) {
   const bool ieee = pair == kPairIeee || pair == kPairFixedIeee;
-  if (pair >= kPairFixedFast &&
-      force_fx_group(pos, n, i0, jb, je, eps2, masses, ieee, smem, part, T, L, (int)grp.tid(),
-                     grp.id()))
-    return;
+  if constexpr (FX) {
+    if (pair >= kPairFixedFast &&
+        force_fx_group(pos, n, i0, jb, je, eps2, masses, ieee, smem, part, T, L, (int)grp.tid(),
+                       grp.id()))
+      return;
+  }
   double s[3];
   if (masses)
     force_f64_tiles<true>(pos, n, i0, jb, je, eps2, masses, ieee, reinterpret_cast<double*>(smem),

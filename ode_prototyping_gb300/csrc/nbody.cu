@@ -31,10 +31,14 @@ enum { kModeRhs = 0, kModeAccWrite = 1, kModeAccAdd = 2 };
 // unevenly spread over the SMs (3001: 2088 us for the 16 steps where they may).
 constexpr unsigned kFewCtas = 76;
 constexpr int kAfterCtasPerSm = 4;
-// Registers for 4 CTAs of 128 threads on an SM (N = 16384 1.66 ms, 1.88 at 5; 162
-// registers and 3 CTAs where the compiler is left to itself, 13 % slower).
-template <int T, int L, bool AFTER = false>
-__global__ void __launch_bounds__(T, 4 * 128 / T) rhs_f64_kernel(const double* __restrict__ pos,
+// FX: with fixed-point pair terms, and registers for 4 CTAs of 128 threads on an SM
+// (N = 16384 1.66 ms, 1.88 at 5; 162 registers and 3 CTAs where the compiler is left
+// to itself, 13 % slower).  Without them, for the calls that ask for the
+// reference's order, a kernel has the registers of the FP64 loop alone (N = 5000, 4
+// ranks of 8 lanes: 2.49 ms with those of the fixed-point one, whose 4 CTAs an SM
+// need a third wave, 2.25 so).
+template <int T, int L, bool AFTER = false, bool FX = true>
+__global__ void __launch_bounds__(T, FX ? 4 * 128 / T : 0) rhs_f64_kernel(const double* __restrict__ pos,
                                                     const double* __restrict__ vel,
                                                     double* __restrict__ out_vel,
                                                     double* __restrict__ out_acc, long long n,
@@ -42,7 +46,7 @@ __global__ void __launch_bounds__(T, 4 * 128 / T) rhs_f64_kernel(const double* _
                                                     const double* __restrict__ masses, int mode,
                                                     int pair) {
   constexpr int BI = T / L;
-  __shared__ __align__(16) unsigned char sh_raw[f64_smem_bytes<T>()];
+  __shared__ __align__(16) unsigned char sh_raw[FX ? f64_smem_bytes<T>() : 32 * T];
   __shared__ double part[BI][3];
   if constexpr (AFTER) {
     after_previous(pos, vel, out_vel, out_acc, masses);
@@ -52,7 +56,7 @@ __global__ void __launch_bounds__(T, 4 * 128 / T) rhs_f64_kernel(const double* _
   const long long i0 = ci.itile * BI;
   long long jb, je;
   j_chunk(n, ci.rank, ci.size, T, jb, je);
-  force_f64_cta<T, L>(pos, n, i0, jb, je, eps2, masses, sh_raw, part, pair);
+  force_f64_cta<T, L, FX>(pos, n, i0, jb, je, eps2, masses, sh_raw, part, pair);
   cluster_combine<BI>(part, ci.rank, ci.size);
   if (ci.rank != 0) return;
   const long long nb = min((long long)BI, n - i0);
@@ -196,13 +200,21 @@ __global__ void __launch_bounds__(T, (PACKED && L == 1 && BPT == 1 ? 9 : 5) * 12
   }
 }
 
-template <int T>
+template <int T, bool FX>
 const void* pick_f64(int L) {
   switch (L) {
-    case 1: return (const void*)rhs_f64_kernel<T, 1>;
-    case 2: return (const void*)rhs_f64_kernel<T, 2>;
-    case 4: return (const void*)rhs_f64_kernel<T, 4>;
-    case 8: return (const void*)rhs_f64_kernel<T, 8>;
+    case 1: return (const void*)rhs_f64_kernel<T, 1, false, FX>;
+    case 2: return (const void*)rhs_f64_kernel<T, 2, false, FX>;
+    case 4: return (const void*)rhs_f64_kernel<T, 4, false, FX>;
+    case 8: return (const void*)rhs_f64_kernel<T, 8, false, FX>;
+    default: return nullptr;
+  }
+}
+const void* pick_f64(const ForceGeom& g, bool fx) {
+  switch (g.T) {
+    case 64: return fx ? pick_f64<64, true>(g.L) : pick_f64<64, false>(g.L);
+    case 128: return fx ? pick_f64<128, true>(g.L) : pick_f64<128, false>(g.L);
+    case 256: return fx ? pick_f64<256, true>(g.L) : pick_f64<256, false>(g.L);
     default: return nullptr;
   }
 }
@@ -212,12 +224,13 @@ const void* pick_f64(int L) {
 bool may_overlap(const ForceGeom& g) {
   return g.n_itiles * g.P <= (long long)kAfterCtasPerSm * num_sms();
 }
+template <bool FX>
 const void* pick_f64_after(const ForceGeom& g) {
   if (g.T != 128 || !may_overlap(g)) return nullptr;
   switch (g.L) {
-    case 2: return (const void*)rhs_f64_kernel<128, 2, true>;
-    case 4: return (const void*)rhs_f64_kernel<128, 4, true>;
-    case 8: return (const void*)rhs_f64_kernel<128, 8, true>;
+    case 2: return (const void*)rhs_f64_kernel<128, 2, true, FX>;
+    case 4: return (const void*)rhs_f64_kernel<128, 4, true, FX>;
+    case 8: return (const void*)rhs_f64_kernel<128, 8, true, FX>;
     default: return nullptr;
   }
 }
@@ -270,13 +283,6 @@ int run_f64(const double* pos, const double* vel, double* out_vel, double* out_a
             double softening, double mass, const double* masses, int mode,
             const gb_force_tiling* tiling, cudaStream_t s) {
   ForceGeom g = choose_geom(n, GB_PREC_F64, tiling, 0);
-  const void* k = nullptr;
-  switch (g.T) {
-    case 64: k = pick_f64<64>(g.L); break;
-    case 128: k = pick_f64<128>(g.L); break;
-    case 256: k = pick_f64<256>(g.L); break;
-  }
-  if (!k) return GB_ERR_UNSUPPORTED;
   double eps2 = softening * softening;
   // Fixed-point pair terms (fixpair.cuh: closer to the exact sum than the
   // reference's operation order, and 14 times as fast at N = 16384) unless the
@@ -288,9 +294,12 @@ int run_f64(const double* pos, const double* vel, double* out_vel, double* out_a
   int pair = want == 1                   ? kPairFixedFast
              : want == 0 && !own_geom ? kPairFixedIeee
                                       : kPairIeee;
+  const bool fx = pair != kPairIeee;
+  const void* k = pick_f64(g, fx);
+  if (!k) return GB_ERR_UNSUPPORTED;
   void* args[] = {(void*)&pos, (void*)&vel, (void*)&out_vel, (void*)&out_acc, (void*)&n,
                   (void*)&eps2, (void*)&mass, (void*)&masses, (void*)&mode, (void*)&pair};
-  const void* ka = pick_f64_after(g);
+  const void* ka = fx ? pick_f64_after<true>(g) : pick_f64_after<false>(g);
   return launch_cluster(ka ? ka : k, g, 0, s, args, ka != nullptr);
 }
 

@@ -212,11 +212,16 @@ __device__ __forceinline__ void stage_unit(const DevTableau& tab, const BatchPar
 // CTA: warp group g of T / G threads, with its own named barrier and its own
 // slice of the shared buffers, integrates one whole system (its single tile).
 // FP64: registers for 4 CTAs of 128 threads on an SM (128 systems of 64 to 4096
-// bodies 1.64 ms a stage, 1.77 at 5, 1.81 at 6).  Mixed: none asked for (0); asked
-// for one CTA the compiler took 122 registers for 80 (one lane, 512 systems of 64
-// to 4096 bodies: 0.475 ms a stage, 0.449 so).
+// bodies 1.64 ms a stage, 1.77 at 5, 1.81 at 6).  Mixed: asked for one CTA the
+// compiler takes 122 registers, for none (0) 80.  The two-lane form, a batch's own
+// choice, has the 122: few systems wait for latency (us a stage: 64 systems of 64
+// to 2000 bodies 42.1 against 43.7, 128 of 64 to 4096 161 against 164), many run
+// longer (512: 503 against 489).  The other forms, which the tuner takes for many,
+// have the 80 (one lane, 512 systems: 449 against 475).
 template <int PREC, int T, int L, int BPT, int G>
-__global__ void __launch_bounds__(T, PREC == GB_PREC_F64 ? 4 * 128 / T : 0)
+__global__ void __launch_bounds__(T, PREC == GB_PREC_F64                          ? 4 * 128 / T
+                                     : T == 128 && L == 2 && BPT == 1 && G == 1 ? 1
+                                                                                : 0)
     batch_stage_kernel(const __grid_constant__ DevTableau tab,
                        const __grid_constant__ BatchParams P, int s) {
   static_assert(G == 1 || (T / G >= 32 && T <= 128 && (T / G / L) * BPT >= 1),

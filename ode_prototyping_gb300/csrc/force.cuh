@@ -863,14 +863,6 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float v) {
   s = t;
 }
 
-// Knuth's error-free sum: s + e == a + b exactly (explicit IEEE adds, so
-// nothing is contracted or reassociated).
-__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
-  s = __fadd_rn(a, b);
-  const float bb = __fsub_rn(s, a);
-  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-}
-
 // (S, E) += (hi, lo) in double-single arithmetic (an unevaluated sum of two
 // floats, about 48 significant bits), renormalised after each addition.
 __device__ __forceinline__ void ds_add(float& S, float& E, float hi, float lo) {

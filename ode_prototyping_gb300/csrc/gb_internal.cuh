@@ -100,6 +100,14 @@ __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a,
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 
+// Knuth's error-free sum: s + e == a + b exactly (explicit IEEE adds, so
+// nothing is contracted or reassociated).
+__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
+  s = __fadd_rn(a, b);
+  const float bb = __fsub_rn(s, a);
+  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+}
+
 // One softened pair term with the reference's operation order
 // (NBodyODE.hpp:89-98): r2 = dx*dx + dy*dy + dz*dz + eps2, den = sqrt(r2)*r2,
 // a = d / den, all IEEE-rounded.

@@ -201,19 +201,13 @@ struct Sum3 {
   float h = 0.f, m = 0.f, l = 0.f;
 };
 
-// Knuth's error-free sum: s + e == a + b.
-__device__ __forceinline__ void exact_sum(float a, float b, float& s, float& e) {
-  s = __fadd_rn(a, b);
-  const float bb = __fsub_rn(s, a);
-  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-}
 // t += h + m + l
 __device__ __forceinline__ void add3(Sum3& t, float h, float m, float l) {
   float e1, e2, e3, s;
-  exact_sum(t.h, h, s, e1);
+  two_sum(t.h, h, s, e1);
   t.h = s;
-  exact_sum(t.m, m, s, e2);
-  exact_sum(s, e1, t.m, e3);
+  two_sum(t.m, m, s, e2);
+  two_sum(s, e1, t.m, e3);
   t.l = __fadd_rn(t.l, __fadd_rn(l, __fadd_rn(e2, e3)));
 }
 // t += a b
@@ -223,9 +217,9 @@ __device__ __forceinline__ void add_product(Sum3& t, float a, float b) {
 }
 __device__ __forceinline__ void add_value(Sum3& t, float a) {
   float e, s;
-  exact_sum(t.h, a, s, e);
+  two_sum(t.h, a, s, e);
   t.h = s;
-  exact_sum(t.m, e, s, e);
+  two_sum(t.m, e, s, e);
   t.m = s;
   t.l = __fadd_rn(t.l, e);
 }
@@ -234,9 +228,9 @@ __device__ __forceinline__ void add_value(Sum3& t, float a) {
 // the middle one as large as the first after a cancellation.
 __device__ __forceinline__ float round3(const Sum3& t) {
   float h, m, l;
-  exact_sum(t.h, t.m, h, m);
-  exact_sum(m, t.l, m, l);
-  exact_sum(h, m, h, m);
+  two_sum(t.h, t.m, h, m);
+  two_sum(m, t.l, m, l);
+  two_sum(h, m, h, m);
   return __fadd_rn(h, __fadd_rn(m, l));
 }
 
